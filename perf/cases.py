@@ -16,9 +16,9 @@ Kinds:
   annulus   Taylor-Couette flow between cylinders, the same outputs;
   batch     uneven cylinder channels advanced together, every case's forces and field.
 
-Fields of runs with 16-bit storage come back in 16 bits, scaled as the storage scales them: that
-is all such a run holds, and how its snapshots are archived.  Force histories come back in 32
-bits, the precision of their per-node terms.
+Fields of runs with 16-bit storage are handed on in 16 bits, scaled as the storage scales them
+(all that such a run holds), to analysis on the GPU.  Force histories come back in 32 bits, the
+precision of their per-node terms.
 """
 import ctypes
 import math
@@ -201,21 +201,23 @@ def _batch_descs(case):
 
 
 def _field_buffers(sim, storage):
-    """Pinned host arrays for the field, and in 16-bit storage its scales and 16-bit copy."""
+    """Pinned host array for the field; in 16-bit storage also its scales and the 16-bit copy that
+    stays on the GPU for analysis there."""
     host = torch.empty((10,) + sim.shape, dtype=torch.float32, pin_memory=True)
     if storage == "f32":
-        return host, None, None
+        return host, None, None, None
     u = sim.desc.u_max
-    scale = torch.tensor([1 / u ** 2] + 3 * [1 / u] + 6 * [1 / u ** 2]).reshape(10, 1, 1, 1)
-    return host, scale, torch.empty(host.shape, dtype=torch.bfloat16 if storage == "bf16" else torch.float16)
+    scale = torch.tensor([1 / u ** 2] + 3 * [1 / u] + 6 * [1 / u ** 2]).reshape(10, 1, 1, 1).cuda()
+    wide = torch.empty(host.shape, dtype=torch.float32, device="cuda")
+    return host, scale, wide, torch.empty_like(wide, dtype=torch.bfloat16 if storage == "bf16" else torch.float16)
 
 
 def _read_field(sim, buffers):
-    host, scale, half = buffers
+    host, scale, wide, half = buffers
     sim.moments(out=host.numpy())
     if half is None:
         return host
-    return half.copy_(host.mul_(scale))
+    return half.copy_(wide.copy_(host, non_blocking=True).mul_(scale))
 
 
 def prepare(case, seed):
