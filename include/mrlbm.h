@@ -152,7 +152,7 @@ typedef struct mrlbm_info {
     int32_t storage;
     int32_t bytes_per_value;
     int32_t n_active_items;  /* work items (tile column x z-segment) the step kernel visits */
-    int32_t tile[3];      /* tile x, tile y, z-segment length used by the step kernel     */
+    int32_t tile[3];      /* x-block (a tile is two wide), tile height, z-segment length   */
     int32_t nb_solid[2];  /* BCSOLID nodes per wall (z walls only)                       */
     int32_t reserved[6];
 } mrlbm_info;
@@ -242,13 +242,12 @@ int mrlbm_write_geometry(const mrlbm_handle *h, const char *dir);
 /* ---- allocation-free step (no counterpart in the reference) ------------------------------------
  * One time step of a fully periodic box (no walls, no inlet / outlet) from m_in to m_out,
  * for callers that cannot allocate device memory: it calls no cudaMalloc / cudaFree and no
- * allocating library routine.  The step kernel's scratch (argument block, work items,
- * diagnostics partials) is one fixed 64 KiB array in the library's device image, which
- * bounds the grid to at most 11776 xy tiles of 32 x 16 nodes (ceil(nx/32) * ceil(ny/16)),
- * e.g. 2048 x 2944 nodes per z plane; larger grids are rejected with MRLBM_ERR_INVALID_ARG.
- * Every call shares that array and it keeps the last call's contents (each call rewrites
- * what it reads and clears its error word); calls that overlap on the GPU (two streams or
- * two host threads) race on it.
+ * allocating library routine.  The step kernel's scratch (diagnostics partials and sums, error
+ * word) is one fixed 64 KiB array in the library's device image; grids are limited to 11776 xy
+ * tiles of 32 x 16 nodes (ceil(nx/32) * ceil(ny/16)), e.g. 2048 x 2944 nodes per z plane, and
+ * larger ones rejected with MRLBM_ERR_INVALID_ARG.  Every call with diag shares that array
+ * (each rewrites what it reads): such calls race on it when they overlap on the GPU (two
+ * streams or two host threads).
  * m_in / m_out: device pointers, 16-byte aligned, not overlapping, FP32 moments in the
  * solver's storage layout: field f of node (x, y, z) at element
  * (((z*ny + y)*ceil(nx/32) + x/32)*10 + f)*32 + x%32, fields in the order of
@@ -264,7 +263,8 @@ int mrlbm_step_periodic_noalloc(const float *m_in, float *m_out, int32_t nx, int
 /* Time every tile height (4, 8, 16) with every z-segment length (the built-in heuristic and
  * powers of two below nz) over `trial_steps` steps and keep the fastest.  The moments, step
  * counter and sampling state are restored afterwards; results do not depend on the tiling.
- * tile_out (optional): {32, tile height, z-segment length}. */
+ * tile_out (optional): {32, tile height, z-segment length}; 32 is the x-block of the moment layout, a tile
+ * being two blocks wide. */
 int mrlbm_autotune(mrlbm_handle *h, int32_t trial_steps, int32_t tile_out[3]);
 /* Several independent cases (uneven grids allowed; one moment storage for all) advanced
  * together: per step one persistent step-kernel launch over the work items of every case,

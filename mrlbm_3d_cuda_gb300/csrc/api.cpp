@@ -56,15 +56,12 @@ void free_all(mrlbm_handle *h) {
     };
     f(h->m[0]);
     f(h->m[1]);
-    f(h->d_word);
+    f(h->d_mark);
     f(h->d_items);
-    f(h->d_args_sp);
     f(h->d_tile_slot);
     f(h->d_side);
     f(h->d_list_xyz);
     f(h->d_list_word);
-    f(h->d_row_base);
-    f(h->d_popbuf);
     for (int w = 0; w < 2; ++w) {
         for (int k = 0; k < 3; ++k) f(h->d_wf[w][k]);
         for (int k = 0; k < 2; ++k) f(h->d_wm[w][k]);
@@ -85,9 +82,9 @@ void free_all(mrlbm_handle *h) {
     f(h->d_ps_avg[1]);
     f(h->d_inlet);
     if (h->own_stream) cudaStreamDestroy(h->own_stream);
-    if (h->side_stream) cudaStreamDestroy(h->side_stream);
+    if (h->list_stream) cudaStreamDestroy(h->list_stream);
     if (h->ev_fork) cudaEventDestroy(h->ev_fork);
-    if (h->ev_join) cudaEventDestroy(h->ev_join);
+    if (h->ev_list) cudaEventDestroy(h->ev_list);
 }
 
 int64_t node_index_for_layout(const mrlbm_handle *h, int64_t lex, int layout) {
@@ -127,14 +124,12 @@ int sync_sr_step(mrlbm_handle *h) {
     return MRLBM_OK;
 }
 
-// Tile height and z-segment length from MRLBM_TILE_Y / MRLBM_LZ, else the defaults: 32 x 16
-// columns (the widest tile amortises the rim rebuild best: at 256^3 FP32 on GB300, 32 x 16 /
-// 32 x 8 / 32 x 4 run at 0.36 / 0.42 / 0.47 ms per step) and lz = 0, the heuristic below.
+// Tile height and z-segment length from MRLBM_TILE_Y / MRLBM_LZ, else 0: choose_tiling's.
 void default_tiling(int &ty, int &lz) {
     const char *ety = std::getenv("MRLBM_TILE_Y");
     const char *elz = std::getenv("MRLBM_LZ");
-    ty = ety ? std::atoi(ety) : 16;
-    if (ty != 4 && ty != 8 && ty != 16) ty = 16;
+    ty = ety ? std::atoi(ety) : 0;
+    if (ty != 4 && ty != 8 && ty != 16) ty = 0;
     lz = elz ? std::max(1, std::atoi(elz)) : 0;
 }
 
@@ -151,11 +146,10 @@ int storage_element_bytes(int storage) {
 int setup_tiling(mrlbm_handle *h, int ty, int lz) {
     const mrlbm_case_desc &d = h->d;
     const Geometry &g = h->geo;
-    if (ty != 4 && ty != 8 && ty != 16) return fail(h, MRLBM_ERR_INVALID_ARG, "tile height must be 4, 8 or 16");
+    choose_tiling(d.nx, d.ny, d.nz, h->storage, h->n_sm, ty, lz);
     CK(h, cudaStreamSynchronize(h->stream));
     for (void **p : {(void **)&h->d_tile_slot, (void **)&h->d_side, (void **)&h->d_items, (void **)&h->d_list_xyz,
-                     (void **)&h->d_list_word, (void **)&h->d_row_base, (void **)&h->d_popbuf,
-                     (void **)&h->d_diag_part}) {
+                     (void **)&h->d_list_word, (void **)&h->d_diag_part}) {
         if (*p) cudaFree(*p);
         *p = nullptr;
     }
@@ -166,13 +160,6 @@ int setup_tiling(mrlbm_handle *h, int ty, int lz) {
     if (per_sm <= 0) per_sm = 1;
     const int resident = per_sm * h->n_sm;
     const int tiles = h->tiles_x * h->tiles_y;
-    if (lz > 0) {
-        lz = std::min(d.nz, lz);
-    } else {
-        // longest z-segment that still gives every resident CTA several work items
-        lz = d.nz;
-        while (lz > 16 && (int64_t)tiles * ((d.nz + lz - 1) / lz) < 4LL * resident) lz = (lz + 1) / 2;
-    }
     h->lz = lz;
     std::vector<uint32_t> word(h->n, 0);
     for (int64_t i = 0; i < h->n; ++i) word[i] = make_word(g.cls[i], g.payload[i], g.frozen[i] != 0, g.stencil[i] != 0);
@@ -194,19 +181,16 @@ int setup_tiling(mrlbm_handle *h, int ty, int lz) {
     }
     h->n_special = n_special;
 
-    // Non-bulk nodes of special tiles, in the order the step kernel exports their pulled
-    // populations: slot, z, tile row, x.  Solid nodes of updated blocks need no populations:
-    // the step kernel collides them in place; frozen nodes are never updated.  Neither is
-    // in the list.
+    // Non-bulk nodes of special tiles, by slot, z, tile row, x.  Solid nodes of updated blocks need
+    // no populations: the step kernel collides them in place; frozen nodes are never updated.
+    // Neither is in the list.
     std::vector<uint64_t> list_xyz;
     std::vector<uint32_t> list_word;
-    std::vector<int32_t> row_base((size_t)n_special * d.nz * h->tile_y, 0);
     for (int t = 0; t < tiles; ++t) {
         if (slot[t] < 0) continue;
         const int x0 = (t % h->tiles_x) * TILE_X, y0 = (t / h->tiles_x) * h->tile_y;
         for (int z = 0; z < d.nz; ++z)
             for (int r = 0; r < h->tile_y; ++r) {
-                row_base[((size_t)slot[t] * d.nz + z) * h->tile_y + r] = (int32_t)list_xyz.size();
                 const int y = y0 + r;
                 if (y >= d.ny) continue;
                 for (int x = x0; x < std::min(d.nx, x0 + TILE_X); ++x) {
@@ -223,29 +207,26 @@ int setup_tiling(mrlbm_handle *h, int ty, int lz) {
     }
     if (list_xyz.size() >= (size_t)INT32_MAX / 27)
         return fail(h, MRLBM_ERR_INVALID_ARG, "too many boundary nodes");
-    h->n_list_pop = (int)list_xyz.size();
-    h->n_list = h->n_list_pop;
+    h->n_list = (int)list_xyz.size();
     h->n_list_blocks = special_list_blocks(h->n_list);
     const int nseg = (d.nz + h->lz - 1) / h->lz;
     // work items are int32 `tile | segment << 20` (decoded in step_kernel)
     if (tiles > (1 << 20) || nseg > (1 << 11))
         return fail(h, MRLBM_ERR_INVALID_ARG,
                     "grid too large for the work-item encoding (at most 2^20 xy tiles and 2^11 z segments)");
-    // tiles without boundary nodes go to the bulk variant of the step kernel, the others to
-    // the variant that reads node words: two launches, each over its own items
-    std::vector<int32_t> items, items_sp;
+    // tiles with boundary nodes first: they cost most, and CTAs take over items in this order
+    std::vector<int32_t> items, plain;
     for (int s = 0; s < nseg; ++s)
         for (int t = 0; t < tiles; ++t)
-            if (!skip[t]) (slot[t] >= 0 ? items_sp : items).push_back(t | (s << 20));
+            if (!skip[t]) (slot[t] >= 0 ? items : plain).push_back(t | (s << 20));
+    h->n_special_items = (int)items.size();
+    items.insert(items.end(), plain.begin(), plain.end());
+    h->special = n_special > 0;
     h->n_items = (int)items.size();
-    h->n_items_sp = (int)items_sp.size();
-    h->n_ctas = h->n_items ? std::max(1, std::min(h->n_items, resident)) : 0;
-    h->n_ctas_sp = h->n_items_sp ? std::max(1, std::min(h->n_items_sp, resident)) : 0;
+    h->n_ctas = h->special ? h->n_items : std::min(h->n_items, resident);
     h->h_items = items;
-    h->h_items_sp = items_sp;
-    items.insert(items.end(), items_sp.begin(), items_sp.end());
 
-    if (h->d_word) {
+    if (h->d_mark) {
         CK(h, upload(&h->d_tile_slot, slot.data(), slot.size()));
         if (n_special > 0) {
             const size_t side_floats = (size_t)n_special * d.nz * TILE_X * h->tile_y * 16;
@@ -255,38 +236,24 @@ int setup_tiling(mrlbm_handle *h, int ty, int lz) {
     }
     CK(h, upload(&h->d_items, items.data(), items.size()));
     CK(h, cudaMalloc((void **)&h->d_diag_part,
-                     (size_t)(h->n_ctas + h->n_ctas_sp + h->n_list_blocks) * 2 * sizeof(double)));
+                     ((size_t)h->n_ctas * h->tile_y + h->n_list_blocks) * 2 * sizeof(double)));
     if (h->n_list > 0) {
         CK(h, upload(&h->d_list_xyz, list_xyz.data(), list_xyz.size()));
         CK(h, upload(&h->d_list_word, list_word.data(), list_word.size()));
-        CK(h, upload(&h->d_row_base, row_base.data(), row_base.size()));
-        if (h->n_list_pop > 0) CK(h, cudaMalloc((void **)&h->d_popbuf, (size_t)h->n_list_pop * 27 * sizeof(float)));
     }
     StepArgs &a = h->args;
-    // a single case's items are uniform: CTAs stride through them, which keeps neighbouring
-    // tiles in flight together (L2 reuse of the rim columns); batches claim items on demand
-    a.work_counter = nullptr;
     a.items = h->d_items;
     a.n_items = h->n_items;
     a.tile_slot = h->d_tile_slot;
     a.side = h->d_side;
     a.list_xyz = h->d_list_xyz;
     a.list_word = h->d_list_word;
-    a.n_list_pop = h->n_list_pop;
     a.n_list = h->n_list;
-    a.popbuf = h->d_popbuf;
-    a.row_base = h->d_row_base;
     a.tiles_x = h->tiles_x;
     a.tiles_y = h->tiles_y;
     a.tile_y = h->tile_y;
     a.lz = h->lz;
     CK(h, cudaMemcpy(h->d_args, &a, sizeof(StepArgs), cudaMemcpyHostToDevice));
-    StepArgs asp = a;
-    asp.items = h->d_items ? h->d_items + h->n_items : nullptr;
-    asp.n_items = h->n_items_sp;
-    asp.work_counter = nullptr;
-    if (!h->d_args_sp) CK(h, cudaMalloc((void **)&h->d_args_sp, sizeof(StepArgs)));
-    CK(h, cudaMemcpy(h->d_args_sp, &asp, sizeof(StepArgs), cudaMemcpyHostToDevice));
     return MRLBM_OK;
 }
 
@@ -311,9 +278,9 @@ int step_handle(mrlbm_handle *h, int32_t nsteps) {
         const bool ws = !ds && h->watchdog_every > 0 && (it + 1) % h->watchdog_every == 0;
         StepLaunch L;
         L.ga = h->d_args;
+        L.args = &h->args;
         L.parity = h->parity;
         L.n_ctas = h->n_ctas;
-        L.full_tiles = h->d.nx % TILE_X == 0 && h->d.ny % h->tile_y == 0;
         if (fs) {
             const int64_t slot = h->force_count % kRing;
             L.force = h->d_force_ring + slot * 10;
@@ -323,30 +290,18 @@ int step_handle(mrlbm_handle *h, int32_t nsteps) {
         }
         const bool sums = ds || ws;
         if (sums) L.diag_part = h->d_diag_part;
-        const int n_step_parts = h->n_ctas + h->n_ctas_sp;
-        // The boundary work of the step runs on the side stream, concurrently with the bulk
-        // tiles: the boundary-tile step kernel, then the node-list kernel (it reads only the
-        // populations that kernel exported) and the wall kernel (it reads only the list
-        // kernel's stencil snapshots); their blocks fill the SMs the bulk launch leaves idle
-        // in its last wave.  No bulk-tile node is read or written by them.
-        cudaStream_t bs = h->stream;
-        if (h->n_items_sp > 0) {
-            StepLaunch Ls = L;
-            Ls.ga = h->d_args_sp;
-            Ls.n_ctas = h->n_ctas_sp;
-            Ls.diag_part = sums ? h->d_diag_part + 2 * h->n_ctas : nullptr;
+        // the node-list kernel reads only the state before the step: it runs on its own stream beside
+        // the step kernel; the wall kernel reads the stencil snapshots of both
+        if (h->n_list > 0) {
             CK(h, cudaEventRecord(h->ev_fork, h->stream));
-            CK(h, cudaStreamWaitEvent(h->side_stream, h->ev_fork, 0));
-            CK(h, launch_step(Ls, h->storage, h->tile_y, true, h->side_stream));
-            bs = h->side_stream;
+            CK(h, cudaStreamWaitEvent(h->list_stream, h->ev_fork, 0));
+            CK(h, launch_special_list(L, h->storage, h->n_list_blocks, sums ? h->d_diag_part + 2 * (size_t)h->n_ctas * h->tile_y : nullptr,
+                                      h->list_stream));
+            CK(h, cudaEventRecord(h->ev_list, h->list_stream));
         }
-        if (h->n_list > 0)
-            CK(h, launch_special_list(L, h->storage, h->n_list_blocks, sums ? h->d_diag_part + 2 * n_step_parts : nullptr,
-                                      bs));
-        if (nb > 0) CK(h, launch_wall(L, h->storage, nb + (fs ? nbf : 0), bs));
-        if (h->n_items_sp > 0) CK(h, cudaEventRecord(h->ev_join, h->side_stream));
-        if (h->n_items > 0) CK(h, launch_step(L, h->storage, h->tile_y, false, h->stream));
-        if (h->n_items_sp > 0) CK(h, cudaStreamWaitEvent(h->stream, h->ev_join, 0));
+        if (h->n_items > 0) CK(h, launch_step(L, h->storage, h->tile_y, h->special, h->stream));
+        if (h->n_list > 0) CK(h, cudaStreamWaitEvent(h->stream, h->ev_list, 0));
+        if (nb > 0) CK(h, launch_wall(L, h->storage, nb + (fs ? nbf : 0), h->stream));
         if (h->ps_start >= 0 && it >= h->ps_start && it <= h->ps_end) {
             // statistics window: the post-step state (buffer parity ^ 1), as the reference's
             // post_process_step samples it
@@ -361,7 +316,7 @@ int step_handle(mrlbm_handle *h, int32_t nsteps) {
                                               h->stream));
         }
         if (sums) {
-            const int parts = n_step_parts + (h->n_list > 0 ? h->n_list_blocks : 0);
+            const int parts = h->n_ctas * h->tile_y + (h->n_list > 0 ? h->n_list_blocks : 0);
             if (ds) {
                 const int64_t slot = h->diag_count % kRing;
                 CK(h, launch_diag_finalize(h->d_diag_part, parts, h->d_diag_ring + slot * 2, h->d_error, h->stream));
@@ -588,9 +543,9 @@ int mrlbm_create(const mrlbm_case_desc *din, mrlbm_handle **out) {
     }
     CK(h.get(), cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking));
     h->stream = h->own_stream;
-    CK(h.get(), cudaStreamCreateWithFlags(&h->side_stream, cudaStreamNonBlocking));
+    CK(h.get(), cudaStreamCreateWithFlags(&h->list_stream, cudaStreamNonBlocking));
     CK(h.get(), cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
-    CK(h.get(), cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming));
+    CK(h.get(), cudaEventCreateWithFlags(&h->ev_list, cudaEventDisableTiming));
 
     // geometry on the host
     const std::string ge = classify(h->d, h->geo);
@@ -634,7 +589,13 @@ int mrlbm_create(const mrlbm_case_desc *din, mrlbm_handle **out) {
     CK(H, cudaMalloc(&h->m[1], mbytes));
     CK(H, cudaMemset(h->m[0], 0, mbytes));
     CK(H, cudaMemset(h->m[1], 0, mbytes));
-    if (any_special) CK(H, upload(&h->d_word, word.data(), word.size()));
+    if (any_special) {
+        const size_t pitch = (size_t)(d.nx + TILE_X - 1) / TILE_X * TILE_X, rows = (size_t)d.ny * d.nz;
+        std::vector<uint8_t> mark(pitch * rows, 0);
+        for (size_t r = 0; r < rows; ++r)
+            for (int x = 0; x < d.nx; ++x) mark[r * pitch + x] = node_mark(word[r * d.nx + x]);
+        CK(H, upload(&h->d_mark, mark.data(), mark.size()));
+    }
     for (int w = 0; w < g.n_walls; ++w) {
         const WallData &wd = g.wall[w];
         CK(H, upload(&h->d_wf[w][0], wd.nx.data(), wd.nx.size()));
@@ -666,7 +627,7 @@ int mrlbm_create(const mrlbm_case_desc *din, mrlbm_handle **out) {
     a.m[0] = h->m[0];
     a.m[1] = h->m[1];
     a.nxb = (d.nx + kXBlock - 1) / kXBlock;
-    a.word = h->d_word;
+    a.mark = h->d_mark;
     a.nx = d.nx;
     a.ny = d.ny;
     a.nz = d.nz;
@@ -705,7 +666,7 @@ int mrlbm_create(const mrlbm_case_desc *din, mrlbm_handle **out) {
     }
     CK(H, cudaMalloc((void **)&h->d_args, sizeof(StepArgs)));
     {
-        int ty = 16, lz = 0;
+        int ty = 0, lz = 0;
         default_tiling(ty, lz);
         const int rc = setup_tiling(H, ty, lz);
         if (rc != MRLBM_OK) return rc;
@@ -750,11 +711,11 @@ int mrlbm_get_info(const mrlbm_handle *h, mrlbm_info *info) {
     info->step = h->step;
     info->storage = h->storage;
     info->bytes_per_value = h->vbytes;
-    info->n_active_items = h->n_items + h->n_items_sp;
-    info->tile[0] = TILE_X;
+    info->n_active_items = h->n_items;
+    info->tile[0] = kXBlock;
     info->tile[1] = h->tile_y;
     info->tile[2] = h->lz;
-    info->reserved[0] = h->n_ctas + h->n_ctas_sp;
+    info->reserved[0] = h->n_ctas;
     info->reserved[1] = h->n_special;
     info->reserved[2] = (int32_t)std::min<int64_t>(h->n_fluid, INT32_MAX);
     return MRLBM_OK;
@@ -867,7 +828,7 @@ int mrlbm_autotune(mrlbm_handle *h, int32_t trial_steps, int32_t tile_out[3]) {
     if (r2 != MRLBM_OK) return r2;
     if (r3 != MRLBM_OK) return r3;
     if (tile_out) {
-        tile_out[0] = TILE_X;
+        tile_out[0] = kXBlock;
         tile_out[1] = h->tile_y;
         tile_out[2] = h->lz;
     }
@@ -881,6 +842,7 @@ int mrlbm_sync(mrlbm_handle *h) {
     int e = 0;
     CK(h, cudaMemcpy(&e, h->d_error, sizeof(int), cudaMemcpyDeviceToHost));
     *h->h_status = e;
+    if (e & kErrorWait) return fail(h, MRLBM_ERR_TIMEOUT, "a wait inside the step kernel ran out");
     if (e & ~kErrorDiverged)
         return fail(h, MRLBM_ERR_CUDA, "device reported a stencil lookup failure (code " + std::to_string(e) + ")");
     if (e & kErrorDiverged)
@@ -1078,8 +1040,7 @@ void batch_free_graphs(mrlbm_batch *b) {
 void batch_free_tables(mrlbm_batch *b) {
     batch_free_graphs(b);
     for (void **p : {(void **)&b->d_cases, (void **)&b->d_items, (void **)&b->d_list_blocks,
-                     (void **)&b->d_wall_blocks, (void **)&b->d_ring, (void **)&b->d_slot, (void **)&b->d_ba,
-                     (void **)&b->d_ba_sp, (void **)&b->d_work}) {
+                     (void **)&b->d_wall_blocks, (void **)&b->d_ring, (void **)&b->d_slot, (void **)&b->d_ba}) {
         if (*p) cudaFree(*p);
         *p = nullptr;
     }
@@ -1098,14 +1059,14 @@ int batch_set_tiling(mrlbm_batch *b, int ty, int lz) {
     const int n = (int)b->h.size();
     std::vector<const StepArgs *> cases(n);
     std::vector<double *> ring(n);
-    std::vector<int2> items, items_sp;
+    std::vector<int2> items, plain;  // tiles with boundary nodes of every case first
     std::vector<int4> lblocks, wblocks;
     for (int c = 0; c < n; ++c) {
         mrlbm_handle *h = b->h[c];
         cases[c] = h->d_args;
         ring[c] = h->d_force_ring;
-        for (int32_t it : h->h_items) items.push_back(make_int2(c, it));
-        for (int32_t it : h->h_items_sp) items_sp.push_back(make_int2(c, it));
+        for (size_t k = 0; k < h->h_items.size(); ++k)
+            ((int)k < h->n_special_items ? items : plain).push_back(make_int2(c, h->h_items[k]));
         if (h->n_list > 0) {
             const int first = (int)lblocks.size();
             for (int k = 0; k < h->n_list_blocks; ++k) lblocks.push_back(make_int4(c, first, h->n_list_blocks, 0));
@@ -1117,15 +1078,10 @@ int batch_set_tiling(mrlbm_batch *b, int ty, int lz) {
             for (int k = 0; k < nblk; ++k) wblocks.push_back(make_int4(c, first, nblk, 0));
         }
     }
+    items.insert(items.end(), plain.begin(), plain.end());
     b->n_items = (int)items.size();
-    b->n_items_sp = (int)items_sp.size();
-    items.insert(items.end(), items_sp.begin(), items_sp.end());
     b->n_list_blocks = (int)lblocks.size();
     b->n_wall_blocks = (int)wblocks.size();
-    int per_sm = step_kernel_max_ctas_per_sm(b->storage, ty);
-    if (per_sm <= 0) per_sm = 1;
-    b->n_ctas = b->n_items ? std::max(1, std::min(b->n_items, per_sm * b->h[0]->n_sm)) : 0;
-    b->n_ctas_sp = b->n_items_sp ? std::max(1, std::min(b->n_items_sp, per_sm * b->h[0]->n_sm)) : 0;
     auto up = [&](auto **dptr, const auto &v) -> cudaError_t {
         using T = typename std::remove_reference<decltype(v)>::type::value_type;
         if (v.empty()) return cudaSuccess;
@@ -1140,10 +1096,7 @@ int batch_set_tiling(mrlbm_batch *b, int ty, int lz) {
     BCK(up(&b->d_wall_blocks, wblocks));
     BCK(cudaMalloc((void **)&b->d_slot, sizeof(int)));
     BCK(cudaMemset(b->d_slot, 0, sizeof(int)));
-    BCK(cudaMalloc((void **)&b->d_work, 2 * sizeof(int)));
-    BCK(cudaMemset(b->d_work, 0, 2 * sizeof(int)));
     BatchArgs ba;
-    ba.work_counter = b->d_work;
     ba.cases = b->d_cases;
     ba.items = b->d_items;
     ba.n_items = b->n_items;
@@ -1153,28 +1106,20 @@ int batch_set_tiling(mrlbm_batch *b, int ty, int lz) {
     ba.force_slot = b->d_slot;
     BCK(cudaMalloc((void **)&b->d_ba, sizeof(BatchArgs)));
     BCK(cudaMemcpy(b->d_ba, &ba, sizeof(BatchArgs), cudaMemcpyHostToDevice));
-    BatchArgs bsp = ba;
-    bsp.items = b->d_items ? b->d_items + b->n_items : nullptr;
-    bsp.n_items = b->n_items_sp;
-    bsp.work_counter = b->d_work + 1;
-    BCK(cudaMalloc((void **)&b->d_ba_sp, sizeof(BatchArgs)));
-    BCK(cudaMemcpy(b->d_ba_sp, &bsp, sizeof(BatchArgs), cudaMemcpyHostToDevice));
     BCK(prepare_step_batch(b->storage, ty));  // both variants, before any capture
     return MRLBM_OK;
 }
 
 // The three batched launches of one step.
 int batch_launch(mrlbm_batch *b, int parity, int force) {
-    BCK(cudaMemsetAsync(b->d_work, 0, 2 * sizeof(int), b->stream));
-    if (b->n_items_sp > 0) {
+    if (b->n_list_blocks > 0) {
         BCK(cudaEventRecord(b->ev_fork, b->stream));
         BCK(cudaStreamWaitEvent(b->side_stream, b->ev_fork, 0));
-        BCK(launch_step_batch(b->d_ba_sp, parity, b->storage, b->tile_y, true, b->n_ctas_sp, b->side_stream));
+        BCK(launch_special_list_batch(b->d_ba, parity, force, b->storage, b->n_list_blocks, b->side_stream));
         BCK(cudaEventRecord(b->ev_join, b->side_stream));
     }
-    if (b->n_items > 0) BCK(launch_step_batch(b->d_ba, parity, b->storage, b->tile_y, false, b->n_ctas, b->stream));
-    if (b->n_items_sp > 0) BCK(cudaStreamWaitEvent(b->stream, b->ev_join, 0));
-    BCK(launch_special_list_batch(b->d_ba, parity, force, b->storage, b->n_list_blocks, b->stream));
+    if (b->n_items > 0) BCK(launch_step_batch(b->d_ba, parity, b->storage, b->tile_y, b->n_items, b->stream));
+    if (b->n_list_blocks > 0) BCK(cudaStreamWaitEvent(b->stream, b->ev_join, 0));
     BCK(launch_wall_batch(b->d_ba, parity, force, b->storage, b->n_wall_blocks, b->stream));
     bool any_sr = false;
     for (const mrlbm_handle *h : b->h) any_sr = any_sr || h->d_sr_step != nullptr;
@@ -1284,8 +1229,9 @@ int mrlbm_batch_create(const mrlbm_case_desc *descs, int32_t n, mrlbm_batch **ou
         h->stream = b->stream;
         h->batch = b.get();
     }
-    int ty = 16, lz = 0;
+    int ty = 0, lz = 0;
     default_tiling(ty, lz);
+    if (ty == 0) ty = 16;  // one height for all cases of the batch
     const int rc = batch_set_tiling(b.get(), ty, lz);
     if (rc != MRLBM_OK) {
         const std::string msg = g_last_error;
@@ -1439,7 +1385,7 @@ int mrlbm_batch_autotune(mrlbm_batch *b, int32_t trial_steps, int32_t tile_out[3
     if (r2 != MRLBM_OK) return r2;
     if (r3 != MRLBM_OK) return r3;
     if (tile_out) {
-        tile_out[0] = TILE_X;
+        tile_out[0] = kXBlock;
         tile_out[1] = b->tile_y;
         tile_out[2] = b->lz;
     }

@@ -32,9 +32,9 @@ struct mrlbm_handle {
     bool host_only = false;
     int dev = 0, n_sm = 0;
     cudaStream_t own_stream = nullptr, stream = nullptr;
-    // the boundary-tile step launch runs beside the bulk one: side stream and fork / join events
-    cudaStream_t side_stream = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    // the node-list launch runs beside the step kernel: its stream and fork / join events
+    cudaStream_t list_stream = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_list = nullptr;
     int storage = 0, vbytes = 4;
     StorageScale sc{};
     int64_t n = 0, fs = 0;
@@ -45,26 +45,24 @@ struct mrlbm_handle {
     // step-kernel configuration
     int tile_y = 8, lz = 32, tiles_x = 0, tiles_y = 0, n_items = 0, n_ctas = 0;
     int64_t n_fluid = 0;
-    uint32_t *d_word = nullptr;
+    uint8_t *d_mark = nullptr;
     int32_t *d_items = nullptr, *d_tile_slot = nullptr;
     float *d_side = nullptr;
     int n_special = 0;
     // non-bulk node list handled by the node-list kernel
     uint64_t *d_list_xyz = nullptr;
     uint32_t *d_list_word = nullptr;
-    int32_t *d_row_base = nullptr;
-    float *d_popbuf = nullptr;
-    int n_list_pop = 0, n_list = 0, n_list_blocks = 0;
+    int n_list = 0, n_list_blocks = 0;
     // walls
     float *d_wf[2][3] = {{nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr}};
     uint32_t *d_wm[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
     int64_t *d_wl[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
     uint32_t *d_tag = nullptr;  // [512]: in masks then out masks
     StepArgs args{};
-    StepArgs *d_args = nullptr;     // work items of tiles without boundary nodes (bulk kernel)
-    StepArgs *d_args_sp = nullptr;  // the same with the work items of tiles holding boundary nodes
-    int n_items_sp = 0, n_ctas_sp = 0;
-    std::vector<int32_t> h_items, h_items_sp;  // host copies of the two work-item lists
+    StepArgs *d_args = nullptr;     // device copy of args
+    bool special = false;           // some tile holds boundary nodes
+    int n_special_items = 0;        // work items of such tiles: the first of the list
+    std::vector<int32_t> h_items;   // host copy of the work-item list
     mrlbm_batch *batch = nullptr;   // owning batch, if any
     int *d_error = nullptr;
     // divergence watchdog: every watchdog_every steps (0: off) the step computes its FP64 mass /
@@ -100,7 +98,7 @@ struct mrlbm_handle {
 struct mrlbm_batch {
     std::vector<mrlbm_handle *> h;
     cudaStream_t stream = nullptr;
-    cudaStream_t side_stream = nullptr;  // boundary-tile step launch, forked / joined by events
+    cudaStream_t side_stream = nullptr;  // node-list launch, forked / joined by events
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     int storage = 0, tile_y = 16, lz = 0;
     int parity = 0;
@@ -109,13 +107,12 @@ struct mrlbm_batch {
     int64_t force_count = 0;  // sampled steps so far (the ring slot of the cases with walls)
     // device tables (BatchArgs and what it points to)
     const StepArgs **d_cases = nullptr;
-    int2 *d_items = nullptr;  // bulk work items, then the boundary-tile work items
+    int2 *d_items = nullptr;  // work items, tiles with boundary nodes first
     int4 *d_list_blocks = nullptr, *d_wall_blocks = nullptr;
     double **d_ring = nullptr;
     int *d_slot = nullptr;
-    BatchArgs *d_ba = nullptr, *d_ba_sp = nullptr;  // bulk / boundary-tile items
-    int n_items = 0, n_ctas = 0, n_items_sp = 0, n_ctas_sp = 0, n_list_blocks = 0, n_wall_blocks = 0;
-    int *d_work = nullptr;  // [2] work-item counters of the two batched step launches
+    BatchArgs *d_ba = nullptr;
+    int n_items = 0, n_list_blocks = 0, n_wall_blocks = 0;
     cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // [parity][force]
 };
 

@@ -24,11 +24,13 @@ template <typename S>
 struct StorageLayout {
     static constexpr int esz = (int)sizeof(S);  // bytes per storage element
     static constexpr int per_node = 10;         // elements per node (32-node run: per_node x 32)
+    static constexpr int words = per_node * esz / 4;  // 32-bit words per node
 };
 template <>
 struct StorageLayout<HybridWord> {
     static constexpr int esz = 4;
     static constexpr int per_node = 7;
+    static constexpr int words = 7;
 };
 inline __host__ __device__ int64_t aos_index(int x, int y, int z, int nxb, int ny, int esz, int per_node = 10) {
     const int64_t run = ((((int64_t)z * ny + y) * nxb + (x >> 5)) * per_node) * kXBlock;
@@ -68,8 +70,8 @@ struct WallArgs {
 struct StepArgs {
     void *m[2] = {nullptr, nullptr};  // ping-pong moment buffers (aos layout)
     int nxb = 0;                      // 32-node x-blocks per row
-    const uint32_t *word = nullptr;     // internal node words (lexicographic); null if all bulk
-    const int32_t *items = nullptr;     // work items: tile index | (z-segment << 20)
+    const uint8_t *mark = nullptr;      // node marks, rows of tiles_x * TILE_X bytes; null if all bulk
+    const int32_t *items = nullptr;     // work items: tile index | (z-segment << 20); null: all, segment by segment
     int n_items = 0;
     const int32_t *tile_slot = nullptr; // per xy tile: -1 plain, >= 0 side-buffer slot
     float *side = nullptr;              // post-stream moments of stencil nodes, 10 floats each
@@ -82,15 +84,10 @@ struct StepArgs {
     WallArgs wall[2];
     const uint32_t *tag_in = nullptr, *tag_out = nullptr;  // [256] BCFLUID masks
     int *error = nullptr;     // sticky device error flag
-    // non-bulk node list (special tiles only): every entry gets its 27 pulled populations
-    // from the step kernel, in (tile slot, z, tile row, x) order (n_list == n_list_pop;
-    // plain stencil nodes and solid nodes are updated by the step kernel itself)
+    // nodes handled by the node-list kernel (those the step kernel does not update itself)
     const uint64_t *list_xyz = nullptr;   // x | y << 21 | z << 42
     const uint32_t *list_word = nullptr;  // node word of each entry
-    int n_list_pop = 0, n_list = 0;
-    float *popbuf = nullptr;              // [27][n_list_pop]
-    const int32_t *row_base = nullptr;    // [slot][z][tile row]: first list entry of the row
-    int *work_counter = nullptr;          // work items claimed beyond the first gridDim.x (zeroed per launch)
+    int n_list = 0;
     // stochastic rounding of 16-bit stores: the step counter that seeds the random bits
     // (null: round to nearest)
     const uint32_t *sr_step = nullptr;
@@ -107,17 +104,16 @@ struct BatchArgs {
     const int4 *wall_blocks = nullptr;       // per wall block: {case, first block of the case, blocks, 0}
     double *const *force_ring = nullptr;     // per case: force ring of the case
     const int *force_slot = nullptr;         // ring slot of the sampled step
-    int *work_counter = nullptr;             // as StepArgs::work_counter, for the batched launch
 };
 
 // Per-step launch parameters.
 struct StepLaunch {
-    const StepArgs *ga = nullptr;  // device copy of the handle's StepArgs
+    const StepArgs *ga = nullptr;    // device copy of the handle's StepArgs
+    const StepArgs *args = nullptr;  // host copy, passed by value to the step kernel
     int parity = 0;                // read m[parity], write m[parity ^ 1]
     double *force = nullptr;       // [2][5] FP64 accumulators of a sampled step, or null
-    double *diag_part = nullptr;   // [grid][2] per-CTA mass / energy partials, or null
-    int n_ctas = 0;
-    bool full_tiles = false;       // every tile whole (nx % 32 == 0, ny % tile_y == 0)
+    double *diag_part = nullptr;   // [n_ctas][tile_y][2] mass / energy partials, or null
+    int n_ctas = 0;                // special: one per work item
 };
 
 // Stencil-buffer index of node (x, y, z) for a special tile slot.
@@ -128,24 +124,28 @@ inline __host__ __device__ int64_t side_index(int slot, int x, int y, int z, int
 
 // storage: 0 f32, 1 f16, 2 bf16
 cudaError_t launch_step(const StepLaunch &l, int storage, int tile_y, bool special, cudaStream_t s);
-cudaError_t launch_step_batch(const BatchArgs *ba, int parity, int storage, int tile_y, bool special, int n_ctas,
-                              cudaStream_t s);
+cudaError_t launch_step_batch(const BatchArgs *ba, int parity, int storage, int tile_y, int n_items, cudaStream_t s);
 cudaError_t prepare_step_batch(int storage, int tile_y);  // before capturing batched launches
 cudaError_t launch_special_list_batch(const BatchArgs *ba, int parity, int force, int storage, int n_blocks,
                                       cudaStream_t s);
 cudaError_t launch_wall_batch(const BatchArgs *ba, int parity, int force, int storage, int n_blocks, cudaStream_t s);
 // Zero the slot of every case's force ring and publish the slot for the batched wall kernel.
 cudaError_t launch_batch_force_begin(double *const *ring, int n_cases, int slot, int *d_slot, cudaStream_t s);
-int step_kernel_smem_bytes(int tile_y);
+// Tile height (4, 8 or 16; any other value on entry: the default) and z-segment length (> 0 on entry:
+// kept, clipped to nz).
+void choose_tiling(int nx, int ny, int nz, int storage, int n_sm, int &ty, int &lz);
 int step_kernel_max_ctas_per_sm(int storage, int tile_y);
 // Curved-wall closure + collision for the wall nodes of both walls, plus the force sums.
 cudaError_t launch_wall(const StepLaunch &l, int storage, int n_total, cudaStream_t s);
-// Closures, stencil snapshots and collision of the listed non-bulk nodes (after launch_step).
+// Closures, stencil snapshots and collision of the listed nodes (reads the state before the step
+// only: independent of launch_step).
 int special_list_blocks(int n_list);
 cudaError_t launch_special_list(const StepLaunch &l, int storage, int n_blocks, double *diag_part, cudaStream_t s);
 // Sum the per-CTA diagnostics partials into out[2] in a fixed order; a non-finite sum sets
 // kErrorDiverged in *error (if given).
 constexpr int kErrorDiverged = 16;
+// A wait inside the step kernel ran out (see packed.cuh).
+constexpr int kErrorWait = 32;
 cudaError_t launch_diag_finalize(const double *part, int n, double *out, int *error, cudaStream_t s);
 
 struct InitArgs {
@@ -181,24 +181,17 @@ cudaError_t launch_inlet_density(const StepArgs *ga, int buf, int storage, doubl
 cudaError_t launch_surface_pressure(const StepArgs *ga, int buf, int storage, int wall, int nb, double *avg, int n_avg,
                                     cudaStream_t s);
 
-// Allocation-free periodic step (mrlbm_step_periodic_noalloc).  Everything the step kernel
-// needs besides the caller's two moment buffers lives in one fixed array in the library's
-// device image, laid out as:
-//   [0, 1536)            StepArgs
-//   [1536, 1552)         mass / energy sums (2 doubles)
-//   [1600, 1604)         error word
-//   [1604, 1608)         work-item counter of the step kernel
-//   [2048, 18432)        per-CTA diagnostics partials, 2 doubles per CTA
-//   [18432, 65536)       work items, one int32 each
+// Allocation-free periodic step (mrlbm_step_periodic_noalloc).  What a step needs on the device
+// besides the caller's two moment buffers lives in one fixed array in the library's image:
+//   [0, 16)              mass / energy sums (2 doubles)
+//   [64, 68)             error word
+//   [1024, 65536)        diagnostics partials, 2 doubles per owner warp
 constexpr int kNoAllocScratchBytes = 64 * 1024;
-constexpr int kNoAllocDiagOffset = 1536;
-constexpr int kNoAllocErrorOffset = 1600;
-constexpr int kNoAllocWorkOffset = 1604;
-constexpr int kNoAllocPartOffset = 2048;
-constexpr int kNoAllocMaxCtas = 1024;
-constexpr int kNoAllocItemsOffset = kNoAllocPartOffset + kNoAllocMaxCtas * 2 * (int)sizeof(double);
-constexpr int kNoAllocMaxItems = (kNoAllocScratchBytes - kNoAllocItemsOffset) / (int)sizeof(int32_t);  // 11776
-constexpr int kNoAllocTileY = 16;
+constexpr int kNoAllocDiagOffset = 0;
+constexpr int kNoAllocErrorOffset = 64;
+constexpr int kNoAllocPartOffset = 1024;
+constexpr int kNoAllocMaxParts = (kNoAllocScratchBytes - kNoAllocPartOffset) / (2 * (int)sizeof(double));
+constexpr int kNoAllocMaxTiles = 11776;  // xy tiles of 32 x 16 nodes
 
 struct NoAllocStep {
     const float *m_in = nullptr;  // FP32 moments in the x-blocked storage layout

@@ -38,8 +38,21 @@ inline uint32_t make_word(uint32_t cls, uint32_t payload, bool frozen, bool sten
     return cls | (frozen ? NW_FROZEN : 0u) | (stencil ? NW_STENCIL : 0u) | (payload << NW_PAYLOAD_SHIFT);
 }
 
-// Step-kernel tiling: a CTA owns a TILE_X x tile_y column of nodes and marches along z.
-constexpr int TILE_X = 32;
+// Marks of a node for the step kernel (a byte): not updated as a bulk node; wall-stencil node, whose
+// post-stream moments the step kernel snapshots; solid node of an updated block, collided in place.
+// A plain bulk node has none; a node with MARK_OTHER alone is the node-list kernel's or frozen.
+constexpr uint32_t MARK_OTHER = 1u, MARK_SNAPSHOT = 2u, MARK_SOLID = 4u;
+inline uint8_t node_mark(uint32_t word) {
+    if (word == 0u) return 0u;
+    if (word == NW_STENCIL) return MARK_SNAPSHOT;
+    if ((word & (NW_CLASS_MASK | NW_FROZEN)) == C_SOLID)
+        return MARK_OTHER | MARK_SOLID | ((word & NW_STENCIL) ? MARK_SNAPSHOT : 0u);
+    return MARK_OTHER;
+}
+
+// Step-kernel tiling: a CTA owns a TILE_X x tile_y column of nodes (two x-blocks wide) and marches
+// along z.
+constexpr int TILE_X = 64;
 
 struct WallData {
     std::vector<int64_t> list;       // lexicographic node index, reference scan order

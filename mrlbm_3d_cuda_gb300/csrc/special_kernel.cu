@@ -1,13 +1,13 @@
-// Boundary and other non-bulk nodes: one thread per listed node, after the step kernel.
+// Boundary and other non-bulk nodes: one thread per listed node, beside the step kernel.
 //
-// The step kernel updates every plain bulk node in its fused pass, including plain fluid
-// nodes whose only mark is the wall-stencil bit (it also writes their snapshot), and collides
-// the solid nodes of updated blocks in place.  For every other node that carries a node word
-// (domain faces / edges / corners, BCFLUID, BCSOLID, curved-wall nodes) it only exports the 27
-// pulled populations to a list-ordered buffer; this kernel applies the node's closure,
-// snapshots stencil nodes for the wall kernel, collides and stores.  Nodes of blocks the
-// reference never updates (frozen) are in no list.  (The C_SOLID branch below is kept for a
-// list that would carry solid nodes; the list built by the host holds none.)
+// The step kernel updates every plain bulk node in its fused pass, including plain fluid nodes
+// whose only mark is the wall-stencil bit (it also writes their snapshot), and collides the solid
+// nodes of updated blocks in place.  Every other node that carries a node word (domain faces /
+// edges / corners, BCFLUID, BCSOLID, curved-wall nodes) is this kernel's: its closure needs single
+// populations, so the thread rebuilds the 27 that the node pulls from the stored moments of its
+// neighbours, applies the closure, snapshots stencil nodes for the wall kernel, collides and stores.
+// It reads the state before the step only, so it runs beside the step kernel.  Nodes of blocks
+// the reference never updates (frozen) are in no list.
 //
 // Reference (paths inside sakthi-lbm/MRLBM_3D_CUDA):
 //   evaluate_bounday_moments dispatch   MRLBM_3D/src/solver/mlbm.cu:166-184
@@ -60,6 +60,59 @@ __device__ __noinline__ Mom pulled_rho_u(const StepArgs &a, const S *__restrict_
         f[q] = g[q];
     }
     return rho_u_of(f);
+}
+
+__host__ __device__ constexpr int direction(int cx, int cy, int cz) {
+    for (int q = 0; q < 27; ++q)
+        if (cxq(q) == cx && cyq(q) == cy && czq(q) == cz) return q;
+    return -1;
+}
+
+// The populations of `mask` pulled by node (x, y, z) with this c_x, on the grid that wraps in every
+// axis, into f[direction * stride].  Three lanes share a node, one per c_x: the three neighbours
+// of a row mostly lie on one line, and the kernel is bound by the rate at which scattered loads touch
+// lines.
+template <typename S>
+__device__ __forceinline__ void pull(const StepArgs &a, const S *__restrict__ src, uint32_t mask, int cx, int x, int y,
+                                     int z, float *f, int stride) {
+    constexpr int WPN = StorageLayout<S>::words;
+    auto wrap = [](int v, int n) { return v < 0 ? v + n : (v >= n ? v - n : v); };
+    const int gx = wrap(x - cx, a.nx);
+    const uint32_t *__restrict__ p = reinterpret_cast<const uint32_t *>(src) + (gx >> 5) * (WPN * kXBlock) + (gx & 31);
+    const int64_t row = (int64_t)a.nxb * (WPN * kXBlock);
+#pragma unroll
+    for (int cz = -1; cz <= 1; ++cz) {
+        const int64_t plane = (int64_t)wrap(z - cz, a.nz) * a.ny;
+        // the loads of the three rows of this plane go out together
+        Raw<S> raw[3];
+#pragma unroll
+        for (int cy = -1; cy <= 1; ++cy) {
+            const int q = cx < 0 ? direction(-1, cy, cz) : (cx > 0 ? direction(1, cy, cz) : direction(0, cy, cz));
+            if (mask >> q & 1u) load_raw_words<S>(p + (plane + wrap(y - cy, a.ny)) * row, raw[cy + 1]);
+            else raw[cy + 1] = Raw<S>{};
+        }
+#pragma unroll
+        for (int cy = -1; cy <= 1; ++cy) {
+            const int q = cx < 0 ? direction(-1, cy, cz) : (cx > 0 ? direction(1, cy, cz) : direction(0, cy, cz));
+            float v[10], g[27];
+            raw_values<S>(raw[cy + 1], v);
+            rebuild<S>(v, a.rho0, a.sc, g);
+            f[q * stride] = cx < 0 ? g[direction(-1, cy, cz)] : (cx > 0 ? g[direction(1, cy, cz)] : g[direction(0, cy, cz)]);
+        }
+    }
+}
+
+// Populations that the closure of a listed node uses.
+__device__ __forceinline__ uint32_t needed(const StepArgs &a, uint32_t w) {
+    const uint32_t cls = w & NW_CLASS_MASK;
+    if (cls == C_INNER || cls == C_OUTER) return a.wall[cls == C_INNER ? 0 : 1].in_mask[w >> NW_PAYLOAD_SHIFT];
+    if (cls == C_BCFLUID_INNER || cls == C_BCFLUID_OUTER) return a.tag_in[(w >> NW_PAYLOAD_SHIFT) & 0xFFu];
+    const uint32_t walls = class_walls(cls);
+    if (walls == 0u || ((walls & 2u) && a.current_update)) return 0x7FFFFFFu;
+    uint32_t m = 0u;
+#pragma unroll
+    for (int q = 0; q < 27; ++q) m |= known_dir(walls, q) ? 1u << q : 0u;
+    return m;
 }
 
 // Closure of one listed node from its pulled populations `fl`.  Returns 0 when the node is
@@ -117,10 +170,7 @@ __device__ __forceinline__ int special_node(const StepArgs &a, int parity, bool 
     }
     if ((w & NW_STENCIL) && slot >= 0) {
         float *e = a.side + side_index(slot, x, y, z, x0, y0, a.nz, TILE_X, a.tile_y) * 16;
-        e[0] = m.rho - a.rho0;
-        e[1] = m.ux; e[2] = m.uy; e[3] = m.uz;
-        e[4] = m.mxx; e[5] = m.myy; e[6] = m.mzz;
-        e[7] = m.mxy; e[8] = m.mxz; e[9] = m.myz;
+        store_side(e, m.rho - a.rho0, m.ux, m.uy, m.uz, m.mxx, m.myy, m.mzz, m.mxy, m.mxz, m.myz);
     }
     if (wall_node) return 0;
     const bool bcf = force && slot >= 0 && (cls == C_BCFLUID_INNER || cls == C_BCFLUID_OUTER);
@@ -132,21 +182,22 @@ __device__ __forceinline__ int special_node(const StepArgs &a, int parity, bool 
         double fo[4];
         masked_momentum(a.tag_out[tag], m, fo);
         float *e = a.side + side_index(slot, x, y, z, x0, y0, a.nz, TILE_X, a.tile_y) * 16;
-        e[10] = (float)(fin[0] - fo[0]);
-        e[11] = (float)(fin[1] - fo[1]);
-        e[12] = (float)(fin[2] - fo[2]);
-        e[13] = (float)(fin[3] - fo[3]);
+        reinterpret_cast<float2 *>(e)[5] = make_float2((float)(fin[0] - fo[0]), (float)(fin[1] - fo[1]));
+        reinterpret_cast<float2 *>(e)[6] = make_float2((float)(fin[2] - fo[2]), (float)(fin[3] - fo[3]));
     }
     return fluid ? 2 : 1;
 }
 
-constexpr int kListThreads = 256;
+// A warp takes 30 nodes at a time: three rounds of ten nodes x three lanes gather the populations into
+// shared memory, then one lane per node applies its closure.
+constexpr int kListWarps = 4, kListThreads = 32 * kListWarps, kListNodes = 30;
 
 // BATCH: each block serves the case named by its entry in BatchArgs::list_blocks.
 template <typename S, bool BATCH>
 __global__ void __launch_bounds__(kListThreads)
     special_list_kernel(const StepArgs *__restrict__ ga, const BatchArgs *__restrict__ ba, int parity, int force,
                         double *__restrict__ diag_part) {
+    __shared__ float gathered[kListWarps][27][kListNodes + 1];
     int b0 = blockIdx.x, nblk = gridDim.x;
     if constexpr (BATCH) {
         const int4 m = ba->list_blocks[blockIdx.x];
@@ -156,30 +207,45 @@ __global__ void __launch_bounds__(kListThreads)
     }
     const StepArgs &a = *ga;
     S *__restrict__ dst = (S *)a.m[parity ^ 1];
-    const int n_pop = a.n_list_pop, n_all = a.n_list;
+    const int n_all = a.n_list;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double dm = 0.0, de = 0.0;
-    for (int i = b0 * blockDim.x + threadIdx.x; i < n_all; i += nblk * blockDim.x) {
-        const uint64_t p = a.list_xyz[i];
-        const int x = (int)(p & 0x1FFFFFu), y = (int)((p >> 21) & 0x1FFFFFu), z = (int)(p >> 42);
-        const uint32_t w = a.list_word[i];
-        float f[27];
+    for (int first = (b0 * kListWarps + warp) * kListNodes; first < n_all; first += nblk * kListWarps * kListNodes) {
+#pragma unroll 1
+        for (int r = 0; r < 3; ++r) {
+            const int j = 10 * r + lane / 3, i = first + j;
+            if (lane < 30 && i < n_all) {
+                const uint64_t p = a.list_xyz[i];
+                pull<S>(a, (const S *)a.m[parity], needed(a, a.list_word[i]), lane % 3 - 1, (int)(p & 0x1FFFFFu),
+                        (int)((p >> 21) & 0x1FFFFFu), (int)(p >> 42), &gathered[warp][0][j], kListNodes + 1);
+            }
+        }
+        __syncwarp();
+        const int i = first + lane;
+        if (lane < kListNodes && i < n_all) {
+            const uint64_t p = a.list_xyz[i];
+            const int x = (int)(p & 0x1FFFFFu), y = (int)((p >> 21) & 0x1FFFFFu), z = (int)(p >> 42);
+            const uint32_t w = a.list_word[i];
+            float f[27];
 #pragma unroll
-        for (int q = 0; q < 27; ++q) f[q] = a.popbuf[(int64_t)q * n_pop + i];
-        const int tx = x / TILE_X, ty = y / a.tile_y;
-        const int slot = a.tile_slot[ty * a.tiles_x + tx];
-        Mom m;
-        const int code = special_node<S>(a, parity, force != 0, w, f, x, y, z, slot, tx * TILE_X, ty * a.tile_y, m);
-        if (code) {
-            const int64_t ai = aos_at<S>(x, y, z, a.nxb, a.ny);
-            if (kScaled<S> && a.sr_step)
-                store_mom_sr<S>(dst, ai, m, a.rho0, a.sc, sr_key(sr_step_seed(*a.sr_step), x, y, z, a.nx, a.ny));
-            else
-                store_mom<S>(dst, ai, m, a.rho0, a.sc);
+            for (int q = 0; q < 27; ++q) f[q] = gathered[warp][q][lane];
+            const int tx = x / TILE_X, ty = y / a.tile_y;
+            const int slot = a.tile_slot[ty * a.tiles_x + tx];
+            Mom m;
+            const int code = special_node<S>(a, parity, force != 0, w, f, x, y, z, slot, tx * TILE_X, ty * a.tile_y, m);
+            if (code) {
+                const int64_t ai = aos_at<S>(x, y, z, a.nxb, a.ny);
+                if (kScaled<S> && a.sr_step)
+                    store_mom_sr<S>(dst, ai, m, a.rho0, a.sc, sr_key(sr_step_seed(*a.sr_step), x, y, z, a.nx, a.ny));
+                else
+                    store_mom<S>(dst, ai, m, a.rho0, a.sc);
+            }
+            if (code == 2 && diag_part) {
+                dm += (double)(m.rho - a.rho0);
+                de += 0.5 * (double)(m.ux * m.ux + m.uy * m.uy + m.uz * m.uz);
+            }
         }
-        if (code == 2 && diag_part) {
-            dm += (double)(m.rho - a.rho0);
-            de += 0.5 * (double)(m.ux * m.ux + m.uy * m.uy + m.uz * m.uz);
-        }
+        __syncwarp();
     }
     if (diag_part) {
         // fixed-order block reduction -> diag_part[blockIdx.x]
@@ -209,8 +275,8 @@ __global__ void __launch_bounds__(kListThreads)
 }  // namespace
 
 int special_list_blocks(int n_list) {
-    const int b = (n_list + kListThreads - 1) / kListThreads;
-    return b < 1 ? 1 : (b > 2048 ? 2048 : b);
+    const int b = (n_list + kListWarps * kListNodes - 1) / (kListWarps * kListNodes);
+    return b < 1 ? 1 : (b > 4096 ? 4096 : b);
 }
 
 cudaError_t launch_special_list(const StepLaunch &l, int storage, int n_blocks, double *diag_part, cudaStream_t s) {

@@ -1,5 +1,5 @@
-// Fused MR-LBM time step: stream + moment evaluation / boundary closure + collision in one
-// pass over HBM (one moment read, one moment write per node).
+// Fused MR-LBM time step: stream + moment evaluation + collision in one pass over HBM (one moment
+// read, one moment write per node).
 //
 // Replaces the reference's two full-grid kernels and their population halo
 // (paths inside sakthi-lbm/MRLBM_3D_CUDA):
@@ -7,13 +7,21 @@
 //   collision_halo_update       MRLBM_3D/src/solver/mlbm.cu:186-242
 //   pop_load_from_halo / pop_save_to_halo / save_pop / streaming
 //                               MRLBM_3D/src/core/D3Q27/halo_interface.cuh:5-201, core/streaming.cuh:6-35
-// The reference streams populations rebuilt from the stored (post-collision) moments:
-// f_q(x) = R(M(x - c_q))_q on a grid that wraps in every axis, then evaluates moments or a
-// boundary closure, then collides.  Here each CTA owns a 32 x TY column of nodes and marches
-// along z.  For every plane it rebuilds the populations of the column plus a one-node rim
-// (neighbour moments read through L2) into shared-memory ring buffers split by c_z, so a
-// node's 27 pulled populations come from planes z-1, z, z+1 without any population array in
-// HBM.  Post-collision moments go to the second ping-pong buffer.
+// The reference streams populations rebuilt from the stored (post-collision) moments,
+// f_q(x) = R(M(x - c_q))_q on a grid that wraps in every axis, then evaluates moments, then
+// collides.  Here a node's 27 pulled populations never leave registers: a lane owns two nodes
+// x, x + 1 of a row (every operation in packed FP32, sm_100's .f32x2), and its warp
+//   y: reads the stored moments of the rows y + 1, y, y - 1 of a plane from shared memory and rebuilds
+//      the nine populations of each that enter row y (c_y = -1, 0, +1);
+//   x: takes the neighbours' across lanes by shuffles;
+//   z: sums each c_z class of the plane (row and column sums) and marches along z with the classes
+//      of two planes in registers.
+// A row is rebuilt three times (139 packed operations a lane instead of 80), but no population crosses
+// shared memory and no warp waits for another: only the copies of the rows' moments are shared.
+// Bound by issue and FP32 throughput with 16-bit storage (600 warp instructions per 64 nodes, 65% of the
+// issue slots), by HBM with FP32 storage (5.6 TB/s).  256^3 on GB300, before (populations exchanged
+// through shared-memory rings between CTA barriers) and now: FP32 335 -> 240 us a step, FP16 283 -> 213,
+// hybrid 298 -> 218, BF16 283 -> 215.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -22,553 +30,720 @@
 #include <string>
 
 #include "mrlbm_internal.h"
+#include "packed.cuh"
 #include "storage.cuh"
 
 namespace mrlbm {
 namespace {
 
-// Populations exchanged through shared memory, split by c_z (the three c = (0,0,c_z)
-// populations stay in registers of the column's owner thread).
-// Eight 5-bit direction indices per class packed in one constant:
-//   up   (c_z = +1, pulled from plane z-1): 9, 11, 16, 18, 19, 22, 23, 25
-//   flat (c_z =  0, pulled from plane z):   1, 2, 3, 4, 7, 8, 13, 14
-//   down (c_z = -1, pulled from plane z+1): 10, 12, 15, 17, 20, 21, 24, 26
-constexpr unsigned long long pack5(int a, int b, int c, int d, int e, int f, int g, int h) {
-    return (unsigned long long)a | (unsigned long long)b << 5 | (unsigned long long)c << 10 |
-           (unsigned long long)d << 15 | (unsigned long long)e << 20 | (unsigned long long)f << 25 |
-           (unsigned long long)g << 30 | (unsigned long long)h << 35;
-}
-constexpr unsigned long long kUpBits = pack5(9, 11, 16, 18, 19, 22, 23, 25);
-constexpr unsigned long long kFlBits = pack5(1, 2, 3, 4, 7, 8, 13, 14);
-constexpr unsigned long long kDnBits = pack5(10, 12, 15, 17, 20, 21, 24, 26);
-__host__ __device__ constexpr int hUp(int j) { return (int)((kUpBits >> (5 * j)) & 31ull); }
-__host__ __device__ constexpr int hFl(int j) { return (int)((kFlBits >> (5 * j)) & 31ull); }
-__host__ __device__ constexpr int hDn(int j) { return (int)((kDnBits >> (5 * j)) & 31ull); }
-
-template <int TY>
+// A CTA owns a column of TILE_X x TY nodes and marches along z.
+//   owner warps (one per row): lane l owns the nodes x0 + 2 l and x0 + 2 l + 1;
+//   halo warps (every NH-th plane each): issue the bulk copies of a plane's rows (own columns, rows
+//     y0 - 1 .. y0 + TY) into a ring of D plane stages, and evaluate the x-pass values that enter the
+//     tile from the columns x0 - 1 and x0 + TILE_X (one lane per row and side), up to D planes
+//     ahead of the owners.
+// A stage is full when its copies have landed and its halo values are written (mbarrier full[s]: the
+// copies' bytes and one arrival) and free again when every owner warp has read it (empty[s], one
+// arrival per owner warp); owners drift apart freely within the ring.  The sequence of stages runs on
+// from one work item to the next, so there is no drain between items.
+template <typename S, int TY, bool SPECIAL>
 struct Geo {
-    static constexpr int NOWN = TILE_X * TY;    // owner threads: one per column, one warp per row
-    static constexpr int NR = 2 * TILE_X + 2 * TY + 4;  // rim columns
-    static constexpr int NRW = (NR + 31) / 32;  // dedicated rim warps
-    static constexpr int NTH = NOWN + 32 * NRW;
-    static constexpr int W = TILE_X + 2;        // shared-memory row pitch (column + rim)
-    static constexpr int NCOL = W * (TY + 2);   // columns incl. rim
-    static constexpr int PLANE = 8 * NCOL;      // floats of one 8-population plane buffer
-    static constexpr int NUP = 4, NFL = 3, NDN = 2;  // ring depths (rim warps run one plane ahead)
-    static constexpr int SMEM = (NUP + NFL + NDN) * PLANE * 4;
+    static constexpr int WPN = StorageLayout<S>::words;      // 32-bit words of one node
+    static constexpr int ROWW = 2 * WPN * kXBlock;           // words of one row (two x-blocks)
+    static constexpr int SIDEC = 2 * (TY + 2);               // columns beside the tile, corners included
+    static constexpr int MARKW = SPECIAL ? TY * TILE_X / 4 : 0;  // node marks of the plane, a byte each
+    static constexpr int STAGEW = (TY + 2) * ROWW + SIDEC * WPN + MARKW;  // words of one plane stage
+    // Stages, and class sums parked in shared memory between planes (all nine class sums and the c_z = +1
+    // class do not fit the owners' 104 registers).  Shared memory and L1 share 256 KB, and the owners'
+    // stores and remaining spills need L1: FP32 256^3 takes 240 us with 3 stages and 3 parked sums (164 KB,
+    // 92 KB of L1), 254 us with 6 parked, 285 us with 4 stages (28 KB of L1: 336 us).
+    static constexpr int D = TY == 16 ? (WPN == 10 ? 3 : (WPN == 7 ? 4 : 5)) : (WPN == 10 ? 4 : (WPN == 7 ? 5 : 6));
+    static constexpr int PARK = TY != 16 ? 0 : (WPN == 10 ? 3 : 6);
+    static constexpr int HALO = 9;                           // floats per row and side: c_y x c_z
+    static constexpr int NH = TY / 4;                        // halo warps
+    static constexpr int NTH = 32 * (TY + NH);
+    // 20 warps share 16,384 registers per scheduler: 96 each at launch (640 x 96 = 61,440), then 104 for the
+    // four warpgroups of owners and 64 for the halo warps (512 x 104 + 128 x 64 = 61,440)
+    static constexpr bool SPLIT = TY == 16;
     static constexpr int MINB = TY == 4 ? 3 : (TY == 8 ? 2 : 1);  // resident CTAs per SM targeted
+    static constexpr int SMEM = D * (STAGEW * 4 + 2 * TY * HALO * 4 + 3 * 8 + 16) + PARK * 32 * TY * 8;
+    static_assert(2 * TY <= 32, "one halo lane per row and side");
+    static_assert(STAGEW % 4 == 0 && ROWW % 4 == 0 && (SIDEC * WPN) % 4 == 0 && (2 * TY * HALO) % 4 == 0 && MARKW % 4 == 0,
+                  "bulk copies and 16-byte accesses on 16-byte boundaries");
 };
 
-constexpr bool need_dir(int q, int rcx, int rcy) {
-    return (rcx == 0 || cxq(q) == rcx) && (rcy == 0 || cyq(q) == rcy);
+// Constants of the rebuild for stored u s_u, m s_m, (rho - rho0) s_r.
+struct RebuildK {
+    float rho0, ir;             // 1 / s_r
+    float h3, h15, h45, h9;     // Hermite factors 3 / s_u, 1.5 / s_m, 4.5 / s_m, 9 / s_m
+};
+template <typename S>
+__device__ __forceinline__ RebuildK rebuild_k(float rho0, const StorageScale &sc) {
+    if constexpr (std::is_same<S, float>::value) return {rho0, 1.0f, 3.0f, 1.5f, 4.5f, 9.0f};
+    else
+        return {rho0, sc.is[0], __fmul_rn(3.0f, sc.is[1]), __fmul_rn(1.5f, sc.is[2]), __fmul_rn(4.5f, sc.is[2]),
+                __fmul_rn(9.0f, sc.is[2])};
 }
 
-// Rebuild the populations of one rim column and store the ones the tile pulls from it
-// (rcx, rcy: the c_x / c_y a population must have to enter the tile from this rim side).
-template <typename S, int RCX, int RCY, int TY>
-__device__ __forceinline__ void rim_store(const Raw<S> &raw, float rho0, const StorageScale &sc, float *up,
-                                          float *fl, float *dn, int col) {
-    constexpr int NC = Geo<TY>::NCOL;
-    float f[27];
-    rebuild<S>(raw, rho0, sc, f);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        if (need_dir(hUp(j), RCX, RCY)) up[j * NC + col] = f[hUp(j)];
-        if (need_dir(hFl(j), RCX, RCY)) fl[j * NC + col] = f[hFl(j)];
-        if (need_dir(hDn(j), RCX, RCY)) dn[j * NC + col] = f[hDn(j)];
+// Ten stored values of one node (float) or of the two nodes of a lane (V2).
+template <typename T>
+struct Stored {
+    T r, ux, uy, uz, mxx, myy, mzz, mxy, mxz, myz;
+};
+
+__host__ __device__ constexpr int direction(int cx, int cy, int cz) {
+    for (int q = 0; q < 27; ++q)
+        if (cxq(q) == cx && cyq(q) == cy && czq(q) == cz) return q;
+    return -1;
+}
+
+// The sign bits of both lanes.
+__device__ __forceinline__ float negated(float a) { return -a; }
+__device__ __forceinline__ V2 negated(V2 a) { return V2{a.v ^ 0x8000000080000000ull}; }
+
+// Populations of one node (float) or of a lane's two (V2) from the stored moments: reconstruct_h of
+// lbm_device.cuh, operation by operation, in units of their weight class.  The weights are 16, 4, 1 and
+// 1/4 times w = 1/54 (as floats too), and a power of two commutes with every rounding, so
+//   f[0] / 16, f[1..6] / 4, f[7..18], 4 f[19..26]
+// all come from r = w rho; the sums below put the factors back.  The caller's unused populations fold
+// away.
+static_assert(kW0 == 16.0f * kW2 && kW1 == 4.0f * kW2 && 4.0f * kW3 == kW2, "weights are powers of two apart");
+template <typename S, typename T>
+__device__ __forceinline__ void rebuild_scaled(const Stored<T> &m, const RebuildK &k, T f[27]) {
+    const T rho = kScaled<S> ? fma(m.r, bc<T>(k.ir), bc<T>(k.rho0)) : add(bc<T>(k.rho0), m.r);
+    const T t = add(add(m.mxx, m.myy), m.mzz);
+    const T h45 = bc<T>(k.h45);
+    const T p0 = fma(bc<T>(-k.h15), t, bc<T>(1.0f));
+    const T ax = fma(h45, m.mxx, p0), ay = fma(h45, m.myy, p0);
+    const T r = mul(rho, bc<T>(kW2)), q = mul(bc<T>(k.h3), r), n = mul(bc<T>(k.h9), r);
+    const T nq = negated(q), nn = negated(n);
+    f[0] = mul(r, p0);
+    {
+        const T ex = mul(r, ax), ey = mul(r, ay), ez = mul(r, fma(h45, m.mzz, p0));
+        f[1] = fma(q, m.ux, ex);
+        f[2] = fma(nq, m.ux, ex);
+        f[3] = fma(q, m.uy, ey);
+        f[4] = fma(nq, m.uy, ey);
+        f[5] = fma(q, m.uz, ez);
+        f[6] = fma(nq, m.uz, ez);
+    }
+    const T upp = add(m.ux, m.uy), upm = sub(m.ux, m.uy);
+    {
+        const T b = mul(r, fma(h45, m.myy, ax));
+        const T cp = fma(n, m.mxy, b), cm = fma(nn, m.mxy, b);
+        f[7] = fma(q, upp, cp);
+        f[8] = fma(nq, upp, cp);
+        f[13] = fma(q, upm, cm);
+        f[14] = fma(nq, upm, cm);
+    }
+    {
+        const T b = mul(r, fma(h45, m.mzz, ax));
+        const T cp = fma(n, m.mxz, b), cm = fma(nn, m.mxz, b);
+        const T sp = add(m.ux, m.uz), sm = sub(m.ux, m.uz);
+        f[9] = fma(q, sp, cp);
+        f[10] = fma(nq, sp, cp);
+        f[15] = fma(q, sm, cm);
+        f[16] = fma(nq, sm, cm);
+    }
+    {
+        const T b = mul(r, fma(h45, m.mzz, ay));
+        const T cp = fma(n, m.myz, b), cm = fma(nn, m.myz, b);
+        const T sp = add(m.uy, m.uz), sm = sub(m.uy, m.uz);
+        f[11] = fma(q, sp, cp);
+        f[12] = fma(nq, sp, cp);
+        f[17] = fma(q, sm, cm);
+        f[18] = fma(nq, sm, cm);
+    }
+    {
+        const T c0 = mul(r, fma(h45, t, p0));
+        const T a = add(m.mxy, m.mxz), b = sub(m.mxy, m.mxz);
+        const T e1 = fma(n, add(a, m.myz), c0), e2 = fma(n, sub(b, m.myz), c0);
+        const T e3 = fma(nn, add(b, m.myz), c0), e4 = fma(nn, sub(a, m.myz), c0);
+        const T u1 = add(upp, m.uz), u2 = sub(upp, m.uz), u3 = add(upm, m.uz), u4 = sub(upm, m.uz);
+        f[19] = fma(q, u1, e1);
+        f[20] = fma(nq, u1, e1);
+        f[21] = fma(q, u2, e2);
+        f[22] = fma(nq, u2, e2);
+        f[23] = fma(q, u3, e3);
+        f[24] = fma(nq, u3, e3);
+        f[26] = fma(q, u4, e4);
+        f[25] = fma(nq, u4, e4);
     }
 }
 
-// Pulled population q of the owner node, read from the ring buffer of its c_z class.
-template <int Q, int TY>
-__device__ __forceinline__ float pull(const float *up, const float *fl, const float *dn, int col) {
-    constexpr int NC = Geo<TY>::NCOL, W = Geo<TY>::W;
-    constexpr int off = -cyq(Q) * W - cxq(Q);
-    if constexpr (czq(Q) == 1) {
-        constexpr int j = Q == 9 ? 0 : Q == 11 ? 1 : Q == 16 ? 2 : Q == 18 ? 3 : Q == 19 ? 4 : Q == 22 ? 5 : Q == 23 ? 6 : 7;
-        return up[j * NC + col + off];
-    } else if constexpr (czq(Q) == 0) {
-        constexpr int j = Q == 1 ? 0 : Q == 2 ? 1 : Q == 3 ? 2 : Q == 4 ? 3 : Q == 7 ? 4 : Q == 8 ? 5 : Q == 13 ? 6 : 7;
-        return fl[j * NC + col + off];
+// Stored values of the lane's two nodes from a row in shared memory (`p`: the lane's first word).
+template <typename S>
+__device__ __forceinline__ Stored<V2> load_pair(const uint32_t *p) {
+    Stored<V2> m;
+    if constexpr (std::is_same<S, float>::value) {
+        V2 w[10];
+#pragma unroll
+        for (int f = 0; f < 10; ++f) w[f].v = *reinterpret_cast<const unsigned long long *>(p + f * kXBlock);
+        m = {w[0], w[1], w[2], w[3], w[4], w[5], w[6], w[7], w[8], w[9]};
+    } else if constexpr (kHybrid<S>) {
+        V2 u[3];
+#pragma unroll
+        for (int f = 0; f < 3; ++f) u[f].v = *reinterpret_cast<const unsigned long long *>(p + f * kXBlock);
+        float2 a[4], b[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint2 w = *reinterpret_cast<const uint2 *>(p + (3 + j) * kXBlock);
+            a[j] = pair_to_f<__half>(w.x);
+            b[j] = pair_to_f<__half>(w.y);
+        }
+        m = {v2(a[0].x, b[0].x), u[0], u[1], u[2], v2(a[0].y, b[0].y), v2(a[1].x, b[1].x), v2(a[1].y, b[1].y),
+             v2(a[2].x, b[2].x), v2(a[2].y, b[2].y), v2(a[3].x, b[3].x)};
     } else {
-        constexpr int j = Q == 10 ? 0 : Q == 12 ? 1 : Q == 15 ? 2 : Q == 17 ? 3 : Q == 20 ? 4 : Q == 21 ? 5 : Q == 24 ? 6 : 7;
-        return dn[j * NC + col + off];
+        float2 a[5], b[5];
+#pragma unroll
+        for (int j = 0; j < 5; ++j) {
+            const uint2 w = *reinterpret_cast<const uint2 *>(p + j * kXBlock);
+            a[j] = pair_to_f<S>(w.x);
+            b[j] = pair_to_f<S>(w.y);
+        }
+        m = {v2(a[0].x, b[0].x), v2(a[0].y, b[0].y), v2(a[1].x, b[1].x), v2(a[1].y, b[1].y), v2(a[2].x, b[2].x),
+             v2(a[2].y, b[2].y), v2(a[3].x, b[3].x), v2(a[3].y, b[3].y), v2(a[4].x, b[4].x), v2(a[4].y, b[4].y)};
     }
+    return m;
 }
 
-// Zeroth, first and second (c_x, c_y) sums of the 3 x 3 populations of one c_z class, from
-// row sums (by c_y) and column sums (by c_x): 19 additions instead of one per term.
+// Stored values of one side column (words SIDEC apart).
+template <typename S, int SIDEC>
+__device__ __forceinline__ Stored<float> side_values(const uint32_t *p) {
+    Raw<S> raw;
+    load_raw_words<S, SIDEC>(p, raw);
+    float v[10];
+    raw_values<S>(raw, v);
+    return {v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], v[8], v[9]};
+}
+
+// Sums of one c_z class over (c_x, c_y): orders 1, c_x, c_y, c_x^2, c_y^2, c_x c_y (the classes c_z = +-1
+// times 4: their populations are in units of a quarter).
 struct ClassSums {
-    float s0, sx, sy, sxx, syy, sxy;
+    V2 s0, sx, sy, sxx, syy, sxy;
 };
-__device__ __forceinline__ ClassSums class_sums(float mm, float m0, float mp, float zm, float zz, float zp, float pm,
-                                                float p0, float pp) {
-    // arguments: f(c_x, c_y) with m = -1, z = 0, p = +1, named <c_x><c_y>
-    const float rp = (mp + zp) + pp, r0 = (m0 + zz) + p0, rm = (mm + zm) + pm;  // by c_y = +1, 0, -1
-    const float cp = (pm + p0) + pp, cm = (mm + m0) + mp;                       // by c_x = +1, -1
-    ClassSums s;
-    s.s0 = (rp + r0) + rm;
-    s.sx = cp - cm;
-    s.sxx = cp + cm;
-    s.sy = rp - rm;
-    s.syy = rp + rm;
-    s.sxy = (pp + mm) - (pm + mp);
-    return s;
-}
 
-// Packed FP32 (sm_100+ add / sub .rn.f32x2): one instruction, two independently IEEE-rounded
-// lanes, so a packed sum gives bit for bit the two scalar sums.
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
-    unsigned long long ra, rb, rd;
-    memcpy(&ra, &a, 8);
-    memcpy(&rb, &b, 8);
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(rd) : "l"(ra), "l"(rb));
-    float2 d;
-    memcpy(&d, &rd, 8);
-    return d;
-}
-
-// class_sums of two classes at once (lane x, lane y), the same operations in the same order
-struct ClassSums2 {
-    float2 s0, sx, sy, sxx, syy, sxy;
+// Post-stream moments of a lane's two nodes: rho - rho0, and u, m with their storage scales.
+struct Pair {
+    V2 r, ux, uy, uz, mxx, myy, mzz, mxy, mxz, myz;
 };
-__device__ __forceinline__ ClassSums2 class_sums2(float2 mm, float2 m0, float2 mp, float2 zm, float2 zz, float2 zp,
-                                                  float2 pm, float2 p0, float2 pp) {
-    const float2 rp = add2(add2(mp, zp), pp), r0 = add2(add2(m0, zz), p0), rm = add2(add2(mm, zm), pm);
-    const float2 cp = add2(add2(pm, p0), pp), cm = add2(add2(mm, m0), mp);
-    ClassSums2 s;
-    s.s0 = add2(add2(rp, r0), rm);
-    s.sx = sub2(cp, cm);
-    s.sxx = add2(cp, cm);
-    s.sy = sub2(rp, rm);
-    s.syy = add2(rp, rm);
-    s.sxy = sub2(add2(pp, mm), add2(pm, mp));
-    return s;
+
+struct Node {
+    float r, ux, uy, uz, mxx, myy, mzz, mxy, mxz, myz;
+};
+__device__ __forceinline__ Node node_of(const Pair &p, int c) {
+    return c == 0 ? Node{lo(p.r), lo(p.ux), lo(p.uy), lo(p.uz), lo(p.mxx), lo(p.myy), lo(p.mzz), lo(p.mxy), lo(p.mxz), lo(p.myz)}
+                  : Node{hi(p.r), hi(p.ux), hi(p.uy), hi(p.uz), hi(p.mxx), hi(p.myy), hi(p.mzz), hi(p.mxy), hi(p.mxz), hi(p.myz)};
 }
 
-// Gather the pulled populations of the owner node and evaluate its moments on the fly,
-// class by class (c_z = +1 from plane z-1, 0 from z, -1 from z+1); the c_z = +1 and c_z = 0
-// classes share packed sums (lane x: +1, lane y: 0).
-// SCALED: u and the second moments come out multiplied by the storage scales su and sm.
-template <int TY, bool SCALED = false>
-__device__ __forceinline__ void gather_evaluate(const float *up, const float *fl, const float *dn, int col, float f0,
-                                                float f5, float f6, Mom &m, float su = 1.0f, float sm = 1.0f) {
-#define MRLBM_P(q) pull<q, TY>(up, fl, dn, col)
-#define MRLBM_P2(a, b) make_float2(MRLBM_P(a), MRLBM_P(b))
-    // (c_x, c_y) = (-1,-1), (-1,0), (-1,1), (0,-1), (0,0), (0,1), (1,-1), (1,0), (1,1):
-    // c_z = +1: 22, 16, 25, 18, 5, 11, 23, 9, 19;  c_z = 0: 8, 2, 14, 4, 0, 3, 13, 1, 7
-    const ClassSums2 uc = class_sums2(MRLBM_P2(22, 8), MRLBM_P2(16, 2), MRLBM_P2(25, 14), MRLBM_P2(18, 4),
-                                      make_float2(f5, f0), MRLBM_P2(11, 3), MRLBM_P2(23, 13), MRLBM_P2(9, 1),
-                                      MRLBM_P2(19, 7));
-    // c_z = -1: 20, 10, 24, 12, 6, 17, 26, 15, 21
-    const ClassSums d = class_sums(MRLBM_P(20), MRLBM_P(10), MRLBM_P(24), MRLBM_P(12), f6, MRLBM_P(17), MRLBM_P(26),
-                                   MRLBM_P(15), MRLBM_P(21));
-#undef MRLBM_P2
-#undef MRLBM_P
-    const float rho = (uc.s0.x + uc.s0.y) + d.s0;
-    const float inv = __frcp_rn(rho);  // correctly rounded, as 1.0f / rho
-    const float iu = SCALED ? __fmul_rn(inv, su) : inv, im = SCALED ? __fmul_rn(inv, sm) : inv;
-    const float cs = SCALED ? __fmul_rn(-kCs2, sm) : -kCs2;
-    m.rho = rho;
-    m.ux = ((uc.sx.x + uc.sx.y) + d.sx) * iu;
-    m.uy = ((uc.sy.x + uc.sy.y) + d.sy) * iu;
-    m.uz = (uc.s0.x - d.s0) * iu;
-    m.mxx = __fmaf_rn((uc.sxx.x + uc.sxx.y) + d.sxx, im, cs);
-    m.myy = __fmaf_rn((uc.syy.x + uc.syy.y) + d.syy, im, cs);
-    m.mzz = __fmaf_rn(uc.s0.x + d.s0, im, cs);
-    m.mxy = ((uc.sxy.x + uc.sxy.y) + d.sxy) * im;
-    m.mxz = (uc.sx.x - d.sx) * im;
-    m.myz = (uc.sy.x - d.sy) * im;
+// m_ab <- (1 - omega) m_ab + omega u_a u_b on scaled moments (collide_h on two nodes).
+__device__ __forceinline__ void collide_pair(Pair &m, float omega, float omega_u) {
+    const V2 om1 = bc<V2>(1.0f - omega), ou = bc<V2>(omega_u);
+    const V2 wx = mul(ou, m.ux), wy = mul(ou, m.uy), wz = mul(ou, m.uz);
+    m.mxx = fma(wx, m.ux, mul(om1, m.mxx));
+    m.myy = fma(wy, m.uy, mul(om1, m.myy));
+    m.mzz = fma(wz, m.uz, mul(om1, m.mzz));
+    m.mxy = fma(wx, m.uy, mul(om1, m.mxy));
+    m.mxz = fma(wx, m.uz, mul(om1, m.mxz));
+    m.myz = fma(wy, m.uz, mul(om1, m.myz));
 }
 
-template <int TY>
-__device__ __forceinline__ void gather_all(const float *up, const float *fl, const float *dn, int col, float f0,
-                                           float f5, float f6, float *f) {
-    f[0] = f0;
-    f[5] = f5;
-    f[6] = f6;
+// The stored words of one node (r: rho - rho0, u and m already scaled); key: random bits of a
+// stochastically rounded store.
+template <typename S, bool SR>
+__device__ __forceinline__ void node_words(const Node &m, float sr, uint32_t key, uint32_t w[]) {
+    if constexpr (std::is_same<S, float>::value) {
+        const float v[10] = {m.r, m.ux, m.uy, m.uz, m.mxx, m.myy, m.mzz, m.mxy, m.mxz, m.myz};
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        f[hUp(j)] = up[j * Geo<TY>::NCOL + col - cyq(hUp(j)) * Geo<TY>::W - cxq(hUp(j))];
-        f[hFl(j)] = fl[j * Geo<TY>::NCOL + col - cyq(hFl(j)) * Geo<TY>::W - cxq(hFl(j))];
-        f[hDn(j)] = dn[j * Geo<TY>::NCOL + col - cyq(hDn(j)) * Geo<TY>::W - cxq(hDn(j))];
+        for (int f = 0; f < 10; ++f) w[f] = __float_as_uint(v[f]);
+    } else {
+        const float r = m.r * sr;
+        if constexpr (kHybrid<S>) {
+            w[0] = __float_as_uint(m.ux);
+            w[1] = __float_as_uint(m.uy);
+            w[2] = __float_as_uint(m.uz);
+            w[3] = round_pair<__half, SR>(r, m.mxx, key, 0);
+            w[4] = round_pair<__half, SR>(m.myy, m.mzz, key, 1);
+            w[5] = round_pair<__half, SR>(m.mxy, m.mxz, key, 2);
+            w[6] = round_pair<__half, SR>(m.myz, 0.0f, key, 3);
+        } else {
+            w[0] = round_pair<S, SR>(r, m.ux, key, 0);
+            w[1] = round_pair<S, SR>(m.uy, m.uz, key, 1);
+            w[2] = round_pair<S, SR>(m.mxx, m.myy, key, 2);
+            w[3] = round_pair<S, SR>(m.mzz, m.mxy, key, 3);
+            w[4] = round_pair<S, SR>(m.mxz, m.myz, key, 4);
+        }
     }
 }
 
-// Rebuild the own-column populations of plane p from raw stored moments into the rings.
-template <typename S, int TY>
-__device__ __forceinline__ void arrive_own(const Raw<S> &raw, float rho0, const StorageScale &sc, float *up,
-                                           float *fl, float *dn, int col, float &c0, float &c5, float &c6) {
-    float f[27];
-    rebuild<S>(raw, rho0, sc, f);
+template <typename S, bool SR>
+__device__ __forceinline__ void store_pair(uint32_t *p, const Pair &m, float sr, uint32_t key0, uint32_t key1) {
+    constexpr int WPN = StorageLayout<S>::words;
+    uint32_t a[WPN], b[WPN];
+    node_words<S, SR>(node_of(m, 0), sr, key0, a);
+    node_words<S, SR>(node_of(m, 1), sr, key1, b);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        up[j * Geo<TY>::NCOL + col] = f[hUp(j)];
-        fl[j * Geo<TY>::NCOL + col] = f[hFl(j)];
-        dn[j * Geo<TY>::NCOL + col] = f[hDn(j)];
-    }
-    c0 = f[0];
-    c5 = f[5];
-    c6 = f[6];
+    for (int f = 0; f < WPN; ++f) *reinterpret_cast<uint2 *>(p + f * kXBlock) = make_uint2(a[f], b[f]);
 }
-
-template <typename S, int TY>
-__device__ __forceinline__ void arrive_rim(const Raw<S> &raw, float rho0, const StorageScale &sc, int side, float *up,
-                                           float *fl, float *dn, int rcol) {
-    switch (side) {
-        case 0: rim_store<S, 0, 1, TY>(raw, rho0, sc, up, fl, dn, rcol); break;
-        case 1: rim_store<S, 0, -1, TY>(raw, rho0, sc, up, fl, dn, rcol); break;
-        case 2: rim_store<S, 1, 0, TY>(raw, rho0, sc, up, fl, dn, rcol); break;
-        case 3: rim_store<S, -1, 0, TY>(raw, rho0, sc, up, fl, dn, rcol); break;
-        case 4: rim_store<S, 1, 1, TY>(raw, rho0, sc, up, fl, dn, rcol); break;
-        case 5: rim_store<S, -1, 1, TY>(raw, rho0, sc, up, fl, dn, rcol); break;
-        case 6: rim_store<S, 1, -1, TY>(raw, rho0, sc, up, fl, dn, rcol); break;
-        default: rim_store<S, -1, -1, TY>(raw, rho0, sc, up, fl, dn, rcol); break;
-    }
+template <typename S, bool SR>
+__device__ __forceinline__ void store_node(uint32_t *p, const Node &m, float sr, uint32_t key) {
+    constexpr int WPN = StorageLayout<S>::words;
+    uint32_t a[WPN];
+    node_words<S, SR>(m, sr, key, a);
+#pragma unroll
+    for (int f = 0; f < WPN; ++f) p[f * kXBlock] = a[f];
 }
 
 // Post-stream (pre-collision) moments of a wall-stencil node into its side-buffer entry, the
 // snapshot the wall kernel interpolates from (the node-list kernel writes the same for the
-// marked nodes it handles); iu / im undo the storage scales of the 16-bit emit.
-template <int TY>
-__device__ __forceinline__ void snapshot_t(float *side, int slot, int x, int y, int z, int x0, int y0, int nz,
-                                           const Mom &m, float rho0, float iu, float im) {
-    float *e = side + side_index(slot, x, y, z, x0, y0, nz, TILE_X, TY) * 16;
-    e[0] = m.rho - rho0;
-    e[1] = m.ux * iu; e[2] = m.uy * iu; e[3] = m.uz * iu;
-    e[4] = m.mxx * im; e[5] = m.myy * im; e[6] = m.mzz * im;
-    e[7] = m.mxy * im; e[8] = m.mxz * im; e[9] = m.myz * im;
+// marked nodes it handles); iu / im undo the storage scales.
+__device__ __forceinline__ void snapshot(float *e, const Node &m, float iu, float im) {
+    store_side(e, m.r, m.ux * iu, m.uy * iu, m.uz * iu, m.mxx * im, m.myy * im, m.mzz * im, m.mxy * im, m.mxz * im,
+               m.myz * im);
 }
 
-// Named CTA barriers (PTX bar.sync / bar.arrive; id 0 is __syncthreads).  A generation
-// completes when `n` threads (whole warps) have arrived; bar.arrive does not wait.
-__device__ __forceinline__ void nb_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
-__device__ __forceinline__ void nb_arrive(int id, int n) {
-    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
+// Storage word of node x = 32 xb (a block's first node) of row y, plane z.
+template <typename S>
+__device__ __forceinline__ int64_t row_word(int xb, int y, int z, int nxb, int ny) {
+    return ((((int64_t)z * ny + y) * nxb + xb) * StorageLayout<S>::words) * kXBlock;
 }
 
-// SPECIAL = false: every node of every item is a plain bulk node (no node words are read).
-// FULL = true: every tile is a whole 32 x TY tile (nx % 32 == 0, ny % TY == 0), so the
-// ragged-edge predicates fold away and the owner branches are warp-uniform.
-//
-// Warp roles and schedule per work item (planes indexed k = 0 .. L+1 from zs-1, L = ze-zs):
-//   owner warps (one per tile row):  rebuild own columns of plane k; for k >= 2 wait FULL(k),
-//       emit plane k-1 (reads up(k-2), flat(k-1), down(k)), then signal DONE(k) if a rim
-//       iteration k+2 will wait for it;
-//   rim warps:  for k >= 4 wait DONE(k-2); rebuild the rim columns of plane k; for k >= 2
-//       signal FULL(k).
-// Plane k's buffers live in ring slots up[k%4], flat[k%3], down[k%2]; their previous
-// occupants (plane k-4 / k-3 / k-2) are last read by the emit of iteration k-2, which both
-// roles wait for before writing (owners through FULL(k-1)).  FULL(k) / DONE(k) use barrier ids
-// 1 + (k&1) / 3 + (k&1); a role can run at most one generation ahead on an id, so
-// consecutive generations never mix.  Counts are always the whole CTA (owner arrivals +
-// rim arrivals), so the rim work of the next plane overlaps the owners' emit.
-template <typename S, int TY, bool SPECIAL, bool BATCH, bool FULL>
-__global__ void __launch_bounds__(Geo<TY>::NTH, Geo<TY>::MINB)
-    step_kernel(const StepArgs *__restrict__ ga, const BatchArgs *__restrict__ ba, const int parity,
+// SPECIAL = false: every node of every item is a plain bulk node (no node marks are read).
+template <typename S, int TY, bool SPECIAL, bool BATCH>
+__global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>::MINB)
+    step_kernel(const __grid_constant__ StepArgs single, const BatchArgs *__restrict__ ba, const int parity,
                 double *__restrict__ diag_part) {
-    using G = Geo<TY>;
-    extern __shared__ float smem[];
-    __shared__ double red[2][TY];
-    // per-case values: fixed for a single case, reloaded per work item in a batch
-    const S *__restrict__ src = nullptr;
-    S *__restrict__ dst = nullptr;
-    int nxb = 0, nx = 0, ny = 0, nz = 0, lz = 0, tiles_x = 0;
-    const int32_t *__restrict__ tile_slot = nullptr;
-    const uint32_t *__restrict__ word = nullptr;
-    float *__restrict__ popbuf = nullptr;
-    float *__restrict__ side = nullptr;  // wall-stencil snapshots of special tiles
-    int n_pop = 0;
-    const int32_t *__restrict__ row_base = nullptr;
-    float omega = 1.f, rho0 = 1.f;
-    StorageScale sc;
-    int64_t plane = 0, zst = 0;  // lexicographic plane (node words), storage elements per z plane
-    bool sr_on = false;          // stochastic rounding of 16-bit stores
-    uint32_t sr_seed = 0u;
-    float omega_u = 1.f;         // omega s_m / s_u^2: collision of scaled 16-bit moments
-    auto load_case = [&](const StepArgs *__restrict__ c) {
-        src = (const S *)c->m[parity];
-        dst = (S *)c->m[parity ^ 1];
-        nxb = c->nxb;
-        nx = c->nx;
-        ny = c->ny;
-        nz = c->nz;
-        lz = c->lz;
-        tiles_x = c->tiles_x;
-        tile_slot = c->tile_slot;
-        word = c->word;
-        popbuf = c->popbuf;
-        side = c->side;
-        n_pop = c->n_list_pop;
-        row_base = c->row_base;
-        omega = c->omega;
-        rho0 = c->rho0;
-        sc = c->sc;
-        plane = (int64_t)nx * ny;
-        zst = (int64_t)ny * nxb * StorageLayout<S>::per_node * kXBlock;
-        if constexpr (kScaled<S>) {
-            sr_on = c->sr_step != nullptr;
-            sr_seed = sr_on ? sr_step_seed(*c->sr_step) : 0u;
-            omega_u = c->omega * (c->sc.s[2] * (c->sc.is[1] * c->sc.is[1]));
+    using G = Geo<S, TY, SPECIAL>;
+    extern __shared__ __align__(128) unsigned char smem[];
+    uint32_t *const stages = reinterpret_cast<uint32_t *>(smem);
+    float *const halos = reinterpret_cast<float *>(smem + G::D * G::STAGEW * 4);
+    // {case, work item, its number} of the item that starts with the stage's plane
+    int4 *const heads = reinterpret_cast<int4 *>(smem + G::D * (G::STAGEW * 4 + 2 * TY * G::HALO * 4));
+    uint64_t *const full = reinterpret_cast<uint64_t *>(heads + G::D);
+    uint64_t *const empty = full + G::D;
+    uint64_t *const landed = empty + G::D;
+    V2 *const park = reinterpret_cast<V2 *>(landed + G::D) + threadIdx.x;  // owners: the thread's slots, 32 TY apart
+    __shared__ __align__(16) uint4 s_slot[2];  // answers to takeover requests, by item parity
+    __shared__ uint64_t s_taken;
+    __shared__ int s_next[2];
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < G::D; ++s) {
+            mbar_init(full + s, 1);
+            mbar_init(empty + s, TY);
+            mbar_init(landed + s, 1);
+        }
+        mbar_init(&s_taken, 1);
+        mbar_init_fence();
+    }
+    __syncthreads();
+    int stage = 0;
+    uint32_t phase = 0;
+    auto next_stage = [&]() {
+        if (++stage == G::D) {
+            stage = 0;
+            phase ^= 1u;
         }
     };
-    if constexpr (!BATCH) load_case(ga);
-    const int n_items = BATCH ? ba->n_items : ga->n_items;
-    const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
-    const bool owner = tid < G::NOWN;
-    const bool diag = diag_part != nullptr;
-    float *const up_base = smem;
-    float *const fl_base = smem + G::NUP * G::PLANE;
-    float *const dn_base = smem + (G::NUP + G::NFL) * G::PLANE;
-    double dmD = 0.0, deD = 0.0;
+    const int n_items = BATCH ? ba->n_items : single.n_items;
 
-    // Work items: the first gridDim.x go by block index, the rest are claimed on demand from
-    // a counter zeroed before every launch, so CTAs that finish early take more (no static
-    // last-wave imbalance).  Without a counter the CTAs stride through the list.
-    int *const work = BATCH ? ba->work_counter : ga->work_counter;
-    __shared__ int s_next;
-    for (int it = blockIdx.x; it < n_items;) {
-        int item;
-        if constexpr (BATCH) {
-            const int2 e = ba->items[it];
-            load_case(ba->cases[e.x]);
-            item = e.y;
-        } else {
-            item = ga->items[it];
-        }
-        const int tile = item & 0xFFFFF, seg = item >> 20;
-        const int tix = tile % tiles_x, tiy = tile / tiles_x;
-        const int x0 = tix * TILE_X, y0 = tiy * TY;
-        const int w = FULL ? TILE_X : min(TILE_X, nx - x0), h = FULL ? TY : min(TY, ny - y0);
-        const int zs = seg * lz, ze = min(zs + lz, nz);
-        const int last = ze - zs + 1;  // last plane index k
-        const int slot = (SPECIAL && tile_slot) ? tile_slot[tile] : -1;
-        const bool own = owner && (FULL || (tx < w && ty < h));
-        const int x = x0 + tx, y = y0 + ty;
-        const int col = (ty + 1) * G::W + (tx + 1);
-        // the column this thread loads and rebuilds: its own, or a rim column for rim warps
-        int rside = -1, ccol = col;
-        int64_t cxy = 0;
-        bool active = own;
-        if (own) {
-            cxy = aos_at<S>(x, y, 0, nxb, ny);
-        } else if (!owner) {
-            int rx, ry, sd;
-            const int r = tid - G::NOWN;
-            if (r < TILE_X) { rx = r; ry = -1; sd = 0; }
-            else if (r < 2 * TILE_X) { rx = r - TILE_X; ry = h; sd = 1; }
-            else if (r < 2 * TILE_X + TY) { rx = -1; ry = r - 2 * TILE_X; sd = 2; }
-            else if (r < 2 * TILE_X + 2 * TY) { rx = w; ry = r - 2 * TILE_X - TY; sd = 3; }
-            else if (r < G::NR) {
-                const int k = r - 2 * TILE_X - 2 * TY;
-                rx = (k & 1) ? w : -1;
-                ry = (k & 2) ? h : -1;
-                sd = 4 + k;
-            } else { rx = 0; ry = 0; sd = -1; }
-            const bool valid = sd >= 0 && ((sd == 0 || sd == 1) ? rx < w : ((sd == 2 || sd == 3) ? ry < h : true));
-            if (valid) {
-                rside = sd;
-                ccol = (ry + 1) * G::W + (rx + 1);
-                int gx = x0 + rx, gy = y0 + ry;
-                gx = gx < 0 ? gx + nx : (gx >= nx ? gx - nx : gx);
-                gy = gy < 0 ? gy + ny : (gy >= ny ? gy - ny : gy);
-                cxy = aos_at<S>(gx, gy, 0, nxb, ny);
-                active = true;
-            }
-        }
-
-        // raw moments of planes k (being rebuilt) and k+1 (in flight); the two buffers swap
-        // roles every plane, so the plane loops are unrolled by two
-        Raw<S> pa, pb;
-        const int zm = zs == 0 ? nz - 1 : zs - 1;
-        if (active) load_words<S>(src, cxy + (int64_t)zm * zst, pa);
-        int zn = zs;  // plane of the next prefetch (wrapped)
-        int64_t loff = cxy + (int64_t)zs * zst;  // its storage offset, advanced per plane
-        int64_t soff = loff;                      // storage offset of the next emitted plane
-        const int64_t wrap = (int64_t)nz * zst;
-        int k3 = 0, k4 = 0;  // k % 3, k % 4
-
-        if (owner) {
-            float c0 = 0.f, c5 = 0.f, c6 = 0.f;   // own-column rest / up / down populations of plane k
-            float p0 = 0.f, p5 = 0.f, pp5 = 0.f;  // f0(k-1), f5(k-1), f5(k-2)
-            float dm = 0.f, de = 0.f;
-            // special tiles: node word and list row base of the plane emitted two planes later,
-            // one queue slot per plane parity
-            uint32_t wqa = 0u, wqb = 0u;
-            int rqa = 0, rqb = 0;
-            const unsigned row_mask = w >= 32 ? 0xffffffffu : ((1u << w) - 1u);
-            // wq / rq: this parity's queue slot (the plane emitted now, refilled for k + 2); wo: the
-            // other slot, which holds the word of the plane rebuilt now
-            auto owner_plane = [&](const int k, const Raw<S> &cur, Raw<S> &nxt, uint32_t &wq, int &rq,
-                                   const uint32_t wo) {
-                float *up = up_base + k4 * G::PLANE;
-                float *flt = fl_base + k3 * G::PLANE;
-                float *dn = dn_base + (k & 1) * G::PLANE;
-                uint32_t wnew = 0u;
-                int rnew = 0;
-                if constexpr (SPECIAL) {
-                    if (slot >= 0 && own && k + 2 <= last) {
-                        const int zq = zs + k;
-                        wnew = word[(int64_t)x + (int64_t)nx * y + (int64_t)zq * plane];
-                        rnew = row_base[((int64_t)slot * nz + zq) * TY + ty];
-                    }
-                }
-                if (own) {
-                    if (k < last) {
-                        load_words<S>(src, loff, nxt);
-                        loff += zst;
-                        if (++zn == nz) {
-                            zn = 0;
-                            loff -= wrap;
-                        }
-                    }
-                    arrive_own<S, TY>(cur, rho0, sc, up, flt, dn, col, c0, c5, c6);
-                    if constexpr (SPECIAL) {
-                        // a solid node of an updated block in the plane rebuilt now (z = zs + k - 1,
-                        // one this segment emits) keeps its stored moments, collided (the reference
-                        // collides every node of an active block): finished here from the words
-                        // in registers, before the emit would need them reloaded
-                        if (k >= 1 && k < last && (wo & NW_CLASS_MASK) == C_SOLID && !(wo & NW_FROZEN)) {
-                            Mom m = decode_words<S>(cur, rho0, sc);
-                            const int zr = zs + k - 1;
-                            const int64_t ar = k >= 2 ? soff + zst : soff;  // soff: plane zs + k - 2
-                            if (wo & NW_STENCIL)
-                                snapshot_t<TY>(side, slot, x, y, zr, x0, y0, nz, m, rho0, 1.0f, 1.0f);
-                            collide(m, omega);
-                            if (kScaled<S> && sr_on)
-                                store_mom_sr<S>(dst, ar, m, rho0, sc, sr_key(sr_seed, x, y, zr, nx, ny));
-                            else
-                                store_mom<S>(dst, ar, m, rho0, sc);
-                        }
-                    }
-                }
-                if (k >= 2) {
-                    nb_sync(1 + (k & 1), G::NTH);  // FULL(k): plane k complete, emits of k-1 done
-                    const int z = zs + k - 2;      // emitted plane
-                    if (own) {
-                        const float *eup = up_base + (k4 >= 2 ? k4 - 2 : k4 + 2) * G::PLANE;  // plane k-2
-                        const float *efl = fl_base + (k3 >= 1 ? k3 - 1 : 2) * G::PLANE;       // plane k-1
-                        const int64_t ai = soff;
-                        uint32_t wd = 0u;
-                        bool exp = false;
-                        unsigned bal = 0u;
-                        if constexpr (SPECIAL) {
-                            if (slot >= 0) {
-                                wd = wq;
-                                // a plain fluid node whose only mark is the wall-stencil bit is
-                                // updated here, like any bulk node, plus its snapshot; every other
-                                // marked node goes to the node-list kernel
-                                exp = wd != 0u && wd != NW_STENCIL && !(wd & NW_FROZEN) &&
-                                      (wd & NW_CLASS_MASK) != C_SOLID;
-                                bal = __ballot_sync(row_mask, exp);
-                            }
-                        }
-                        const bool snap = SPECIAL && wd == NW_STENCIL;
-                        if (wd == 0u || snap) {
-                            Mom m;
-                            if constexpr (std::is_same<S, float>::value) {
-                                gather_evaluate<TY>(eup, efl, dn, col, p0, pp5, c6, m);
-                                if (snap) snapshot_t<TY>(side, slot, x, y, z, x0, y0, nz, m, rho0, 1.0f, 1.0f);
-                                if (diag) {
-                                    dm += m.rho - rho0;
-                                    de += 0.5f * (m.ux * m.ux + m.uy * m.uy + m.uz * m.uz);
-                                }
-                                collide(m, omega);
-                                store_mom<S>(dst, ai, m, rho0, sc);
-                            } else {
-                                // u and m come out with their storage scales: no unscaling on
-                                // the way in (rebuild) and no scaling on the way out
-                                gather_evaluate<TY, true>(eup, efl, dn, col, p0, pp5, c6, m, sc.s[1], sc.s[2]);
-                                if (snap) snapshot_t<TY>(side, slot, x, y, z, x0, y0, nz, m, rho0, sc.is[1], sc.is[2]);
-                                if (diag) {
-                                    dm += m.rho - rho0;
-                                    de += 0.5f * (m.ux * m.ux + m.uy * m.uy + m.uz * m.uz) * (sc.is[1] * sc.is[1]);
-                                }
-                                collide_h(m, omega, omega_u);
-                                if (sr_on)
-                                    store_scaled_sr<S>(dst, ai, m, rho0, sc, sr_key(sr_seed, x, y, z, nx, ny));
-                                else
-                                    store_scaled<S>(dst, ai, m, rho0, sc);
-                            }
-                        } else if (exp) {
-                            // non-bulk node: hand its pulled populations to the node-list kernel
-                            float fw[27];
-                            gather_all<TY>(eup, efl, dn, col, p0, pp5, c6, fw);
-                            float *pq = popbuf + (rq + __popc(bal & ((1u << tx) - 1u)));
-#pragma unroll
-                            for (int q = 0; q < 27; ++q) pq[(int64_t)q * n_pop] = fw[q];
-                        }
-                    }
-                    if (k + 2 <= last) nb_arrive(3 + (k & 1), G::NTH);  // DONE(k)
-                    soff += zst;
-                }
-                wq = wnew;
-                rq = rnew;
-                pp5 = p5;
-                p5 = c5;
-                p0 = c0;
-                k3 = k3 == 2 ? 0 : k3 + 1;
-                k4 = (k4 + 1) & 3;
+    if (warp >= TY) {
+        if constexpr (G::SPLIT) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+        // ---- halo warps ------------------------------------------------------------------------
+        bool ok = true;
+        const int hw = warp - TY;
+        int q = 0;        // planes so far, over all items: plane q is halo warp q % NH's
+        int n = 0;        // items so far
+        // Work items.  SPECIAL: one CTA per item is launched, and a CTA that finishes its item takes over
+        // one that has not started (tiles with boundary nodes and the cases of a batch cost unevenly).
+        // Otherwise the CTAs stride through the items.
+        const bool leader = threadIdx.x == 32 * TY;
+        for (int it = blockIdx.x; it >= 0 && it < n_items;) {
+            if (SPECIAL && leader) takeover_request(s_slot + (n & 1), &s_taken);
+            int2 head;
+            if constexpr (BATCH) head = ba->items[it];
+            else head = make_int2(0, single.items ? single.items[it] : (it % (single.tiles_x * single.tiles_y)) |
+                                                                       ((it / (single.tiles_x * single.tiles_y)) << 20));
+            const StepArgs &a = BATCH ? *ba->cases[head.x] : single;
+            const int nx = a.nx, ny = a.ny, nz = a.nz, nxb = a.nxb;
+            const uint32_t *__restrict__ src = reinterpret_cast<const uint32_t *>(a.m[parity]);
+            const RebuildK K = rebuild_k<S>(a.rho0, a.sc);
+            const int tile = head.y & 0xFFFFF, seg = head.y >> 20;
+            const int tix = tile % a.tiles_x, tiy = tile / a.tiles_x;
+            const int x0 = tix * TILE_X, y0 = tiy * TY;
+            const int w = min(TILE_X, nx - x0), h = min(TY, ny - y0);
+            const int zs = seg * a.lz, ze = min(zs + a.lz, nz), last = ze - zs + 1;
+            const int64_t zst = (int64_t)ny * nxb * G::WPN * kXBlock;
+            auto wrap = [](int v, int n) { return v < 0 ? v + n : (v >= n ? v - n : v); };
+            // rows of the bulk copies: lane r copies row y0 - 1 + r
+            const uint32_t row_bytes = (uint32_t)min(2, nxb - 2 * tix) * G::WPN * kXBlock * 4;
+            const bool copies = lane < h + 2;
+            const int64_t copy_off = copies ? row_word<S>(2 * tix, wrap(y0 - 1 + lane, ny), 0, nxb, ny) : 0;
+            // node marks of the planes that this segment updates (row by row)
+            const uint32_t mark_pitch = (uint32_t)a.tiles_x * TILE_X;
+            const uint8_t *marks = SPECIAL && lane < h && a.tile_slot && a.tile_slot[tile] >= 0
+                                       ? a.mark + ((int64_t)zs * ny + y0 + lane) * mark_pitch + x0
+                                       : nullptr;
+            const bool tile_marked = SPECIAL && __shfl_sync(0xffffffffu, marks != nullptr, 0);
+            auto marked = [&](int k) { return tile_marked && k >= 1 && k < last; };
+            // columns beside the tile: column c = side * (TY + 2) + row + 1 is
+            // x0 - 1 (side 0, entering with c_x = +1) or x0 + w (side 1), rows -1 .. h; lane c fetches
+            // column c, and the columns past the 32nd are spread over the lanes
+            auto side_column = [&](int c) {
+                const int sd = c / (TY + 2), r = c - sd * (TY + 2) - 1;
+                if (sd > 1 || r > h) return (int64_t)-1;
+                const int gx = wrap(sd ? x0 + w : x0 - 1, nx);
+                return row_word<S>(gx >> 5, wrap(y0 + r, ny), 0, nxb, ny) + (gx & 31);
             };
-            for (int k = 0; k <= last; k += 2) {
-                owner_plane(k, pa, pb, wqa, rqa, wqb);
-                if (k + 1 <= last) owner_plane(k + 1, pb, pa, wqb, rqb, wqa);
-            }
-            if (diag) {
-                dmD += (double)dm;
-                deD += (double)de;
-            }
-        } else {
-            auto rim_plane = [&](const int k, const Raw<S> &cur, Raw<S> &nxt) {
-                if (k >= 4) nb_sync(3 + (k & 1), G::NTH);  // DONE(k-2): ring slots of plane k are free
+            const int64_t col_off = side_column(lane);
+            constexpr int EXTRA = G::SIDEC > 32 ? G::SIDEC - 32 : 0;  // 4 for 16 rows
+            constexpr int NE = EXTRA ? EXTRA : 1, PER = 32 / NE;  // words of such a column fetched per round
+            const int64_t ext_off = EXTRA ? side_column(32 + lane % NE) : -1;
+            const int side = lane / TY, row = lane - side * TY;  // the column this lane evaluates
+            const bool active = side < 2 && row < h;
+            const int mine = (hw + G::NH - q % G::NH) % G::NH;  // this warp's first plane of the item
+            int zk = (zs == 0 ? nz - 1 : zs - 1) + mine;
+            if (zk >= nz) zk -= nz;
+            for (int k = 0; k <= last; ++k, ++q, next_stage()) {
+                if ((k - mine) % G::NH != 0) continue;
+                // The halo warps wait for a free stage in turn, each asleep at a hardware barrier until the one
+                // before it has passed (polling costs issue slots).  Plane q waits for the release of plane
+                // q - D; the turn before has seen that of q - 1 - D, so the release two uses back on the stage
+                // is past, which the one parity bit of the wait could not tell from the last one.
+                if (G::NH > 1 && q > 0) token_wait(3 + hw);
+                if (ok) ok = mbar_wait(empty + stage, phase ^ 1u);
+                if (G::NH > 1) token_pass(3 + (hw + 1) % G::NH);
+                if (!ok) continue;
+                uint32_t *const sp = stages + stage * G::STAGEW;
+                uint32_t *const cp = sp + (TY + 2) * G::ROWW;  // [word][column]
+                if (lane == 0) {
+                    if (k == 0) heads[stage] = make_int4(head.x, head.y, it, 0);
+                    mbar_expect_tx(landed + stage, row_bytes * (h + 2) + (marked(k) ? TILE_X * (uint32_t)h : 0u));
+                    mbar_arrive(landed + stage);
+                }
+                __syncwarp();
+                const uint32_t *const zsrc = src + zk * zst;
+                if (copies) bulk_load(sp + lane * G::ROWW, zsrc + copy_off, row_bytes, landed + stage);
+                if (marked(k) && lane < h)
+                    bulk_load(cp + G::SIDEC * G::WPN + lane * (TILE_X / 4), marks + (int64_t)(k - 1) * ny * mark_pitch, TILE_X,
+                              landed + stage);
+                // (not through L1: a line per word would push out what the owners spill)
+                uint32_t w0[G::WPN], w1[(G::WPN + PER - 1) / PER];
+                if (col_off >= 0) {
+#pragma unroll
+                    for (int f = 0; f < G::WPN; ++f) w0[f] = load_uncached(zsrc + col_off + f * kXBlock);
+                }
+                if (EXTRA && ext_off >= 0) {
+#pragma unroll
+                    for (int i = 0; i < (G::WPN + PER - 1) / PER; ++i) {
+                        const int f = i * PER + lane / NE;
+                        if (f < G::WPN) w1[i] = load_uncached(zsrc + ext_off + f * kXBlock);
+                    }
+                }
+                if (col_off >= 0) {
+#pragma unroll
+                    for (int f = 0; f < G::WPN; ++f) cp[f * G::SIDEC + lane] = w0[f];
+                }
+                if (EXTRA && ext_off >= 0) {
+#pragma unroll
+                    for (int i = 0; i < (G::WPN + PER - 1) / PER; ++i) {
+                        const int f = i * PER + lane / NE;
+                        if (f < G::WPN) cp[f * G::SIDEC + 32 + lane % NE] = w1[i];
+                    }
+                }
+                __syncwarp();
+                zk += G::NH;
+                while (zk >= nz) zk -= nz;
                 if (active) {
-                    if (k < last) {
-                        load_words<S>(src, loff, nxt);
-                        loff += zst;
-                        if (++zn == nz) {
-                            zn = 0;
-                            loff -= wrap;
+                    float *e = halos + ((stage * 2 + side) * TY + row) * G::HALO;
+#pragma unroll
+                    for (int cy = -1; cy <= 1; ++cy) {
+                        float f[27];
+                        rebuild_scaled<S>(side_values<S, G::SIDEC>(cp + side * (TY + 2) + row + 1 - cy), K, f);
+#pragma unroll
+                        for (int cz = -1; cz <= 1; ++cz)
+                            e[3 * (cy + 1) + cz + 1] = side ? f[direction(-1, cy, cz)] : f[direction(1, cy, cz)];
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(full + stage);
+            }
+            if constexpr (SPECIAL) {
+                // one answer for all halo warps (two slots: the next one is written a barrier after the
+                // last read of this one)
+                if (leader) {
+                    const bool answered = mbar_wait(&s_taken, n & 1);
+                    s_next[n & 1] = answered ? takeover_result(s_slot + (n & 1)) : -1;
+                    ok = ok && answered;
+                }
+                asm volatile("bar.sync 2, %0;" ::"r"(32 * G::NH) : "memory");
+                it = s_next[n & 1];
+                ++n;
+            } else {
+                it += (int)gridDim.x;
+            }
+        }
+        if (q % G::NH == hw) {
+            if (G::NH > 1 && q > 0) token_wait(3 + hw);
+            if (ok) ok = mbar_wait(empty + stage, phase ^ 1u);
+            if (ok && lane == 0) {
+                heads[stage] = make_int4(0, -1, 0, 0);  // end mark
+                mbar_arrive(landed + stage);
+                mbar_arrive(full + stage);
+            }
+        }
+        if (!ok && lane == 0) {
+            // a wait ran out: report, and leave only when the copies in flight have landed (a stage
+            // that was never issued just runs into the wait's limit)
+            atomicOr(BATCH ? ba->cases[0]->error : single.error, kErrorWait);
+            for (int s = 0; s < G::D; ++s)
+                if (!mbar_wait(landed + s, 0)) mbar_wait(landed + s, 1);
+        }
+    } else {
+        if constexpr (G::SPLIT) asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+        // ---- owner warps -----------------------------------------------------------------------
+        bool ok = true;
+        int items = 0;
+        while (ok) {
+            // landed before full, here and in every plane: rows past the tile's last one skip the waits on
+            // full, and only the landing of a stage (its refill follows the release of its last use) makes
+            // the one parity bit of that wait unambiguous
+            ok = mbar_wait(landed + stage, phase) && mbar_wait(full + stage, phase);
+            if (!ok) break;
+            const int4 head = heads[stage];
+            if (head.y < 0) break;
+            const StepArgs &a = BATCH ? *ba->cases[head.x] : single;
+            const int nx = a.nx, ny = a.ny, nxb = a.nxb;
+            const RebuildK K = rebuild_k<S>(a.rho0, a.sc);
+            const int tile = head.y & 0xFFFFF, seg = head.y >> 20;
+            const int tix = tile % a.tiles_x, tiy = tile / a.tiles_x;
+            const int x0 = tix * TILE_X, y0 = tiy * TY;
+            const int w = min(TILE_X, nx - x0), h = min(TY, ny - y0);
+            const int zs = seg * a.lz, ze = min(zs + a.lz, a.nz), last = ze - zs + 1;
+            const int y = y0 + warp, x = x0 + 2 * lane;
+            const bool own = warp < h && 2 * lane < w;
+            const int last_lane = (w >> 1) - 1;
+            const int64_t zst = (int64_t)ny * nxb * G::WPN * kXBlock;
+            const int in_row = (lane >> 4) * (G::WPN * kXBlock) + 2 * (lane & 15);  // the lane's word in a row
+            uint32_t *dst = reinterpret_cast<uint32_t *>(a.m[parity ^ 1]) + row_word<S>(2 * tix, y, zs, nxb, ny) + in_row;
+            const float su = kScaled<S> ? a.sc.s[1] : 1.0f, sm = kScaled<S> ? a.sc.s[2] : 1.0f;
+            const float iu = kScaled<S> ? a.sc.is[1] : 1.0f, im = kScaled<S> ? a.sc.is[2] : 1.0f;
+            const float omega = a.omega, omega_u = kScaled<S> ? a.omega * (sm * (iu * iu)) : a.omega;
+            const float cs = kScaled<S> ? __fmul_rn(-kCs2, sm) : -kCs2;
+            const bool sr_on = kScaled<S> && a.sr_step != nullptr;
+            const uint32_t sr_seed = sr_on ? sr_step_seed(*a.sr_step) : 0u;
+            const int slot = SPECIAL && a.tile_slot ? a.tile_slot[tile] : -1;  // -1: no boundary nodes
+            float *side = SPECIAL ? a.side + side_index(slot, x, y, zs, x0, y0, a.nz, TILE_X, TY) * 16 : nullptr;
+            uint32_t marks = 0u;  // of the lane's nodes in plane k - 1, a byte each
+            float dm = 0.f, de = 0.f;
+
+            // times 4, of the plane emitted next: sums of its c_z = +1 and 0 classes (c_z = +1 from the plane
+            // below), and of its c_z = +1 class alone; c_z = +1 class of the plane read last
+            V2 pr, px, py, pxx, pyy, pxy, u0s, uxs, uys;
+            ClassSums up;
+            pr.v = px.v = py.v = pxx.v = pyy.v = pxy.v = u0s.v = uxs.v = uys.v = 0ull;
+            up = {pr, pr, pr, pr, pr, pr};
+
+            // store the collided moments of the lane's nodes (u0, u1: which of them) in plane z
+            auto put = [&](uint32_t *p, const Pair &o, bool u0, bool u1, int z) {
+                const float sr = a.sc.s[0];
+                if (sr_on) {
+                    const uint32_t k0 = sr_key(sr_seed, x, y, z, nx, ny), k1 = sr_key(sr_seed, x + 1, y, z, nx, ny);
+                    if (u0 && u1) store_pair<S, true>(p, o, sr, k0, k1);
+                    else if (u0 || u1) store_node<S, true>(p + !u0, node_of(o, u0 ? 0 : 1), sr, u0 ? k0 : k1);
+                } else {
+                    if (u0 && u1) store_pair<S, false>(p, o, sr, 0u, 0u);
+                    else if (u0 || u1) store_node<S, false>(p + !u0, node_of(o, u0 ? 0 : 1), sr, 0u);
+                }
+            };
+            auto plane = [&](const int k) {
+                if (k > 0 && ok) ok = mbar_wait(landed + stage, phase);
+                if (!ok) return;
+                Pair o;
+                V2 rho4;  // 4 rho, as the sums in `o`
+                uint32_t marks_in = 0u;
+                if (warp < h) {
+                    const uint32_t *sp = stages + stage * G::STAGEW + warp * G::ROWW + in_row;
+                    const float *hv = halos + ((stage * 2 + (lane >= 16 || lane == last_lane)) * TY + warp) * G::HALO;
+                    // the nine populations of the row y - cy that enter this row, shifted along x;
+                    // g[cx + 1][cz + 1]
+                    auto pulled = [&](auto cyc, V2 (&g)[3][3]) {
+                        constexpr int cy = decltype(cyc)::value;
+                        V2 f[27];
+                        rebuild_scaled<S>(load_pair<S>(sp + (1 - cy) * G::ROWW), K, f);
+                        // the side columns' populations are evaluated meanwhile
+                        if (cy == -1 && k > 0) ok = mbar_wait(full + stage, phase);
+                        const float e[3] = {hv[3 * (cy + 1)], hv[3 * (cy + 1) + 1], hv[3 * (cy + 1) + 2]};
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) {
+                            const V2 fp = f[direction(1, cy, c - 1)], fm = f[direction(-1, cy, c - 1)];
+                            const float left = __shfl_up_sync(0xffffffffu, hi(fp), 1);
+                            const float right = __shfl_down_sync(0xffffffffu, lo(fm), 1);
+                            g[2][c] = v2(lane == 0 ? e[c] : left, lo(fp));
+                            g[1][c] = f[direction(0, cy, c - 1)];
+                            g[0][c] = v2(hi(fm), lane == last_lane ? e[c] : right);
+                        }
+                    };
+                    // row by row into each class's row and column sums (c_y = -1, 0, +1), where a population
+                    // with one zero less among (c_x, c_y) weighs 4 times as much
+                    const V2 four = bc<V2>(4.0f);
+                    V2 mm[3], pm[3], rm[3], cm[3], cp[3], r0[3], g[3][3];
+                    pulled(std::integral_constant<int, -1>{}, g);
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        mm[c] = g[0][c];
+                        pm[c] = g[2][c];
+                        rm[c] = add(fma(g[1][c], four, g[0][c]), g[2][c]);
+                    }
+                    pulled(std::integral_constant<int, 0>{}, g);
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        r0[c] = add(fma(g[1][c], four, g[0][c]), g[2][c]);  // a quarter of it
+                        cp[c] = fma(g[2][c], four, pm[c]);
+                        cm[c] = fma(g[0][c], four, mm[c]);
+                    }
+                    if constexpr (SPECIAL) {
+                        // a solid node of an updated block keeps its stored moments, collided (the reference
+                        // collides every node of an active block); a plain fluid node whose only mark is the
+                        // wall-stencil bit is updated like any bulk node, plus its snapshot; every other
+                        // marked node is the node-list kernel's, or frozen
+                        if (slot >= 0 && own && k >= 1 && k < last)
+                            marks_in = *reinterpret_cast<const uint16_t *>(
+                                reinterpret_cast<const uint8_t *>(stages + stage * G::STAGEW + (TY + 2) * G::ROWW + G::SIDEC * G::WPN) +
+                                warp * TILE_X + 2 * lane);
+                        const bool q0 = marks_in & MARK_SOLID, q1 = marks_in & (MARK_SOLID << 8);
+                        if (q0 || q1) {
+                            const Stored<V2> q = load_pair<S>(sp + G::ROWW);
+                            // unscaled, collided and scaled again, as the reference order rounds it
+                            Pair so{q.r, q.ux, q.uy, q.uz, q.mxx, q.myy, q.mzz, q.mxy, q.mxz, q.myz};
+                            auto rescale = [&](V2 u, V2 v) {
+                                for (V2 *p : {&so.ux, &so.uy, &so.uz}) *p = mul(*p, u);
+                                for (V2 *p : {&so.mxx, &so.myy, &so.mzz, &so.mxy, &so.mxz, &so.myz}) *p = mul(*p, v);
+                            };
+                            if constexpr (kScaled<S>) {
+                                so.r = sub(fma(q.r, bc<V2>(K.ir), bc<V2>(K.rho0)), bc<V2>(K.rho0));
+                                rescale(bc<V2>(iu), bc<V2>(im));
+                            }
+                            float *const e = side + (int64_t)(k - 1) * (TILE_X * TY * 16);
+                            if (q0 && (marks_in & MARK_SNAPSHOT)) snapshot(e, node_of(so, 0), 1.0f, 1.0f);
+                            if (q1 && (marks_in & (MARK_SNAPSHOT << 8))) snapshot(e + 16, node_of(so, 1), 1.0f, 1.0f);
+                            collide_pair(so, omega, omega);
+                            if constexpr (kScaled<S>) rescale(bc<V2>(su), bc<V2>(sm));
+                            put(dst + (k >= 2 ? zst : 0), so, q0, q1, zs + k - 1);
                         }
                     }
-                    arrive_rim<S, TY>(cur, rho0, sc, rside, up_base + k4 * G::PLANE, fl_base + k3 * G::PLANE,
-                                      dn_base + (k & 1) * G::PLANE, ccol);
-                }
-                if (k >= 2) nb_arrive(1 + (k & 1), G::NTH);  // FULL(k)
-                k3 = k3 == 2 ? 0 : k3 + 1;
-                k4 = (k4 + 1) & 3;
-            };
-            for (int k = 0; k <= last; k += 2) {
-                rim_plane(k, pa, pb);
-                if (k + 1 <= last) rim_plane(k + 1, pb, pa);
-            }
-        }
-        if (tid == 0) s_next = work ? (int)gridDim.x + atomicAdd(work, 1) : it + (int)gridDim.x;
-        __syncthreads();  // the next item reuses the rings from slot 0
-        it = s_next;
-    }
-
-    if (diag) {
-        // deterministic block reduction of the owner threads' FP64 partials -> diag_part[blockIdx.x]
+                    pulled(std::integral_constant<int, 1>{}, g);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(empty + stage);
+                    auto finish = [&](int c) {
+                        const V2 rp = add(fma(g[1][c], four, g[0][c]), g[2][c]);
+                        const V2 cpc = add(cp[c], g[2][c]), cmc = add(cm[c], g[0][c]);
+                        return ClassSums{add(fma(r0[c], four, rp), rm[c]), sub(cpc, cmc), sub(rp, rm[c]), add(cpc, cmc), add(rp, rm[c]),
+                                         sub(add(g[2][c], mm[c]), add(pm[c], g[0][c]))};
+                    };
+                    const ClassSums dn = finish(0);
+                    {
+                        V2 *const v[] = {&uys, &uxs, &pxy, &pyy, &pxx, &u0s, &py, &px, &pr};
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            dmD += __shfl_down_sync(0xffffffffu, dmD, o);
-            deD += __shfl_down_sync(0xffffffffu, deD, o);
-        }
-        if (tx == 0 && owner) {
-            red[0][ty] = dmD;
-            red[1][ty] = deD;
-        }
-        __syncthreads();
-        if (tid == 0) {
-            double s0 = 0.0, s1 = 0.0;
-            for (int i = 0; i < TY; ++i) {
-                s0 += red[0][i];
-                s1 += red[1][i];
+                        for (int i = 0; i < G::PARK; ++i) *v[i] = park[i * 32 * TY];
+                    }
+                    rho4 = add(pr, dn.s0);
+                    o.ux = add(px, dn.sx);
+                    o.uy = add(py, dn.sy);
+                    o.uz = sub(u0s, dn.s0);
+                    o.mxx = add(pxx, dn.sxx);
+                    o.myy = add(pyy, dn.syy);
+                    o.mzz = add(u0s, dn.s0);
+                    o.mxy = add(pxy, dn.sxy);
+                    o.mxz = sub(uxs, dn.sx);
+                    o.myz = sub(uys, dn.sy);
+                    const ClassSums flat = finish(1);
+                    pr = fma(flat.s0, four, up.s0);
+                    px = fma(flat.sx, four, up.sx);
+                    py = fma(flat.sy, four, up.sy);
+                    pxx = fma(flat.sxx, four, up.sxx);
+                    pyy = fma(flat.syy, four, up.syy);
+                    pxy = fma(flat.sxy, four, up.sxy);
+                    u0s = up.s0;
+                    uxs = up.sx;
+                    uys = up.sy;
+                    {
+                        V2 *const v[] = {&uys, &uxs, &pxy, &pyy, &pxx, &u0s, &py, &px, &pr};
+#pragma unroll
+                        for (int i = 0; i < G::PARK; ++i) park[i * 32 * TY] = *v[i];
+                    }
+                    up = finish(2);
+                } else {
+                    if (lane == 0) mbar_arrive(empty + stage);
+                }
+                next_stage();
+                if (k >= 2) {
+                    if (own) {
+                        const V2 rho = mul(rho4, bc<V2>(0.25f));
+                        const V2 inv = v2(__frcp_rn(lo(rho)), __frcp_rn(hi(rho)));  // correctly rounded
+                        const V2 vu = mul(inv, bc<V2>(0.25f * su)), vm = kScaled<S> ? mul(inv, bc<V2>(0.25f * sm)) : vu;
+                        o.r = sub(rho, bc<V2>(a.rho0));
+                        o.ux = mul(o.ux, vu);
+                        o.uy = mul(o.uy, vu);
+                        o.uz = mul(o.uz, vu);
+                        o.mxx = fma(o.mxx, vm, bc<V2>(cs));
+                        o.myy = fma(o.myy, vm, bc<V2>(cs));
+                        o.mzz = fma(o.mzz, vm, bc<V2>(cs));
+                        o.mxy = mul(o.mxy, vm);
+                        o.mxz = mul(o.mxz, vm);
+                        o.myz = mul(o.myz, vm);
+                        bool u0 = true, u1 = true;  // nodes updated here
+                        if constexpr (SPECIAL) {
+                            u0 = !(marks & MARK_OTHER);
+                            u1 = !(marks & (MARK_OTHER << 8));
+                            float *const e = side + (int64_t)(k - 2) * (TILE_X * TY * 16);
+                            if (u0 && (marks & MARK_SNAPSHOT)) snapshot(e, node_of(o, 0), iu, im);
+                            if (u1 && (marks & (MARK_SNAPSHOT << 8))) snapshot(e + 16, node_of(o, 1), iu, im);
+                        }
+                        if (diag_part) {
+                            const float ke = 0.5f * (iu * iu);
+                            const V2 e2 = fma(o.ux, o.ux, fma(o.uy, o.uy, mul(o.uz, o.uz)));
+                            if (u0) {
+                                dm += lo(o.r);
+                                de += ke * lo(e2);
+                            }
+                            if (u1) {
+                                dm += hi(o.r);
+                                de += ke * hi(e2);
+                            }
+                        }
+                        collide_pair(o, omega, omega_u);
+                        put(dst, o, u0, u1, zs + k - 2);
+                    }
+                    dst += zst;
+                }
+                marks = marks_in;
+            };
+#pragma unroll 1
+            for (int k = 0; k <= last && ok; ++k) plane(k);
+            if (diag_part) {
+                // the warp's sums over the item -> their slot of diag_part (items of a strided launch that
+                // share a CTA share its slots, in order): the same sums whichever CTA takes the item
+                double dmD = (double)dm, deD = (double)de;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    dmD += __shfl_down_sync(0xffffffffu, dmD, o);
+                    deD += __shfl_down_sync(0xffffffffu, deD, o);
+                }
+                if (lane == 0) {
+                    const int at = (SPECIAL ? head.z : (int)blockIdx.x) * TY + warp;
+                    if (!SPECIAL && items > 0) {
+                        dmD += diag_part[2 * at + 0];
+                        deD += diag_part[2 * at + 1];
+                    }
+                    diag_part[2 * at + 0] = dmD;
+                    diag_part[2 * at + 1] = deD;
+                }
+                ++items;
             }
-            diag_part[2 * blockIdx.x + 0] = s0;
-            diag_part[2 * blockIdx.x + 1] = s1;
         }
+        if (!ok && lane == 0) atomicOr(BATCH ? ba->cases[0]->error : single.error, kErrorWait);
     }
 }
 
@@ -600,7 +775,7 @@ __global__ void diag_finalize_kernel(const double *__restrict__ part, int n, dou
 // Opt the kernel into its dynamic shared memory once per device (the attribute belongs to the
 // current device's context; never set inside a stream capture: batched launches are prepared
 // before their graphs are captured).  Devices past the 64th are configured on every launch.
-template <typename S, int TY, bool SP, bool BATCH, bool FULL = false>
+template <typename S, int TY, bool SP, bool BATCH>
 cudaError_t configure_t() {
     static std::atomic<unsigned long long> configured{0ull};
     int dev = 0;
@@ -608,136 +783,79 @@ cudaError_t configure_t() {
     if (e != cudaSuccess) return e;
     const unsigned long long bit = dev >= 0 && dev < 64 ? 1ull << dev : 0ull;
     if (bit && (configured.load(std::memory_order_acquire) & bit)) return cudaSuccess;
-    e = cudaFuncSetAttribute(step_kernel<S, TY, SP, BATCH, FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             Geo<TY>::SMEM);
+    if constexpr (Geo<S, TY, SP>::SPLIT) {
+        // the register split hands out exactly what the launch allocates: refuse a build whose launch
+        // allocates less (the owners would wait for registers that never come)
+        cudaFuncAttributes at;
+        if ((e = cudaFuncGetAttributes(&at, step_kernel<S, TY, SP, BATCH>)) != cudaSuccess) return e;
+        if ((at.numRegs + 7) / 8 * 8 * Geo<S, TY, SP>::NTH < 32 * (TY * 104 + Geo<S, TY, SP>::NH * 64))
+            return cudaErrorLaunchOutOfResources;
+    }
+    e = cudaFuncSetAttribute(step_kernel<S, TY, SP, BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             Geo<S, TY, SP>::SMEM);
     if (e != cudaSuccess) return e;
     configured.fetch_or(bit, std::memory_order_acq_rel);
     return cudaSuccess;
 }
 
-template <typename S, int TY, bool SP, bool BATCH, bool FULL = false>
-cudaError_t launch_t(const StepArgs *ga, const BatchArgs *ba, int parity, double *diag_part, int n_ctas,
-                     cudaStream_t s) {
-    const cudaError_t e = configure_t<S, TY, SP, BATCH, FULL>();
+template <typename S, int TY, bool SP, bool BATCH>
+cudaError_t launch_t(const StepArgs &a, const BatchArgs *ba, int parity, double *diag_part, int n_ctas, cudaStream_t s) {
+    const cudaError_t e = configure_t<S, TY, SP, BATCH>();
     if (e != cudaSuccess) return e;
-    step_kernel<S, TY, SP, BATCH, FULL><<<n_ctas, Geo<TY>::NTH, Geo<TY>::SMEM, s>>>(ga, ba, parity, diag_part);
+    step_kernel<S, TY, SP, BATCH><<<n_ctas, Geo<S, TY, SP>::NTH, Geo<S, TY, SP>::SMEM, s>>>(a, ba, parity, diag_part);
     return cudaGetLastError();
 }
 
-// `full`: whole tiles only; used by the single-case bulk variant (the other variants keep the
-// ragged-edge predicates)
-template <typename S, bool SP, bool BATCH>
-cudaError_t launch_s(const StepArgs *ga, const BatchArgs *ba, int parity, double *diag_part, int n_ctas, int tile_y,
-                     bool full, cudaStream_t s) {
-    if constexpr (!SP && !BATCH) {
-        if (full) {
-            switch (tile_y) {
-                case 4: return launch_t<S, 4, false, false, true>(ga, ba, parity, diag_part, n_ctas, s);
-                case 8: return launch_t<S, 8, false, false, true>(ga, ba, parity, diag_part, n_ctas, s);
-                case 16: return launch_t<S, 16, false, false, true>(ga, ba, parity, diag_part, n_ctas, s);
-                default: return cudaErrorInvalidValue;
-            }
+// Run f(storage type tag, tile-height tag) for the storage mode and tile height.
+template <typename T>
+struct Tag {
+    using type = T;
+};
+template <typename F>
+auto dispatch(int storage, int tile_y, F f) -> decltype(f(Tag<float>{}, std::integral_constant<int, 4>{})) {
+    auto height = [&](auto tag) {
+        switch (tile_y) {
+            case 4: return f(tag, std::integral_constant<int, 4>{});
+            case 8: return f(tag, std::integral_constant<int, 8>{});
+            default: return f(tag, std::integral_constant<int, 16>{});
         }
-    }
-    switch (tile_y) {
-        case 4: return launch_t<S, 4, SP, BATCH>(ga, ba, parity, diag_part, n_ctas, s);
-        case 8: return launch_t<S, 8, SP, BATCH>(ga, ba, parity, diag_part, n_ctas, s);
-        case 16: return launch_t<S, 16, SP, BATCH>(ga, ba, parity, diag_part, n_ctas, s);
-        default: return cudaErrorInvalidValue;
+    };
+    switch (storage) {
+        case MRLBM_STORAGE_F16: return height(Tag<__half>{});
+        case MRLBM_STORAGE_BF16: return height(Tag<__nv_bfloat16>{});
+        case MRLBM_STORAGE_F16_U32: return height(Tag<HybridWord>{});
+        default: return height(Tag<float>{});
     }
 }
-
-template <typename S, int TY>
-int occ_t() {
-    int n = 0;
-    cudaFuncSetAttribute(step_kernel<S, TY, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         Geo<TY>::SMEM);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, step_kernel<S, TY, true, false, false>, Geo<TY>::NTH,
-                                                      Geo<TY>::SMEM) !=
-        cudaSuccess)
-        return 0;
-    return n;
-}
-template <typename S>
-int occ_s(int ty) {
-    switch (ty) {
-        case 4: return occ_t<S, 4>();
-        case 8: return occ_t<S, 8>();
-        case 16: return occ_t<S, 16>();
-        default: return 0;
-    }
+bool known(int storage, int tile_y) {
+    return storage >= MRLBM_STORAGE_F32 && storage <= MRLBM_STORAGE_F16_U32 && (tile_y == 4 || tile_y == 8 || tile_y == 16);
 }
 
 }  // namespace
 
 cudaError_t launch_step(const StepLaunch &l, int storage, int tile_y, bool special, cudaStream_t s) {
-    const StepArgs *ga = l.ga;
-    switch (storage) {
-        case MRLBM_STORAGE_F32:
-            return special ? launch_s<float, true, false>(ga, nullptr, l.parity, l.diag_part, l.n_ctas, tile_y, false, s)
-                           : launch_s<float, false, false>(ga, nullptr, l.parity, l.diag_part, l.n_ctas, tile_y,
-                                                           l.full_tiles, s);
-        case MRLBM_STORAGE_F16:
-            return special ? launch_s<__half, true, false>(ga, nullptr, l.parity, l.diag_part, l.n_ctas, tile_y, false, s)
-                           : launch_s<__half, false, false>(ga, nullptr, l.parity, l.diag_part, l.n_ctas, tile_y,
-                                                            l.full_tiles, s);
-        case MRLBM_STORAGE_BF16:
-            return special ? launch_s<__nv_bfloat16, true, false>(ga, nullptr, l.parity, l.diag_part, l.n_ctas, tile_y,
-                                                                  false, s)
-                           : launch_s<__nv_bfloat16, false, false>(ga, nullptr, l.parity, l.diag_part, l.n_ctas,
-                                                                   tile_y, l.full_tiles, s);
-        case MRLBM_STORAGE_F16_U32:
-            return special ? launch_s<HybridWord, true, false>(ga, nullptr, l.parity, l.diag_part, l.n_ctas, tile_y,
-                                                                  false, s)
-                           : launch_s<HybridWord, false, false>(ga, nullptr, l.parity, l.diag_part, l.n_ctas,
-                                                                   tile_y, l.full_tiles, s);
-        default: return cudaErrorInvalidValue;
-    }
-}
-
-template <typename S, int TY>
-cudaError_t prepare_ty() {
-    const cudaError_t e = configure_t<S, TY, true, true>();
-    return e != cudaSuccess ? e : configure_t<S, TY, false, true>();
-}
-
-template <typename S>
-cudaError_t prepare_s(int tile_y) {
-    switch (tile_y) {
-        case 4: return prepare_ty<S, 4>();
-        case 8: return prepare_ty<S, 8>();
-        case 16: return prepare_ty<S, 16>();
-        default: return cudaErrorInvalidValue;
-    }
+    if (!known(storage, tile_y)) return cudaErrorInvalidValue;
+    return dispatch(storage, tile_y, [&](auto t, auto ty) {
+        using S = typename decltype(t)::type;
+        return special ? launch_t<S, ty(), true, false>(*l.args, nullptr, l.parity, l.diag_part, l.n_ctas, s)
+                       : launch_t<S, ty(), false, false>(*l.args, nullptr, l.parity, l.diag_part, l.n_ctas, s);
+    });
 }
 
 cudaError_t prepare_step_batch(int storage, int tile_y) {
-    switch (storage) {
-        case MRLBM_STORAGE_F32: return prepare_s<float>(tile_y);
-        case MRLBM_STORAGE_F16: return prepare_s<__half>(tile_y);
-        case MRLBM_STORAGE_BF16: return prepare_s<__nv_bfloat16>(tile_y);
-        case MRLBM_STORAGE_F16_U32: return prepare_s<HybridWord>(tile_y);
-        default: return cudaErrorInvalidValue;
-    }
+    if (!known(storage, tile_y)) return cudaErrorInvalidValue;
+    return dispatch(storage, tile_y, [&](auto t, auto ty) {
+        using S = typename decltype(t)::type;
+        return configure_t<S, ty(), true, true>();
+    });
 }
 
-cudaError_t launch_step_batch(const BatchArgs *ba, int parity, int storage, int tile_y, bool special, int n_ctas,
-                              cudaStream_t s) {
-    switch (storage) {
-        case MRLBM_STORAGE_F32:
-            return special ? launch_s<float, true, true>(nullptr, ba, parity, nullptr, n_ctas, tile_y, false, s)
-                           : launch_s<float, false, true>(nullptr, ba, parity, nullptr, n_ctas, tile_y, false, s);
-        case MRLBM_STORAGE_F16:
-            return special ? launch_s<__half, true, true>(nullptr, ba, parity, nullptr, n_ctas, tile_y, false, s)
-                           : launch_s<__half, false, true>(nullptr, ba, parity, nullptr, n_ctas, tile_y, false, s);
-        case MRLBM_STORAGE_BF16:
-            return special ? launch_s<__nv_bfloat16, true, true>(nullptr, ba, parity, nullptr, n_ctas, tile_y, false, s)
-                           : launch_s<__nv_bfloat16, false, true>(nullptr, ba, parity, nullptr, n_ctas, tile_y, false, s);
-        case MRLBM_STORAGE_F16_U32:
-            return special ? launch_s<HybridWord, true, true>(nullptr, ba, parity, nullptr, n_ctas, tile_y, false, s)
-                           : launch_s<HybridWord, false, true>(nullptr, ba, parity, nullptr, n_ctas, tile_y, false, s);
-        default: return cudaErrorInvalidValue;
-    }
+cudaError_t launch_step_batch(const BatchArgs *ba, int parity, int storage, int tile_y, int n_items, cudaStream_t s) {
+    if (!known(storage, tile_y)) return cudaErrorInvalidValue;
+    return dispatch(storage, tile_y, [&](auto t, auto ty) {
+        using S = typename decltype(t)::type;
+        return launch_t<S, ty(), true, true>(StepArgs(), ba, parity, nullptr, n_items, s);
+    });
 }
 
 cudaError_t launch_diag_finalize(const double *part, int n, double *out, int *error, cudaStream_t s) {
@@ -745,64 +863,61 @@ cudaError_t launch_diag_finalize(const double *part, int n, double *out, int *er
     return cudaGetLastError();
 }
 
-int step_kernel_smem_bytes(int tile_y) {
-    switch (tile_y) {
-        case 4: return Geo<4>::SMEM;
-        case 8: return Geo<8>::SMEM;
-        case 16: return Geo<16>::SMEM;
-        default: return 0;
-    }
+int step_kernel_max_ctas_per_sm(int storage, int tile_y) {
+    if (!known(storage, tile_y)) return 0;
+    return dispatch(storage, tile_y, [&](auto t, auto ty) {
+        using S = typename decltype(t)::type;
+        int n = 0;
+        if (configure_t<S, ty(), true, false>() != cudaSuccess) return 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, step_kernel<S, ty(), true, false>, Geo<S, ty(), true>::NTH,
+                                                          Geo<S, ty(), true>::SMEM) != cudaSuccess)
+            return 0;
+        return n;
+    });
 }
 
-int step_kernel_max_ctas_per_sm(int storage, int tile_y) {
-    switch (storage) {
-        case MRLBM_STORAGE_F32: return occ_s<float>(tile_y);
-        case MRLBM_STORAGE_F16: return occ_s<__half>(tile_y);
-        case MRLBM_STORAGE_BF16: return occ_s<__nv_bfloat16>(tile_y);
-        case MRLBM_STORAGE_F16_U32: return occ_s<HybridWord>(tile_y);
-        default: return 0;
+void choose_tiling(int nx, int ny, int nz, int storage, int n_sm, int &ty, int &lz) {
+    if (ty != 4 && ty != 8 && ty != 16) ty = 16;
+    const int64_t slots = (int64_t)std::max(1, step_kernel_max_ctas_per_sm(storage, ty)) * n_sm;
+    const int64_t tiles = (int64_t)((nx + TILE_X - 1) / TILE_X) * ((ny + ty - 1) / ty);
+    if (lz > 0) {
+        lz = std::min(nz, lz);
+        return;
+    }
+    int64_t best = INT64_MAX;
+    for (int nseg = 1; nseg <= std::min(nz, 1 << 11); ++nseg) {
+        const int l = (nz + nseg - 1) / nseg;
+        const int64_t waves = (tiles * ((nz + l - 1) / l) + slots - 1) / slots;
+        const int64_t cost = waves * (2 * l + 7);
+        if (cost < best) {
+            best = cost;
+            lz = l;
+        }
     }
 }
 
 // ---- allocation-free periodic step --------------------------------------------------------
-// For callers that cannot allocate device memory: the step kernel's own scratch (its argument
-// block, work-item list, diagnostics partials and sums, error word) lives in this fixed array
-// of the library's device image, kNoAllocScratchBytes = 64 KiB, laid out as in kernels.h.
-// Every call shares it and it keeps the last call's contents; calls that overlap on the GPU
-// (two streams, or two host threads) race on it.
+// For callers that cannot allocate device memory: what a step needs besides the caller's buffers
+// (diagnostics partials and sums, error word) lives in this fixed array of the library's device
+// image, laid out as in kernels.h; the argument block travels with the launch.  Every call that
+// asks for diagnostics shares the array: such calls race on it when they overlap on the GPU (two
+// streams, or two host threads).
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
-
-static_assert(sizeof(StepArgs) <= kNoAllocDiagOffset, "StepArgs outgrew its scratch slot");
-static_assert(kNoAllocItemsOffset < kNoAllocScratchBytes, "scratch layout");
 
 namespace {
 
 constexpr int kNoAllocMaxDevices = 64;
 std::mutex g_noalloc_mu;
-// per device, set up on its first call: the scratch array's device address, the SM count and
-// the resident step-kernel CTAs per SM
+// per device, set up on its first call: the scratch array's device address and the SM count
 struct NoAllocDevice {
     void *scratch = nullptr;
-    int n_sm = 0, per_sm = 0;
+    int n_sm = 0;
 };
 NoAllocDevice g_noalloc_dev[kNoAllocMaxDevices];
 
-// Write the argument block, clear the error word and fill the work items (every xy tile of
-// every z segment, segment-major) inside the scratch array: one launch, no host staging.
-__global__ void noalloc_setup_kernel(const StepArgs a, unsigned char *scratch, int tiles, int n_items) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) {
-        *(StepArgs *)scratch = a;
-        *(int *)(scratch + kNoAllocErrorOffset) = 0;
-        *(int *)(scratch + kNoAllocWorkOffset) = 0;
-    }
-    int32_t *items = (int32_t *)(scratch + kNoAllocItemsOffset);
-    for (int j = i; j < n_items; j += gridDim.x * blockDim.x) items[j] = (j % tiles) | ((j / tiles) << 20);
-}
-
 // Set-up of device `dev` (the current device), once: the scratch array's device address (in
-// host code the array's name is only a host-side stand-in), its SM count and the step kernel's
-// occupancy.  Host-side queries only; nothing is allocated.
+// host code the array's name is only a host-side stand-in) and its SM count.  Host-side queries
+// only; nothing is allocated.
 cudaError_t noalloc_device(int dev, NoAllocDevice &out) {
     std::lock_guard<std::mutex> lock(g_noalloc_mu);
     NoAllocDevice &d = g_noalloc_dev[dev];
@@ -813,8 +928,7 @@ cudaError_t noalloc_device(int dev, NoAllocDevice &out) {
         int n_sm = 0;
         if ((e = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
         d.n_sm = n_sm;
-        d.per_sm = std::max(1, occ_s<float>(kNoAllocTileY));
-        d.scratch = p;
+                d.scratch = p;
     }
     out = d;
     return cudaSuccess;
@@ -856,11 +970,10 @@ int noalloc_periodic_step(const NoAllocStep &p, std::string &err) {
         err = std::string(fn) + "input and output moment buffers overlap";
         return MRLBM_ERR_INVALID_ARG;
     }
-    const int tiles_x = (p.nx + TILE_X - 1) / TILE_X, tiles_y = (p.ny + kNoAllocTileY - 1) / kNoAllocTileY;
-    const int tiles = tiles_x * tiles_y;
-    if (tiles > kNoAllocMaxItems) {
-        err = std::string(fn) + "grid too large for the fixed 64 KiB scratch: " + std::to_string(tiles) +
-              " xy tiles of 32 x 16 nodes, at most " + std::to_string(kNoAllocMaxItems);
+    const int64_t patches = (int64_t)((p.nx + 31) / 32) * ((p.ny + 15) / 16);
+    if (patches > kNoAllocMaxTiles) {
+        err = std::string(fn) + "grid too large for the fixed 64 KiB scratch: " + std::to_string(patches) +
+              " xy tiles of 32 x 16 nodes, at most " + std::to_string(kNoAllocMaxTiles);
         return MRLBM_ERR_INVALID_ARG;
     }
 
@@ -885,51 +998,39 @@ int noalloc_periodic_step(const NoAllocStep &p, std::string &err) {
     if ((e = noalloc_device(dev, nd)) != cudaSuccess) return noalloc_cuda_fail(e, "device set-up", err);
     unsigned char *scratch = (unsigned char *)nd.scratch;
 
-    // tiling: 32 x 16 columns; the longest z segment that still gives every resident CTA
-    // several items, lengthened if the item list would not fit the scratch or the segment
-    // number its 11-bit field of the work item (tile | segment << 20)
-    const int resident = nd.per_sm * nd.n_sm;
-    int lz = p.nz;
-    while (lz > 16 && (int64_t)tiles * ((p.nz + lz - 1) / lz) < 4LL * resident) lz = (lz + 1) / 2;
-    const int max_seg = std::min(kNoAllocMaxItems / tiles, 1 << 11);
-    if ((p.nz + lz - 1) / lz > max_seg) lz = (p.nz + max_seg - 1) / max_seg;
-    const int nseg = (p.nz + lz - 1) / lz;
-    const int n_items = tiles * nseg;
-    const int n_ctas = std::max(1, std::min(std::min(n_items, resident), kNoAllocMaxCtas));
+    int ty = 0, lz = 0;
+    choose_tiling(p.nx, p.ny, p.nz, MRLBM_STORAGE_F32, nd.n_sm, ty, lz);
+    const int tiles_x = (p.nx + TILE_X - 1) / TILE_X, tiles_y = (p.ny + ty - 1) / ty;
+    const int n_items = tiles_x * tiles_y * ((p.nz + lz - 1) / lz);
+    const int n_ctas = std::min(std::min(n_items, step_kernel_max_ctas_per_sm(MRLBM_STORAGE_F32, ty) * nd.n_sm),
+                                kNoAllocMaxParts / ty);
 
     StepArgs sa;
     sa.m[0] = const_cast<float *>(p.m_in);
     sa.m[1] = p.m_out;
     sa.nxb = (p.nx + kXBlock - 1) / kXBlock;
-    sa.items = (const int32_t *)(scratch + kNoAllocItemsOffset);
-    sa.n_items = n_items;
+    sa.n_items = n_items;  // no list: item i is tile i % tiles of segment i / tiles
     sa.nx = p.nx;
     sa.ny = p.ny;
     sa.nz = p.nz;
     sa.tiles_x = tiles_x;
     sa.tiles_y = tiles_y;
-    sa.tile_y = kNoAllocTileY;
+    sa.tile_y = ty;
     sa.lz = lz;
     sa.omega = p.omega;
     sa.rho0 = p.rho0;
     for (int k = 0; k < 3; ++k) sa.sc.s[k] = sa.sc.is[k] = 1.f;
     sa.error = (int *)(scratch + kNoAllocErrorOffset);
-    sa.work_counter = (int *)(scratch + kNoAllocWorkOffset);
-
-    noalloc_setup_kernel<<<(n_items + 255) / 256, 256, 0, p.stream>>>(sa, scratch, tiles, n_items);
-    if ((e = cudaGetLastError()) != cudaSuccess) return noalloc_cuda_fail(e, "set-up launch", err);
-    StepLaunch L;
-    L.ga = (const StepArgs *)scratch;
-    L.parity = 0;
-    L.n_ctas = n_ctas;
     double *part = (double *)(scratch + kNoAllocPartOffset);
     double *sums = (double *)(scratch + kNoAllocDiagOffset);
-    if (p.diag_host) L.diag_part = part;
-    if ((e = launch_t<float, kNoAllocTileY, false, false>(L.ga, nullptr, 0, L.diag_part, L.n_ctas, p.stream)) !=
-        cudaSuccess)
+    StepLaunch L;
+    L.args = &sa;
+    L.n_ctas = n_ctas;
+    L.diag_part = p.diag_host ? part : nullptr;
+    if ((e = launch_step(L, MRLBM_STORAGE_F32, ty, false, p.stream)) != cudaSuccess)
         return noalloc_cuda_fail(e, "step launch", err);
     if (p.diag_host) {
-        if ((e = launch_diag_finalize(part, n_ctas, sums, nullptr, p.stream)) != cudaSuccess)
+        if ((e = launch_diag_finalize(part, n_ctas * ty, sums, nullptr, p.stream)) != cudaSuccess)
             return noalloc_cuda_fail(e, "diagnostics launch", err);
         double v[2];
         if ((e = cudaMemcpyAsync(v, sums, sizeof(v), cudaMemcpyDeviceToHost, p.stream)) != cudaSuccess ||

@@ -204,51 +204,26 @@ __device__ __forceinline__ void load_raw(const S *__restrict__ base, int64_t ai,
     }
 }
 
-// Load the stored words of a node without decoding them.
-template <typename S>
-__device__ __forceinline__ void load_words(const S *__restrict__ base, int64_t ai, Raw<S> &r) {
+// Load the stored words of a node without decoding them (`p`: its first word, the others STEP apart).
+template <typename S, int STEP = kXBlock>
+__device__ __forceinline__ void load_raw_words(const uint32_t *__restrict__ p, Raw<S> &r) {
     if constexpr (std::is_same<S, float>::value) {
-        const float *p = base + ai;
 #pragma unroll
-        for (int k = 0; k < 10; ++k) r.v[k] = p[k * kXBlock];
+        for (int k = 0; k < 10; ++k) r.v[k] = __uint_as_float(p[k * STEP]);
     } else if constexpr (kHybrid<S>) {
-        const uint32_t *p = reinterpret_cast<const uint32_t *>(base + ai);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) r.u[k] = __uint_as_float(p[k * kXBlock]);
+        for (int k = 0; k < 3; ++k) r.u[k] = __uint_as_float(p[k * STEP]);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) r.w[k] = p[(3 + k) * kXBlock];
+        for (int k = 0; k < 4; ++k) r.w[k] = p[(3 + k) * STEP];
     } else {
-        const uint32_t *p = reinterpret_cast<const uint32_t *>(base + ai);
 #pragma unroll
-        for (int j = 0; j < 5; ++j) r.w[j] = p[j * kXBlock];
+        for (int j = 0; j < 5; ++j) r.w[j] = p[j * STEP];
     }
 }
 
-// Populations of a node from its loaded words (rebuild of the decoded values).
+// The ten stored (scaled) values of a node from its loaded words.
 template <typename S>
-__device__ __forceinline__ void rebuild(const Raw<S> &r, float rho0, const StorageScale &sc, float f[27]) {
-    if constexpr (std::is_same<S, float>::value) {
-        rebuild<S>(r.v, rho0, sc, f);
-    } else if constexpr (kHybrid<S>) {
-        float v[10];
-        hybrid_values(r.u, r.w, v);
-        rebuild<S>(v, rho0, sc, f);
-    } else {
-        float v[10];
-#pragma unroll
-        for (int j = 0; j < 5; ++j) {
-            const float2 t = pair_to_f<S>(r.w[j]);
-            v[2 * j] = t.x;
-            v[2 * j + 1] = t.y;
-        }
-        rebuild<S>(v, rho0, sc, f);
-    }
-}
-
-// Moments (full rho) of a node from its loaded words: load_mom without the load.
-template <typename S>
-__device__ __forceinline__ Mom decode_words(const Raw<S> &r, float rho0, const StorageScale &sc) {
-    float v[10];
+__device__ __forceinline__ void raw_values(const Raw<S> &r, float v[10]) {
     if constexpr (std::is_same<S, float>::value) {
 #pragma unroll
         for (int k = 0; k < 10; ++k) v[k] = r.v[k];
@@ -262,7 +237,6 @@ __device__ __forceinline__ Mom decode_words(const Raw<S> &r, float rho0, const S
             v[2 * j + 1] = t.y;
         }
     }
-    return decode<S>(v, rho0, sc);
 }
 
 template <typename S>
@@ -332,49 +306,19 @@ __device__ __forceinline__ void store_mom_sr(S *__restrict__ base, int64_t ai, c
     }
 }
 
-// Stores of moments already held with the storage scales (u s_u, m s_m; rho as the full
-// density), as the bulk emit of the step kernel computes them for 16-bit storage.
-template <typename S>
-__device__ __forceinline__ void store_scaled(S *__restrict__ base, int64_t ai, const Mom &m, float rho0,
-                                             const StorageScale &sc) {
-    static_assert(!std::is_same<S, float>::value, "FP32 storage holds physical moments");
-    uint32_t *w = reinterpret_cast<uint32_t *>(base + ai);
-    if constexpr (kHybrid<S>) {
-        w[0 * kXBlock] = __float_as_uint(m.ux);
-        w[1 * kXBlock] = __float_as_uint(m.uy);
-        w[2 * kXBlock] = __float_as_uint(m.uz);
-        w[3 * kXBlock] = pair_from_f<__half>((m.rho - rho0) * sc.s[0], m.mxx);
-        w[4 * kXBlock] = pair_from_f<__half>(m.myy, m.mzz);
-        w[5 * kXBlock] = pair_from_f<__half>(m.mxy, m.mxz);
-        w[6 * kXBlock] = pair_from_f<__half>(m.myz, 0.0f);
-        return;
-    }
-    w[0 * kXBlock] = pair_from_f<S>((m.rho - rho0) * sc.s[0], m.ux);
-    w[1 * kXBlock] = pair_from_f<S>(m.uy, m.uz);
-    w[2 * kXBlock] = pair_from_f<S>(m.mxx, m.myy);
-    w[3 * kXBlock] = pair_from_f<S>(m.mzz, m.mxy);
-    w[4 * kXBlock] = pair_from_f<S>(m.mxz, m.myz);
+// One stored 16-bit pair, j-th of its node, rounded to nearest or stochastically (random bits from `key`).
+template <typename S, bool SR>
+__device__ __forceinline__ uint32_t round_pair(float a, float b, uint32_t key, int j) {
+    if constexpr (SR) return pair_from_f_sr<S>(a, b, mix32(key + (uint32_t)j * 0x9e3779b9u));
+    else return pair_from_f<S>(a, b);
 }
-template <typename S>
-__device__ __forceinline__ void store_scaled_sr(S *__restrict__ base, int64_t ai, const Mom &m, float rho0,
-                                                const StorageScale &sc, uint32_t key) {
-    static_assert(!std::is_same<S, float>::value, "FP32 storage holds physical moments");
-    uint32_t *w = reinterpret_cast<uint32_t *>(base + ai);
-    if constexpr (kHybrid<S>) {
-        w[0 * kXBlock] = __float_as_uint(m.ux);
-        w[1 * kXBlock] = __float_as_uint(m.uy);
-        w[2 * kXBlock] = __float_as_uint(m.uz);
-        w[3 * kXBlock] = pair_from_f_sr<__half>((m.rho - rho0) * sc.s[0], m.mxx, mix32(key));
-        w[4 * kXBlock] = pair_from_f_sr<__half>(m.myy, m.mzz, mix32(key + 0x9e3779b9u));
-        w[5 * kXBlock] = pair_from_f_sr<__half>(m.mxy, m.mxz, mix32(key + 0x3c6ef372u));
-        w[6 * kXBlock] = pair_from_f_sr<__half>(m.myz, 0.0f, mix32(key + 0xdaa66d2bu));
-        return;
-    }
-    w[0 * kXBlock] = pair_from_f_sr<S>((m.rho - rho0) * sc.s[0], m.ux, mix32(key));
-    w[1 * kXBlock] = pair_from_f_sr<S>(m.uy, m.uz, mix32(key + 0x9e3779b9u));
-    w[2 * kXBlock] = pair_from_f_sr<S>(m.mxx, m.myy, mix32(key + 0x3c6ef372u));
-    w[3 * kXBlock] = pair_from_f_sr<S>(m.mzz, m.mxy, mix32(key + 0xdaa66d2bu));
-    w[4 * kXBlock] = pair_from_f_sr<S>(m.mxz, m.myz, mix32(key + 0x78dde6e4u));
+
+// A side-buffer entry (16 floats, 64-byte aligned): rho - rho0, u, m of a wall-stencil node.
+__device__ __forceinline__ void store_side(float *e, float r, float ux, float uy, float uz, float mxx, float myy,
+                                           float mzz, float mxy, float mxz, float myz) {
+    reinterpret_cast<float4 *>(e)[0] = make_float4(r, ux, uy, uz);
+    reinterpret_cast<float4 *>(e)[1] = make_float4(mxx, myy, mzz, mxy);
+    reinterpret_cast<float2 *>(e)[4] = make_float2(mxz, myz);
 }
 
 // One stored field of a node (the stored, scaled value) and its store: the layout of each
