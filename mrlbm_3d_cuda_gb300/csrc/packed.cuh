@@ -109,11 +109,18 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t b
                  : "memory");
 }
 
-// A word that is not kept in L1.
+// Words that are not kept in L1.
 __device__ __forceinline__ uint32_t load_uncached(const uint32_t *p) {
     uint32_t v;
     asm volatile("ld.global.L1::no_allocate.b32 %0, [%1];" : "=r"(v) : "l"(p));
     return v;
+}
+
+__device__ __forceinline__ void store_uncached(uint32_t *p, uint32_t a) {
+    asm volatile("st.global.L1::no_allocate.b32 [%0], %1;" ::"l"(p), "r"(a) : "memory");
+}
+__device__ __forceinline__ void store_uncached(uint32_t *p, uint32_t a, uint32_t b) {
+    asm volatile("st.global.L1::no_allocate.v2.b32 [%0], {%1, %2};" ::"l"(p), "r"(a), "r"(b) : "memory");
 }
 
 // Cluster launch control: a running CTA takes over a CTA of its grid that has not started yet.

@@ -276,14 +276,20 @@ __device__ __forceinline__ void node_words(const Node &m, float sr, uint32_t key
     }
 }
 
-template <typename S, bool SR>
+// The collided moments leave past L1 (UNCACHED), which is then left to what the owners spill: FP32 at 256^3
+// 240.6 -> 232.5 us a step, an FP32 annulus 250 -> 240, a cylinder wake in hybrid storage 363 -> 349.  Plain
+// hybrid tiles spill nothing that comes back and are 1 % slower so (218 -> 221): they store as usual.
+template <typename S, bool SR, bool UNCACHED>
 __device__ __forceinline__ void store_pair(uint32_t *p, const Pair &m, float sr, uint32_t key0, uint32_t key1) {
     constexpr int WPN = StorageLayout<S>::words;
     uint32_t a[WPN], b[WPN];
     node_words<S, SR>(node_of(m, 0), sr, key0, a);
     node_words<S, SR>(node_of(m, 1), sr, key1, b);
 #pragma unroll
-    for (int f = 0; f < WPN; ++f) *reinterpret_cast<uint2 *>(p + f * kXBlock) = make_uint2(a[f], b[f]);
+    for (int f = 0; f < WPN; ++f) {
+        if constexpr (UNCACHED) store_uncached(p + f * kXBlock, a[f], b[f]);
+        else *reinterpret_cast<uint2 *>(p + f * kXBlock) = make_uint2(a[f], b[f]);
+    }
 }
 template <typename S, bool SR>
 __device__ __forceinline__ void store_node(uint32_t *p, const Node &m, float sr, uint32_t key) {
@@ -291,7 +297,7 @@ __device__ __forceinline__ void store_node(uint32_t *p, const Node &m, float sr,
     uint32_t a[WPN];
     node_words<S, SR>(m, sr, key, a);
 #pragma unroll
-    for (int f = 0; f < WPN; ++f) p[f * kXBlock] = a[f];
+    for (int f = 0; f < WPN; ++f) store_uncached(p + f * kXBlock, a[f]);
 }
 
 // Post-stream (pre-collision) moments of a wall-stencil node into its side-buffer entry, the
@@ -546,14 +552,15 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
             up = {pr, pr, pr, pr, pr, pr};
 
             // store the collided moments of the lane's nodes (u0, u1: which of them) in plane z
+            constexpr bool UNCACHED = SPECIAL || !kHybrid<S>;
             auto put = [&](uint32_t *p, const Pair &o, bool u0, bool u1, int z) {
                 const float sr = a.sc.s[0];
                 if (sr_on) {
                     const uint32_t k0 = sr_key(sr_seed, x, y, z, nx, ny), k1 = sr_key(sr_seed, x + 1, y, z, nx, ny);
-                    if (u0 && u1) store_pair<S, true>(p, o, sr, k0, k1);
+                    if (u0 && u1) store_pair<S, true, UNCACHED>(p, o, sr, k0, k1);
                     else if (u0 || u1) store_node<S, true>(p + !u0, node_of(o, u0 ? 0 : 1), sr, u0 ? k0 : k1);
                 } else {
-                    if (u0 && u1) store_pair<S, false>(p, o, sr, 0u, 0u);
+                    if (u0 && u1) store_pair<S, false, UNCACHED>(p, o, sr, 0u, 0u);
                     else if (u0 || u1) store_node<S, false>(p + !u0, node_of(o, u0 ? 0 : 1), sr, 0u);
                 }
             };
