@@ -146,7 +146,7 @@ int storage_element_bytes(int storage) {
 int setup_tiling(mrlbm_handle *h, int ty, int lz) {
     const mrlbm_case_desc &d = h->d;
     const Geometry &g = h->geo;
-    choose_tiling(d.nx, d.ny, d.nz, h->storage, h->n_sm, ty, lz);
+    if (ty != 4 && ty != 8 && ty != 16) ty = 16;
     CK(h, cudaStreamSynchronize(h->stream));
     for (void **p : {(void **)&h->d_tile_slot, (void **)&h->d_side, (void **)&h->d_items, (void **)&h->d_list_xyz,
                      (void **)&h->d_list_word, (void **)&h->d_diag_part}) {
@@ -160,7 +160,6 @@ int setup_tiling(mrlbm_handle *h, int ty, int lz) {
     if (per_sm <= 0) per_sm = 1;
     const int resident = per_sm * h->n_sm;
     const int tiles = h->tiles_x * h->tiles_y;
-    h->lz = lz;
     std::vector<uint32_t> word(h->n, 0);
     for (int64_t i = 0; i < h->n; ++i) word[i] = make_word(g.cls[i], g.payload[i], g.frozen[i] != 0, g.stencil[i] != 0);
     std::vector<int32_t> slot(tiles, -1);
@@ -181,34 +180,42 @@ int setup_tiling(mrlbm_handle *h, int ty, int lz) {
     }
     h->n_special = n_special;
 
-    // Non-bulk nodes of special tiles, by slot, z, tile row, x.  Solid nodes of updated blocks need
-    // no populations: the step kernel collides them in place; frozen nodes are never updated.
-    // Neither is in the list.
-    std::vector<uint64_t> list_xyz;
-    std::vector<uint32_t> list_word;
+    // Non-bulk nodes of special tiles, by slot, kind of closure, z, tile row, x: the lanes of a warp of the
+    // node-list kernel then mostly run one closure.  Solid nodes of updated blocks need no populations:
+    // the step kernel collides them in place; frozen nodes are never updated.  Neither is in the list.
+    auto kind = [](uint32_t cls) {
+        return cls == C_INNER || cls == C_OUTER ? 0 : (cls == C_BCFLUID_INNER || cls == C_BCFLUID_OUTER ? 1 : (cls < C_NORTH ? 2 : 3));
+    };
+    std::vector<uint64_t> list_xyz, by_xyz[4];
+    std::vector<uint32_t> list_word, by_word[4];
     for (int t = 0; t < tiles; ++t) {
         if (slot[t] < 0) continue;
         const int x0 = (t % h->tiles_x) * TILE_X, y0 = (t / h->tiles_x) * h->tile_y;
         for (int z = 0; z < d.nz; ++z)
-            for (int r = 0; r < h->tile_y; ++r) {
-                const int y = y0 + r;
-                if (y >= d.ny) continue;
+            for (int y = y0; y < std::min(d.ny, y0 + h->tile_y); ++y)
                 for (int x = x0; x < std::min(d.nx, x0 + TILE_X); ++x) {
-                    const int64_t i = x + (int64_t)d.nx * (y + (int64_t)d.ny * z);
-                    const uint32_t wd = word[i];
+                    const uint32_t wd = word[x + (int64_t)d.nx * (y + (int64_t)d.ny * z)];
                     // plain fluid nodes marked only as wall-stencil nodes are updated (and
                     // snapshotted) by the step kernel itself
                     if (wd == 0u || wd == NW_STENCIL || (wd & NW_FROZEN)) continue;
-                    if ((wd & NW_CLASS_MASK) == C_SOLID) continue;
-                    list_xyz.push_back((uint64_t)x | ((uint64_t)y << 21) | ((uint64_t)z << 42));
-                    list_word.push_back(wd);
+                    const uint32_t cls = wd & NW_CLASS_MASK;
+                    if (cls == C_SOLID) continue;
+                    by_xyz[kind(cls)].push_back((uint64_t)x | ((uint64_t)y << 21) | ((uint64_t)z << 42));
+                    by_word[kind(cls)].push_back(wd);
                 }
-            }
+        for (int k = 0; k < 4; ++k) {
+            list_xyz.insert(list_xyz.end(), by_xyz[k].begin(), by_xyz[k].end());
+            list_word.insert(list_word.end(), by_word[k].begin(), by_word[k].end());
+            by_xyz[k].clear();
+            by_word[k].clear();
+        }
     }
     if (list_xyz.size() >= (size_t)INT32_MAX / 27)
         return fail(h, MRLBM_ERR_INVALID_ARG, "too many boundary nodes");
     h->n_list = (int)list_xyz.size();
     h->n_list_blocks = special_list_blocks(h->n_list);
+    choose_tiling(d.nx, d.ny, d.nz, h->storage, h->n_sm, ty, lz, tiles - (int)std::count(skip.begin(), skip.end(), 1), h->n_list);
+    h->lz = lz;
     const int nseg = (d.nz + h->lz - 1) / h->lz;
     // work items are int32 `tile | segment << 20` (decoded in step_kernel)
     if (tiles > (1 << 20) || nseg > (1 << 11))
@@ -284,23 +291,28 @@ int step_handle(mrlbm_handle *h, int32_t nsteps) {
         if (fs) {
             const int64_t slot = h->force_count % kRing;
             L.force = h->d_force_ring + slot * 10;
-            CK(h, cudaMemsetAsync(L.force, 0, 10 * sizeof(double), h->stream));
+            // the node-list kernel zeroes the slot
+            if (h->n_list == 0) CK(h, cudaMemsetAsync(L.force, 0, 10 * sizeof(double), h->stream));
             h->force_steps[slot] = it;
             ++h->force_count;
         }
         const bool sums = ds || ws;
         if (sums) L.diag_part = h->d_diag_part;
-        // the node-list kernel reads only the state before the step: it runs on its own stream beside
-        // the step kernel; the wall kernel reads the stencil snapshots of both
+        // The node-list kernel reads only the state before the step: it runs on its own stream beside the step
+        // kernel, and starts when the last CTA of that has: a step CTA needs a whole SM and would wait until
+        // the list runs out of blocks (annulus 29.9 -> 26.1 ms per 100 steps).  The wall kernel reads the stencil
+        // snapshots of both.
+        if (h->n_list > 0 && h->n_items > 0) L.placed = h->ev_fork;
+        if (h->n_items > 0) CK(h, launch_step(L, h->storage, h->tile_y, h->special, h->stream));
         if (h->n_list > 0) {
-            CK(h, cudaEventRecord(h->ev_fork, h->stream));
+            if (!L.placed) CK(h, cudaEventRecord(h->ev_fork, h->stream));
             CK(h, cudaStreamWaitEvent(h->list_stream, h->ev_fork, 0));
-            CK(h, launch_special_list(L, h->storage, h->n_list_blocks, sums ? h->d_diag_part + 2 * (size_t)h->n_ctas * h->tile_y : nullptr,
+            CK(h, launch_special_list(L, h->storage, h->n_list_blocks,
+                                      sums ? h->d_diag_part + 2 * (size_t)h->n_ctas * h->tile_y : nullptr,
                                       h->list_stream));
             CK(h, cudaEventRecord(h->ev_list, h->list_stream));
+            CK(h, cudaStreamWaitEvent(h->stream, h->ev_list, 0));
         }
-        if (h->n_items > 0) CK(h, launch_step(L, h->storage, h->tile_y, h->special, h->stream));
-        if (h->n_list > 0) CK(h, cudaStreamWaitEvent(h->stream, h->ev_list, 0));
         if (nb > 0) CK(h, launch_wall(L, h->storage, nb, nbf, h->stream));
         if (h->ps_start >= 0 && it >= h->ps_start && it <= h->ps_end) {
             // statistics window: the post-step state (buffer parity ^ 1), as the reference's
@@ -1049,8 +1061,17 @@ void batch_free_tables(mrlbm_batch *b) {
 // Tile every case with (ty, lz) and rebuild the merged work-item and block tables.
 int batch_set_tiling(mrlbm_batch *b, int ty, int lz) {
     BCK(cudaStreamSynchronize(b->stream));
+    int l = lz;
+    if (l <= 0) {
+        std::vector<int> tiles, nz;
+        for (const mrlbm_handle *h : b->h) {
+            tiles.push_back(((h->d.nx + TILE_X - 1) / TILE_X) * ((h->d.ny + ty - 1) / ty));
+            nz.push_back(h->d.nz);
+        }
+        l = choose_batch_lz(tiles, nz, b->storage, b->h[0]->n_sm, ty);
+    }
     for (mrlbm_handle *h : b->h) {
-        const int rc = setup_tiling(h, ty, lz);
+        const int rc = setup_tiling(h, ty, l);
         if (rc != MRLBM_OK) return rc;
     }
     batch_free_tables(b);

@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cstdint>
+#include <vector>
 #include <string>
 
 #include <cuda_runtime.h>
@@ -114,6 +115,7 @@ struct StepLaunch {
     double *force = nullptr;       // [2][5] FP64 accumulators of a sampled step, or null
     double *diag_part = nullptr;   // [n_ctas][tile_y][2] mass / energy partials, or null
     int n_ctas = 0;                // special: one per work item
+    cudaEvent_t placed = nullptr;  // recorded when the last CTA of the step kernel has started, or null
 };
 
 // Stencil-buffer index of node (x, y, z) for a special tile slot.
@@ -132,8 +134,10 @@ cudaError_t launch_wall_batch(const BatchArgs *ba, int parity, int force, int st
 // Zero the slot of every case's force ring and publish the slot for the batched wall kernel.
 cudaError_t launch_batch_force_begin(double *const *ring, int n_cases, int slot, int *d_slot, cudaStream_t s);
 // Tile height (4, 8 or 16; any other value on entry: the default) and z-segment length (> 0 on entry:
-// kept, clipped to nz).
-void choose_tiling(int nx, int ny, int nz, int storage, int n_sm, int &ty, int &lz);
+// kept, clipped to nz); active: tiles that are updated (0: all); list_nodes: nodes of the node-list kernel.
+void choose_tiling(int nx, int ny, int nz, int storage, int n_sm, int &ty, int &lz, int active = 0, int list_nodes = 0);
+// z-segment length of a batch's merged items: tiles[c] of nz[c] planes each.
+int choose_batch_lz(const std::vector<int> &tiles, const std::vector<int> &nz, int storage, int n_sm, int ty);
 int step_kernel_max_ctas_per_sm(int storage, int tile_y);
 // Curved-wall closure + collision for the nb wall nodes of both walls, plus, on a sampled step, the force
 // sums over them and the nbf fluid nodes beside the walls.

@@ -20,6 +20,8 @@
 //   evaluate_incoming_moments_rotated   MRLBM_3D/src/boundary/curvedLBM.cu:5-59
 //   moment_collision                    MRLBM_3D/src/solver/mlbm.cu:3-16
 //   compute_force_mass_kernel (BCFLUID part)  MRLBM_3D/src/statistics/forces.cu:25-133
+#include <type_traits>
+
 #include "mrlbm_internal.h"
 #include "storage.cuh"
 
@@ -68,6 +70,42 @@ __host__ __device__ constexpr int direction(int cx, int cy, int cz) {
     return -1;
 }
 
+// One population f_(cx, CY, CZ) from the stored values of its node, cx at run time: reconstruct_h, whose
+// populations all have the form W [fma(q, s, fma(n, c, r E))] with s = (cx ux + CY uy) + CZ uz and
+// c = (cx CY mxy + cx CZ mxz) + CY CZ myz.  Signs and zeros are exact, and the weights are powers of two
+// apart (as floats too), so this rounds as reconstruct_h does in all 27 cases.
+static_assert(kW0 == 16.0f * kW2 && kW1 == 4.0f * kW2 && 4.0f * kW3 == kW2, "weights are powers of two apart");
+template <typename S, int CY, int CZ>
+__device__ __forceinline__ float population(const float v[10], int cx, float rho0, const StorageScale &sc) {
+    const bool f32 = std::is_same<S, float>::value;
+    const float h3 = f32 ? 3.0f : __fmul_rn(3.0f, sc.is[1]), h15 = f32 ? 1.5f : __fmul_rn(1.5f, sc.is[2]);
+    const float h45 = f32 ? 4.5f : __fmul_rn(4.5f, sc.is[2]), h9 = f32 ? 9.0f : __fmul_rn(9.0f, sc.is[2]);
+    const float rho = f32 ? __fadd_rn(rho0, v[0]) : __fmaf_rn(v[0], sc.is[0], rho0);
+    const float ux = v[1], uy = v[2], uz = v[3], mxx = v[4], myy = v[5], mzz = v[6], mxy = v[7], mxz = v[8], myz = v[9];
+    const float sx = (float)cx;  // products with it are exact
+    const float t = __fadd_rn(__fadd_rn(mxx, myy), mzz);
+    const float p0 = __fmaf_rn(-h15, t, 1.0f);
+    const float a0 = cx ? __fmaf_rn(h45, mxx, p0) : p0;
+    float e = a0;
+    if constexpr (CY != 0 && CZ != 0) e = cx ? __fmaf_rn(h45, t, p0) : __fmaf_rn(h45, mzz, __fmaf_rn(h45, myy, p0));
+    else if constexpr (CY != 0) e = __fmaf_rn(h45, myy, a0);
+    else if constexpr (CZ != 0) e = __fmaf_rn(h45, mzz, a0);
+    const float r = __fmul_rn(rho, kW2), q = __fmul_rn(h3, r), n = __fmul_rn(h9, r);
+    float f = __fmul_rn(r, e);
+    if constexpr (CY != 0 || CZ != 0) {
+        float c = CY == 0 ? 0.f : (CY > 0 ? sx * mxy : -(sx * mxy));
+        if constexpr (CZ != 0) c = CY == 0 ? (CZ > 0 ? sx * mxz : -(sx * mxz)) : __fadd_rn(c, CZ > 0 ? sx * mxz : -(sx * mxz));
+        if constexpr (CY * CZ != 0) c = CY * CZ > 0 ? __fadd_rn(c, myz) : __fsub_rn(c, myz);
+        f = __fmaf_rn(n, c, f);
+    }
+    float s = sx * ux;
+    if constexpr (CY != 0) s = CY > 0 ? __fadd_rn(s, uy) : __fsub_rn(s, uy);
+    if constexpr (CZ != 0) s = CZ > 0 ? __fadd_rn(s, uz) : __fsub_rn(s, uz);
+    f = __fmaf_rn(q, s, f);
+    constexpr float w = (CY ? 1.0f : 4.0f) * (CZ ? 1.0f : 4.0f) * 0.25f;
+    return f * (cx ? w : 4.0f * w);
+}
+
 // The populations of `mask` pulled by node (x, y, z) with this c_x, on the grid that wraps in every
 // axis, into f[direction * stride].  Three lanes share a node, one per c_x: the three neighbours
 // of a row mostly lie on one line, and the kernel is bound by the rate at which scattered loads touch
@@ -80,26 +118,34 @@ __device__ __forceinline__ void pull(const StepArgs &a, const S *__restrict__ sr
     const int gx = wrap(x - cx, a.nx);
     const uint32_t *__restrict__ p = reinterpret_cast<const uint32_t *>(src) + (gx >> 5) * (WPN * kXBlock) + (gx & 31);
     const int64_t row = (int64_t)a.nxb * (WPN * kXBlock);
+    // the loads of all nine rows go out together
+    Raw<S> raw[9];
 #pragma unroll
     for (int cz = -1; cz <= 1; ++cz) {
-        const int64_t plane = (int64_t)wrap(z - cz, a.nz) * a.ny;
-        // the loads of the three rows of this plane go out together
-        Raw<S> raw[3];
+        const int64_t first = (int64_t)wrap(z - cz, a.nz) * a.ny;
 #pragma unroll
         for (int cy = -1; cy <= 1; ++cy) {
+            const int r = 3 * (cz + 1) + cy + 1;
             const int q = cx < 0 ? direction(-1, cy, cz) : (cx > 0 ? direction(1, cy, cz) : direction(0, cy, cz));
-            if (mask >> q & 1u) load_raw_words<S>(p + (plane + wrap(y - cy, a.ny)) * row, raw[cy + 1]);
-            else raw[cy + 1] = Raw<S>{};
-        }
-#pragma unroll
-        for (int cy = -1; cy <= 1; ++cy) {
-            const int q = cx < 0 ? direction(-1, cy, cz) : (cx > 0 ? direction(1, cy, cz) : direction(0, cy, cz));
-            float v[10], g[27];
-            raw_values<S>(raw[cy + 1], v);
-            rebuild<S>(v, a.rho0, a.sc, g);
-            f[q * stride] = cx < 0 ? g[direction(-1, cy, cz)] : (cx > 0 ? g[direction(1, cy, cz)] : g[direction(0, cy, cz)]);
+            if (mask >> q & 1u) load_raw_words<S>(p + (first + wrap(y - cy, a.ny)) * row, raw[r]);
+            else raw[r] = Raw<S>{};
         }
     }
+    auto put = [&](auto cyc, auto czc) {
+        constexpr int cy = decltype(cyc)::value, cz = decltype(czc)::value;
+        const int q = cx < 0 ? direction(-1, cy, cz) : (cx > 0 ? direction(1, cy, cz) : direction(0, cy, cz));
+        float v[10];
+        raw_values<S>(raw[3 * (cz + 1) + cy + 1], v);
+        f[q * stride] = population<S, cy, cz>(v, cx, a.rho0, a.sc);
+    };
+    auto plane = [&](auto czc) {
+        put(std::integral_constant<int, -1>{}, czc);
+        put(std::integral_constant<int, 0>{}, czc);
+        put(std::integral_constant<int, 1>{}, czc);
+    };
+    plane(std::integral_constant<int, -1>{});
+    plane(std::integral_constant<int, 0>{});
+    plane(std::integral_constant<int, 1>{});
 }
 
 // Populations that the closure of a listed node uses.
@@ -188,14 +234,14 @@ __device__ __forceinline__ int special_node(const StepArgs &a, int parity, bool 
     return fluid ? 2 : 1;
 }
 
-// A warp takes 30 nodes at a time: three rounds of ten nodes x three lanes gather the populations into
+// A warp takes kListNodes nodes at a time: rounds of ten nodes x three lanes gather the populations into
 // shared memory, then one lane per node applies its closure.
-constexpr int kListWarps = 4, kListThreads = 32 * kListWarps, kListNodes = 30;
+constexpr int kListWarps = 4, kListThreads = 32 * kListWarps, kListNodes = 10;
 
 // BATCH: each block serves the case named by its entry in BatchArgs::list_blocks.
 template <typename S, bool BATCH>
 __global__ void __launch_bounds__(kListThreads)
-    special_list_kernel(const StepArgs *__restrict__ ga, const BatchArgs *__restrict__ ba, int parity, int force,
+    special_list_kernel(const StepArgs *__restrict__ ga, const BatchArgs *__restrict__ ba, int parity, double *force,
                         double *__restrict__ diag_part) {
     __shared__ float gathered[kListWarps][27][kListNodes + 1];
     int b0 = blockIdx.x, nblk = gridDim.x;
@@ -206,13 +252,15 @@ __global__ void __launch_bounds__(kListThreads)
         nblk = m.z;
     }
     const StepArgs &a = *ga;
+    // a sampled step: the wall kernel, launched after this one, adds into the slot
+    if (!BATCH && force && blockIdx.x == 0 && threadIdx.x < 10) force[threadIdx.x] = 0.0;
     S *__restrict__ dst = (S *)a.m[parity ^ 1];
     const int n_all = a.n_list;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double dm = 0.0, de = 0.0;
     for (int first = (b0 * kListWarps + warp) * kListNodes; first < n_all; first += nblk * kListWarps * kListNodes) {
 #pragma unroll 1
-        for (int r = 0; r < 3; ++r) {
+        for (int r = 0; r < kListNodes / 10; ++r) {
             const int j = 10 * r + lane / 3, i = first + j;
             if (lane < 30 && i < n_all) {
                 const uint64_t p = a.list_xyz[i];
@@ -232,7 +280,7 @@ __global__ void __launch_bounds__(kListThreads)
             const int tx = x / TILE_X, ty = y / a.tile_y;
             const int slot = a.tile_slot[ty * a.tiles_x + tx];
             Mom m;
-            const int code = special_node<S>(a, parity, force != 0, w, f, x, y, z, slot, tx * TILE_X, ty * a.tile_y, m);
+            const int code = special_node<S>(a, parity, force != nullptr, w, f, x, y, z, slot, tx * TILE_X, ty * a.tile_y, m);
             if (code) {
                 const int64_t ai = aos_at<S>(x, y, z, a.nxb, a.ny);
                 if (kScaled<S> && a.sr_step)
@@ -280,7 +328,7 @@ int special_list_blocks(int n_list) {
 }
 
 cudaError_t launch_special_list(const StepLaunch &l, int storage, int n_blocks, double *diag_part, cudaStream_t s) {
-    const int f = l.force != nullptr;
+    double *const f = l.force;
     switch (storage) {
         case MRLBM_STORAGE_F32:
             special_list_kernel<float, false><<<n_blocks, kListThreads, 0, s>>>(l.ga, nullptr, l.parity, f, diag_part);
@@ -304,20 +352,22 @@ cudaError_t launch_special_list(const StepLaunch &l, int storage, int n_blocks, 
 cudaError_t launch_special_list_batch(const BatchArgs *ba, int parity, int force, int storage, int n_blocks,
                                       cudaStream_t s) {
     if (n_blocks <= 0) return cudaSuccess;
+    // any non-null pointer makes it a sampled step (the batch has zeroed its cases' slots)
+    double *const f = force ? reinterpret_cast<double *>(1) : nullptr;
     switch (storage) {
         case MRLBM_STORAGE_F32:
-            special_list_kernel<float, true><<<n_blocks, kListThreads, 0, s>>>(nullptr, ba, parity, force, nullptr);
+            special_list_kernel<float, true><<<n_blocks, kListThreads, 0, s>>>(nullptr, ba, parity, f, nullptr);
             break;
         case MRLBM_STORAGE_F16:
-            special_list_kernel<__half, true><<<n_blocks, kListThreads, 0, s>>>(nullptr, ba, parity, force, nullptr);
+            special_list_kernel<__half, true><<<n_blocks, kListThreads, 0, s>>>(nullptr, ba, parity, f, nullptr);
             break;
         case MRLBM_STORAGE_BF16:
             special_list_kernel<__nv_bfloat16, true>
-                <<<n_blocks, kListThreads, 0, s>>>(nullptr, ba, parity, force, nullptr);
+                <<<n_blocks, kListThreads, 0, s>>>(nullptr, ba, parity, f, nullptr);
             break;
         case MRLBM_STORAGE_F16_U32:
             special_list_kernel<HybridWord, true>
-                <<<n_blocks, kListThreads, 0, s>>>(nullptr, ba, parity, force, nullptr);
+                <<<n_blocks, kListThreads, 0, s>>>(nullptr, ba, parity, f, nullptr);
             break;
         default: return cudaErrorInvalidValue;
     }

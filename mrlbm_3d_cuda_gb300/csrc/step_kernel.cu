@@ -366,7 +366,6 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
         // Otherwise the CTAs stride through the items.
         const bool leader = threadIdx.x == 32 * TY;
         for (int it = blockIdx.x; it >= 0 && it < n_items;) {
-            if (SPECIAL && leader) takeover_request(s_slot + (n & 1), &s_taken);
             int2 head;
             if constexpr (BATCH) head = ba->items[it];
             else head = make_int2(0, single.items ? single.items[it] : (it % (single.tiles_x * single.tiles_y)) |
@@ -411,8 +410,13 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
             const int mine = (hw + G::NH - q % G::NH) % G::NH;  // this warp's first plane of the item
             int zk = (zs == 0 ? nz - 1 : zs - 1) + mine;
             if (zk >= nz) zk -= nz;
+            // The next item is asked for as the last planes of this one are issued: the answer is there before
+            // their stages are free, and an item whose CTA is only late (the node-list kernel's blocks are in
+            // its place) is not put behind this one's whole length (an annulus of 132 items: 321 -> 265 us a step).
+            if (SPECIAL && leader && mine > last) takeover_request(s_slot + (n & 1), &s_taken);
             for (int k = 0; k <= last; ++k, ++q, next_stage()) {
                 if ((k - mine) % G::NH != 0) continue;
+                if (SPECIAL && leader && k + G::NH > last) takeover_request(s_slot + (n & 1), &s_taken);
                 // The halo warps wait for a free stage in turn, each asleep at a hardware barrier until the one
                 // before it has passed (polling costs issue slots).  Plane q waits for the release of plane
                 // q - D; the turn before has seen that of q - 1 - D, so the release two uses back on the stage
@@ -806,11 +810,22 @@ cudaError_t configure_t() {
 }
 
 template <typename S, int TY, bool SP, bool BATCH>
-cudaError_t launch_t(const StepArgs &a, const BatchArgs *ba, int parity, double *diag_part, int n_ctas, cudaStream_t s) {
+cudaError_t launch_t(const StepArgs &a, const BatchArgs *ba, int parity, double *diag_part, int n_ctas, cudaStream_t s,
+                     cudaEvent_t placed = nullptr) {
     const cudaError_t e = configure_t<S, TY, SP, BATCH>();
     if (e != cudaSuccess) return e;
-    step_kernel<S, TY, SP, BATCH><<<n_ctas, Geo<S, TY, SP>::NTH, Geo<S, TY, SP>::SMEM, s>>>(a, ba, parity, diag_part);
-    return cudaGetLastError();
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeLaunchCompletionEvent;
+    at[0].val.launchCompletionEvent.event = placed;
+    at[0].val.launchCompletionEvent.flags = 0;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(n_ctas);
+    c.blockDim = dim3(Geo<S, TY, SP>::NTH);
+    c.dynamicSmemBytes = Geo<S, TY, SP>::SMEM;
+    c.stream = s;
+    c.attrs = at;
+    c.numAttrs = placed ? 1 : 0;
+    return cudaLaunchKernelEx(&c, step_kernel<S, TY, SP, BATCH>, a, ba, parity, diag_part);
 }
 
 // Run f(storage type tag, tile-height tag) for the storage mode and tile height.
@@ -844,8 +859,8 @@ cudaError_t launch_step(const StepLaunch &l, int storage, int tile_y, bool speci
     if (!known(storage, tile_y)) return cudaErrorInvalidValue;
     return dispatch(storage, tile_y, [&](auto t, auto ty) {
         using S = typename decltype(t)::type;
-        return special ? launch_t<S, ty(), true, false>(*l.args, nullptr, l.parity, l.diag_part, l.n_ctas, s)
-                       : launch_t<S, ty(), false, false>(*l.args, nullptr, l.parity, l.diag_part, l.n_ctas, s);
+        return special ? launch_t<S, ty(), true, false>(*l.args, nullptr, l.parity, l.diag_part, l.n_ctas, s, l.placed)
+                       : launch_t<S, ty(), false, false>(*l.args, nullptr, l.parity, l.diag_part, l.n_ctas, s, l.placed);
     });
 }
 
@@ -883,24 +898,54 @@ int step_kernel_max_ctas_per_sm(int storage, int tile_y) {
     });
 }
 
-void choose_tiling(int nx, int ny, int nz, int storage, int n_sm, int &ty, int &lz) {
+// A work item of l planes costs about 2 l + 7 units (of half a plane: filling and draining its pipeline is
+// the 7).  The node-list kernel runs beside the step kernel on the SMs that have no item, its rest after
+// it: 0.03 units of an SM per node in FP32 (annulus: 196 k nodes, 69 us on 152 SMs, a unit 1.56 us),
+// less with fewer words a node, and a block's latency of 5 units at least.  With that term a channel of 16
+// planes takes l = 3 instead of 2 (31.3 instead of 40.0 us a step), an annulus of 129 planes 52 instead of 43
+// (237, 247; 24: 253, 64: 252).
+void choose_tiling(int nx, int ny, int nz, int storage, int n_sm, int &ty, int &lz, int active, int list_nodes) {
     if (ty != 4 && ty != 8 && ty != 16) ty = 16;
-    const int64_t slots = (int64_t)std::max(1, step_kernel_max_ctas_per_sm(storage, ty)) * n_sm;
-    const int64_t tiles = (int64_t)((nx + TILE_X - 1) / TILE_X) * ((ny + ty - 1) / ty);
     if (lz > 0) {
         lz = std::min(nz, lz);
         return;
     }
-    int64_t best = INT64_MAX;
+    const int64_t slots = (int64_t)std::max(1, step_kernel_max_ctas_per_sm(storage, ty)) * n_sm;
+    const int64_t tiles = active > 0 ? active : (int64_t)((nx + TILE_X - 1) / TILE_X) * ((ny + ty - 1) / ty);
+    const double list = (storage == MRLBM_STORAGE_F32 ? 0.03 : (storage == MRLBM_STORAGE_F16_U32 ? 0.024 : 0.02)) * list_nodes;
+    double best = 1e300;
     for (int nseg = 1; nseg <= std::min(nz, 1 << 11); ++nseg) {
         const int l = (nz + nseg - 1) / nseg;
-        const int64_t waves = (tiles * ((nz + l - 1) / l) + slots - 1) / slots;
-        const int64_t cost = waves * (2 * l + 7);
+        const int64_t items = tiles * ((nz + l - 1) / l), t = (items + slots - 1) / slots * (2 * l + 7);
+        const double rest = list - (double)(slots * t - items * (2 * l + 7));
+        const double cost = (double)t + (rest > 0.0 ? std::max(rest / (double)slots, 5.0) : 0.0);
         if (cost < best) {
             best = cost;
             lz = l;
         }
     }
+}
+
+// A batch has many more items than the SMs hold, and a CTA takes the next one as it finishes: the items'
+// total counts (long segments), and half of the longest as the tail.
+int choose_batch_lz(const std::vector<int> &tiles, const std::vector<int> &nz, int storage, int n_sm, int ty) {
+    const double slots = (double)std::max(1, step_kernel_max_ctas_per_sm(storage, ty)) * n_sm;
+    const int top = *std::max_element(nz.begin(), nz.end());
+    double best = 1e300;
+    int lz = 1;
+    for (int l = 1; l <= top; ++l) {
+        double work = 0.0;
+        for (size_t c = 0; c < nz.size(); ++c) {
+            const int seg = (nz[c] + l - 1) / l;
+            work += (double)tiles[c] * (2.0 * nz[c] + 7.0 * seg);
+        }
+        const double cost = work / slots + 0.5 * (2.0 * l + 7.0);
+        if (cost < best) {
+            best = cost;
+            lz = l;
+        }
+    }
+    return lz;
 }
 
 // ---- allocation-free periodic step --------------------------------------------------------
