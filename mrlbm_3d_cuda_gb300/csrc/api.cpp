@@ -313,7 +313,7 @@ int step_handle(mrlbm_handle *h, int32_t nsteps) {
             CK(h, cudaEventRecord(h->ev_list, h->list_stream));
             CK(h, cudaStreamWaitEvent(h->stream, h->ev_list, 0));
         }
-        if (nb > 0) CK(h, launch_wall(L, h->storage, nb, nbf, h->stream));
+        if (nb > 0) CK(h, launch_wall(L, h->storage, nb + (fs ? nbf : 0), h->stream));
         if (h->ps_start >= 0 && it >= h->ps_start && it <= h->ps_end) {
             // statistics window: the post-step state (buffer parity ^ 1), as the reference's
             // post_process_step samples it
@@ -1092,10 +1092,10 @@ int batch_set_tiling(mrlbm_batch *b, int ty, int lz) {
             const int first = (int)lblocks.size();
             for (int k = 0; k < h->n_list_blocks; ++k) lblocks.push_back(make_int4(c, first, h->n_list_blocks, 0));
         }
-        const int nw = (int)(h->geo.wall[0].list.size() + h->geo.wall[1].list.size());
-        const int nf = (int)(h->geo.wall[0].fluid_list.size() + h->geo.wall[1].fluid_list.size());
+        const int nw = (int)(h->geo.wall[0].list.size() + h->geo.wall[1].list.size() +
+                             h->geo.wall[0].fluid_list.size() + h->geo.wall[1].fluid_list.size());
         if (nw > 0) {
-            const int first = (int)wblocks.size(), nblk = wall_kernel_blocks(b->storage, nw, nf);
+            const int first = (int)wblocks.size(), nblk = (nw + 127) / 128;
             for (int k = 0; k < nblk; ++k) wblocks.push_back(make_int4(c, first, nblk, 0));
         }
     }

@@ -139,10 +139,8 @@ void choose_tiling(int nx, int ny, int nz, int storage, int n_sm, int &ty, int &
 // z-segment length of a batch's merged items: tiles[c] of nz[c] planes each.
 int choose_batch_lz(const std::vector<int> &tiles, const std::vector<int> &nz, int storage, int n_sm, int ty);
 int step_kernel_max_ctas_per_sm(int storage, int tile_y);
-// Curved-wall closure + collision for the nb wall nodes of both walls, plus, on a sampled step, the force
-// sums over them and the nbf fluid nodes beside the walls.
-cudaError_t launch_wall(const StepLaunch &l, int storage, int nb, int nbf, cudaStream_t s);
-int wall_kernel_blocks(int storage, int nb, int nbf);
+// Curved-wall closure + collision for the wall nodes of both walls, plus the force sums.
+cudaError_t launch_wall(const StepLaunch &l, int storage, int n_total, cudaStream_t s);
 // Closures, stencil snapshots and collision of the listed nodes (reads the state before the step
 // only: independent of launch_step).
 int special_list_blocks(int n_list);

@@ -21,8 +21,6 @@
 namespace mrlbm {
 namespace {
 
-constexpr int kWallThreads = 128, kWallNodes = kWallThreads / 2;  // threads a block; nodes in pairs
-
 struct VM {
     float ux, uy, uz, mxx, myy, mzz, mxy, mxz, myz;
 };
@@ -258,321 +256,19 @@ __global__ void __launch_bounds__(128)
     if (threadIdx.x < 10) atomicAdd(force + threadIdx.x, red[threadIdx.x][0]);
 }
 
-// ---- FP32 storage: two lanes a node ------------------------------------------------------------
-// The kernel is a chain of dependent scattered loads (node, tile slot, nine side-buffer entries) and then
-// of 27 x 30 dependent sums; DRAM, L2 and issue slots are all below 45 %.  Two lanes a node, one per
-// probe point and per equation of the closure, halve what a lane loads (80 -> 40 values in flight, 128 -> 96
-// registers) and sums: 139 k wall nodes of an annulus 50 -> 36 us, 12 k of a cylinder 18 -> 12 us.
-// The compiler fuses products and sums here in another order than in wall_kernel: of the wall nodes of an
-// annulus 1 in 2000 ends a step one ulp from it.  FP32 fields stay within 4e-6 over 100 steps, but 16-bit storage
-// turns such an ulp into one of its own, so those modes keep the kernel of one lane a node.
-
-// The ten moments of a side-buffer entry, 16 bytes a load: a lane's entry is 64 bytes of its own.
-__device__ __forceinline__ void load_entry(const float *e, float v[10]) {
-    const float4 a = reinterpret_cast<const float4 *>(e)[0], b = reinterpret_cast<const float4 *>(e)[1];
-    const float2 c = reinterpret_cast<const float2 *>(e)[4];
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-    v[8] = c.x; v[9] = c.y;
-}
-
-// The four side-buffer entries around a probe point in the plane z, and the point's place among them.
-struct Corners {
-    const float *p00, *p10, *p01, *p11;
-    float xd, yd;
-};
-__device__ __forceinline__ bool locate(const StepArgs &a, float px, float py, int z, Corners &c) {
-    const int x0 = (int)floorf(px), y0 = (int)floorf(py);
-    c.xd = px - (float)x0;
-    c.yd = py - (float)y0;
-    c.p00 = side_entry(a, x0, y0, z);
-    c.p10 = side_entry(a, x0 + 1, y0, z);
-    c.p01 = side_entry(a, x0, y0 + 1, z);
-    c.p11 = side_entry(a, x0 + 1, y0 + 1, z);
-    return c.p00 && c.p10 && c.p01 && c.p11;
-}
-
-// interp_rotate from loaded entries.
-__device__ __forceinline__ void interp_rotate_pair(const float q00[10], const float q10[10], const float q01[10],
-                                              const float q11[10], float xd, float yd, float nx, float ny, VM &vm) {
-    float v[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) {
-        const float r0 = (1.0f - xd) * q00[k + 1] + xd * q10[k + 1];
-        const float r1 = (1.0f - xd) * q01[k + 1] + xd * q11[k + 1];
-        v[k] = (1.0f - yd) * r0 + yd * r1;
-    }
-    const float ux = v[0], uy = v[1], uz = v[2], mxx = v[3], myy = v[4], mzz = v[5], mxy = v[6], mxz = v[7],
-                myz = v[8];
-    const float c = nx, s = ny;
-    const float s2 = 2.0f * s * c, c2 = c * c - s * s;
-    vm.ux = ux * c + uy * s;
-    vm.uy = -ux * s + uy * c;
-    vm.uz = uz;
-    vm.mxx = mxx * c * c + myy * s * s + mxy * s2;
-    vm.myy = mxx * s * s + myy * c * c - mxy * s2;
-    vm.mzz = mzz;
-    vm.mxy = mxy * c2 + 0.5f * (myy - mxx) * s2;
-    vm.mxz = mxz * c + myz * s;
-    vm.myz = myz * c - mxz * s;
-}
-
-__device__ __forceinline__ float extrapolate_pair(float d, float vw, float v1, float v2) {
-    const float d2 = d * d;
-    const float c1 = 1.0f - 0.5f * d2 + 1.5f * d;
-    const float c2 = d2 - 2.0f * d;
-    const float c3 = -0.5f * (d2 - d);
-    return __fmaf_rn(c3, v2, __fmaf_rn(c2, v1, __fmul_rn(c1, vw)));
-}
-
-// closure_rotated by two adjacent lanes for one node, the even one (odd = false) for the sums of the m'_xy
-// equation, the odd one for m'_xz's; both return the closed moments.
-__device__ void closure_rotated_pair(const StepArgs &a, bool odd, float c, float s, uint32_t inm, uint32_t outm, const VM &e,
-                                Mom &m) {
-    const float s2 = 2.0f * s * c, c2 = c * c - s * s;
-    constexpr float cbf = 4.5f;  // 0.5 * 3 * 3
-    float A = 0.f, E = 0.f, D = 0.f;
-    float B11 = 0.f, B22 = 0.f, B33 = 0.f, B12 = 0.f, B13 = 0.f, B23 = 0.f;
-    float F11 = 0.f, F22 = 0.f, F33 = 0.f, F12 = 0.f, F13 = 0.f, F23 = 0.f;
-    const bool strong = a.wall_strong != 0;
-#pragma unroll
-    for (int q = 0; q < 27; ++q) {
-        const float cx = (float)cxq(q), cy = (float)cyq(q), cz = (float)czq(q);
-        const float cxp = cx * c + cy * s;
-        const float cyp = -cx * s + cy * c;
-        const float czp = cz;
-        const float hxx = cxp * cxp - kCs2, hyy = cyp * cyp - kCs2, hzz = czp * czp - kCs2;
-        const float hxy = cxp * cyp, hxz = cxp * czp, hyz = cyp * czp;
-        const float wq = weight(q);
-        const float cf = cbf * wq;
-        const float Ai = wq * (1.0f + 3.0f * (e.ux * cxp + e.uy * cyp + e.uz * czp));
-        const float Ei = Ai + cf * (e.ux * e.ux * hxx + e.uy * e.uy * hyy + e.uz * e.uz * hzz + 2.0f * e.ux * e.uy * hxy +
-                                    2.0f * e.ux * e.uz * hxz + 2.0f * e.uy * e.uz * hyz);
-        if (strong ? (outm & (1u << q)) != 0 : false) {
-            A += Ai;
-            E += Ei;
-            B11 += cf * hxx; B22 += cf * hyy; B33 += cf * hzz;
-            B12 += cf * hxy; B13 += cf * hxz; B23 += cf * hyz;
-        }
-        if (inm & (1u << q)) {
-            if (!strong) E += Ei;
-            const float h = odd ? hxz : hxy;
-            D += Ai * h;
-            F11 += (cf * hxx) * h; F22 += (cf * hyy) * h; F33 += (cf * hzz) * h;
-            F12 += (cf * hxy) * h; F13 += (cf * hxz) * h; F23 += (cf * hyz) * h;
-        }
-    }
-    const float rhoI = m.rho, mI = odd ? m.mxz : m.mxy;
-    float G = E;
-    if (strong) {
-        const float om1 = 1.0f - a.omega;
-        G = om1 * A + a.omega * E;
-        const float t = om1 * mI;
-        F11 -= t * B11; F22 -= t * B22; F33 -= t * B33; F12 -= t * B12; F13 -= t * B13; F23 -= t * B23;
-    }
-    const float R = G * mI - D;
-    const float ca = 2.0f * F12, cb = 2.0f * F13;
-    const float cc = R - e.mxx * F11 - e.myy * F22 - e.mzz * F33 - 2.0f * e.myz * F23;
-    // the two equations a1 m'_xy + b1 m'_xz = c1 (even lane) and a2 m'_xy + b2 m'_xz = c2 (odd lane)
-    const unsigned pair = 3u << (threadIdx.x & 30u);
-    const float oa = __shfl_xor_sync(pair, ca, 1), ob = __shfl_xor_sync(pair, cb, 1), oc = __shfl_xor_sync(pair, cc, 1);
-    const float a1 = odd ? oa : ca, b1 = odd ? ob : cb, c1 = odd ? oc : cc;
-    const float a2 = odd ? ca : oa, b2 = odd ? cb : ob, c2v = odd ? cc : oc;
-    const float inv = 1.0f / (a2 * b1 - a1 * b2);
-    const float mxyp = (b1 * c2v - b2 * c1) * inv;
-    const float mxzp = (a2 * c1 - a1 * c2v) * inv;
-    m.ux = e.ux * c - e.uy * s;
-    m.uy = e.ux * s + e.uy * c;
-    m.uz = e.uz;
-    m.mxx = e.mxx * c * c + e.myy * s * s - mxyp * s2;
-    m.myy = e.mxx * s * s + e.myy * c * c + mxyp * s2;
-    m.mzz = e.mzz;
-    m.mxy = (e.mxx - e.myy) * 0.5f * s2 + mxyp * c2;
-    m.mxz = mxzp * c - e.myz * s;
-    m.myz = mxzp * s + e.myz * c;
-    if (strong) {
-        const float om1 = 1.0f - a.omega;
-        const float den = G + om1 * (e.mxx * B11 + e.myy * B22 + e.mzz * B33 + 2.0f * mxyp * B12 + 2.0f * mxzp * B13 +
-                                     2.0f * e.myz * B23);
-        m.rho = rhoI / den;
-    } else {
-        m.rho = rhoI / E;
-    }
-}
-
-// Coordinates of a node from its index.
-__device__ __forceinline__ void coordinates(int64_t node, int nx, int ny, int &x, int &y, int &z) {
-    const int64_t plane = (int64_t)nx * ny;
-    if (((node | plane) >> 32) == 0) {  // 32-bit divisions cost a third
-        const uint32_t row = (uint32_t)node / (uint32_t)nx;
-        x = (int)((uint32_t)node - row * (uint32_t)nx);
-        z = (int)(row / (uint32_t)ny);
-        y = (int)(row - (uint32_t)z * (uint32_t)ny);
-    } else {
-        x = (int)(node % nx);
-        y = (int)((node / nx) % ny);
-        z = (int)(node / plane);
-    }
-}
-
-// The first blocks finish the wall nodes, two lanes a node (one per probe point and per equation of
-// the closure); the others add up the force of the fluid nodes beside the walls (force != nullptr).
-// BATCH: each block serves the case named by its entry in BatchArgs::wall_blocks; the force
-// sums of a sampled step go to that case's ring slot BatchArgs::force_slot.
-template <bool BATCH>
-__global__ void __launch_bounds__(kWallThreads)
-    wall_pair_kernel(const StepArgs *__restrict__ ga, const BatchArgs *__restrict__ ba, int parity, double *force) {
-    int b0 = blockIdx.x;
-    if constexpr (BATCH) {
-        const int4 m = ba->wall_blocks[blockIdx.x];
-        ga = ba->cases[m.x];
-        b0 = blockIdx.x - m.y;
-        force = force ? ba->force_ring[m.x] + (int64_t)(*ba->force_slot) * 10 : nullptr;
-    }
-    const StepArgs &a = *ga;
-    const int nb0 = a.wall[0].nb, nb = nb0 + a.wall[1].nb;
-    const int wall_blocks = (nb + kWallNodes - 1) / kWallNodes;
-    int wi = -1;  // the wall that acc belongs to
-    double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    if (b0 < wall_blocks) {
-        const int i = b0 * kWallNodes + (int)(threadIdx.x >> 1);
-        const bool odd = threadIdx.x & 1;
-        if (i < nb) {
-            const int w = i < nb0 ? 0 : 1;
-            const int bi = i < nb0 ? i : i - nb0;
-            const WallArgs &W = a.wall[w];
-            int x, y, z;
-            coordinates(W.list[bi], a.nx, a.ny, x, y, z);
-            const float *e0 = side_entry(a, x, y, z);
-            const float nx = W.nx[bi], ny = W.ny[bi], delta = W.delta[bi];
-            const uint32_t inm = W.in_mask[bi], outm = W.out_mask[bi];
-            const float xw = a.xc + W.r_wall * nx, yw = a.yc + W.r_wall * ny;
-            const float x1 = xw + W.dir * nx, y1 = yw + W.dir * ny;
-            const float x2 = xw + W.dir * 2.0f * nx, y2 = yw + W.dir * 2.0f * ny;
-            Corners c;
-            const bool found = locate(a, odd ? x2 : x1, odd ? y2 : y1, z, c);
-            const unsigned pair = 3u << (threadIdx.x & 30u);
-            if (!e0) {
-                atomicOr(a.error, 1);
-            } else if (!__all_sync(pair, found)) {
-                atomicOr(a.error, 2);
-            } else {
-                // the entries go out together
-                float own[10], q[4][10];
-                load_entry(e0, own);
-                load_entry(c.p00, q[0]);
-                load_entry(c.p10, q[1]);
-                load_entry(c.p01, q[2]);
-                load_entry(c.p11, q[3]);
-                Mom m;
-                m.rho = a.rho0 + own[0];
-                m.ux = own[1]; m.uy = own[2]; m.uz = own[3];
-                m.mxx = own[4]; m.myy = own[5]; m.mzz = own[6];
-                m.mxy = own[7]; m.mxz = own[8]; m.myz = own[9];
-                VM v;
-                interp_rotate_pair(q[0], q[1], q[2], q[3], c.xd, c.yd, nx, ny, v);
-                auto probes = [&](float vw, float mine) {
-                    const float other = __shfl_xor_sync(pair, mine, 1);
-                    return extrapolate_pair(delta, vw, odd ? other : mine, odd ? mine : other);
-                };
-                const float uw = W.u_wall[0], vw = W.u_wall[1], ww = W.u_wall[2];
-                VM ex;
-                ex.ux = probes(uw, v.ux);
-                ex.uy = probes(vw, v.uy);
-                ex.uz = probes(ww, v.uz);
-                ex.mxx = probes(uw * uw, v.mxx);
-                ex.myy = probes(vw * vw, v.myy);
-                ex.mzz = probes(ww * ww, v.mzz);
-                ex.myz = probes(vw * ww, v.myz);
-                ex.mxy = ex.mxz = 0.f;
-                closure_rotated_pair(a, odd, nx, ny, inm, outm, ex, m);
-                // sampled: the even lane sums the incoming populations, the odd one the outgoing ones
-                // of the collided node
-                Mom o = m;
-                collide(o, a.omega);
-                if (!odd) {
-                    const int64_t ai = aos_at<float>(x, y, z, a.nxb, a.ny);
-                    store_mom<float>((float *)a.m[parity ^ 1], ai, o, a.rho0, a.sc);
-                }
-                if (force) {
-                    double f[4];
-                    masked_momentum(odd ? outm : inm, odd ? o : m, f);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) acc[k] = f[k] - __shfl_xor_sync(pair, f[k], 1);  // even: in - out
-                    acc[4] = ((double)x - a.xc) * acc[1] - ((double)y - a.yc) * acc[0];
-                    if (!odd) wi = w;
-                }
-            }
-        }
-    } else if (force) {
-        const int j = (b0 - wall_blocks) * kWallThreads + (int)threadIdx.x;
-        const int nbf0 = a.wall[0].nbf, nbf = nbf0 + a.wall[1].nbf;
-        if (j < nbf) {
-            const int w = j < nbf0 ? 0 : 1;
-            int x, y, z;
-            coordinates(a.wall[w].fluid_list[j < nbf0 ? j : j - nbf0], a.nx, a.ny, x, y, z);
-            const float *e = side_entry(a, x, y, z);
-            if (!e) {
-                atomicOr(a.error, 4);
-            } else {
-                const double fx = e[10], fy = e[11];
-                acc[0] = fx;
-                acc[1] = fy;
-                acc[2] = e[12];
-                acc[3] = e[13];
-                acc[4] = ((double)x - a.xc) * fy - ((double)y - a.yc) * fx;
-                wi = w;
-            }
-        }
-    }
-    if (!force) return;
-    // sums per warp and wall, then over the block's warps; a wall that no lane has adds nothing
-    __shared__ double red[kWallThreads / 32][10];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-#pragma unroll
-    for (int w = 0; w < 2; ++w) {
-        const bool any = __any_sync(0xffffffffu, wi == w);
-#pragma unroll
-        for (int k = 0; k < 5; ++k) {
-            double v = wi == w ? acc[k] : 0.0;
-            if (any)
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-            if (lane == 0) red[warp][5 * w + k] = v;
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x < 10) {
-        double v = 0.0;
-#pragma unroll
-        for (int k = 0; k < kWallThreads / 32; ++k) v += red[k][threadIdx.x];
-        if (v != 0.0) atomicAdd(force + threadIdx.x, v);
-    }
-}
-
 }  // namespace
 
-int wall_kernel_blocks(int storage, int nb, int nbf) {
-    if (storage == MRLBM_STORAGE_F32)
-        return (nb + kWallNodes - 1) / kWallNodes + (nbf + kWallThreads - 1) / kWallThreads;
-    return (nb + nbf + kWallThreads - 1) / kWallThreads;
-}
-
-cudaError_t launch_wall(const StepLaunch &l, int storage, int nb, int nbf, cudaStream_t s) {
-    const int blocks = wall_kernel_blocks(storage, nb, l.force ? nbf : 0);
-    if (blocks <= 0) return cudaSuccess;
+cudaError_t launch_wall(const StepLaunch &l, int storage, int n_total, cudaStream_t s) {
+    if (n_total <= 0) return cudaSuccess;
+    const int blocks = (n_total + 127) / 128;
     switch (storage) {
-        case MRLBM_STORAGE_F32:
-            wall_pair_kernel<false><<<blocks, kWallThreads, 0, s>>>(l.ga, nullptr, l.parity, l.force);
-            break;
-        case MRLBM_STORAGE_F16:
-            wall_kernel<__half, false><<<blocks, kWallThreads, 0, s>>>(l.ga, nullptr, l.parity, l.force);
-            break;
+        case MRLBM_STORAGE_F32: wall_kernel<float, false><<<blocks, 128, 0, s>>>(l.ga, nullptr, l.parity, l.force); break;
+        case MRLBM_STORAGE_F16: wall_kernel<__half, false><<<blocks, 128, 0, s>>>(l.ga, nullptr, l.parity, l.force); break;
         case MRLBM_STORAGE_BF16:
-            wall_kernel<__nv_bfloat16, false><<<blocks, kWallThreads, 0, s>>>(l.ga, nullptr, l.parity, l.force);
+            wall_kernel<__nv_bfloat16, false><<<blocks, 128, 0, s>>>(l.ga, nullptr, l.parity, l.force);
             break;
         case MRLBM_STORAGE_F16_U32:
-            wall_kernel<HybridWord, false><<<blocks, kWallThreads, 0, s>>>(l.ga, nullptr, l.parity, l.force);
+            wall_kernel<HybridWord, false><<<blocks, 128, 0, s>>>(l.ga, nullptr, l.parity, l.force);
             break;
         default: return cudaErrorInvalidValue;
     }
@@ -584,13 +280,13 @@ cudaError_t launch_wall_batch(const BatchArgs *ba, int parity, int force, int st
     // any non-null pointer switches force accumulation on; the kernel takes the case's slot
     double *f = force ? reinterpret_cast<double *>(1) : nullptr;
     switch (storage) {
-        case MRLBM_STORAGE_F32: wall_pair_kernel<true><<<n_blocks, kWallThreads, 0, s>>>(nullptr, ba, parity, f); break;
-        case MRLBM_STORAGE_F16: wall_kernel<__half, true><<<n_blocks, kWallThreads, 0, s>>>(nullptr, ba, parity, f); break;
+        case MRLBM_STORAGE_F32: wall_kernel<float, true><<<n_blocks, 128, 0, s>>>(nullptr, ba, parity, f); break;
+        case MRLBM_STORAGE_F16: wall_kernel<__half, true><<<n_blocks, 128, 0, s>>>(nullptr, ba, parity, f); break;
         case MRLBM_STORAGE_BF16:
-            wall_kernel<__nv_bfloat16, true><<<n_blocks, kWallThreads, 0, s>>>(nullptr, ba, parity, f);
+            wall_kernel<__nv_bfloat16, true><<<n_blocks, 128, 0, s>>>(nullptr, ba, parity, f);
             break;
         case MRLBM_STORAGE_F16_U32:
-            wall_kernel<HybridWord, true><<<n_blocks, kWallThreads, 0, s>>>(nullptr, ba, parity, f);
+            wall_kernel<HybridWord, true><<<n_blocks, 128, 0, s>>>(nullptr, ba, parity, f);
             break;
         default: return cudaErrorInvalidValue;
     }
