@@ -300,7 +300,7 @@ int step_handle(mrlbm_handle *h, int32_t nsteps) {
         if (sums) L.diag_part = h->d_diag_part;
         // The node-list kernel reads only the state before the step: it runs on its own stream beside the step
         // kernel, and starts when the last CTA of that has: a step CTA needs a whole SM and would wait until
-        // the list runs out of blocks (annulus 29.9 -> 26.1 ms per 100 steps).  The wall kernel reads the stencil
+        // the list runs out of blocks (an annulus 299 -> 261 us a step).  The wall kernel reads the stencil
         // snapshots of both.
         if (h->n_list > 0 && h->n_items > 0) L.placed = h->ev_fork;
         if (h->n_items > 0) CK(h, launch_step(L, h->storage, h->tile_y, h->special, h->stream));

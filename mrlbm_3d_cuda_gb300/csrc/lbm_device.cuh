@@ -30,8 +30,8 @@ struct Mom {
 // f_q = w_q rho [1 + 3 c.u + 4.5 (c_a c_b - delta_ab / 3) m_ab], second-order Hermite,
 // as even part +- odd part: w_q rho E_q +- 3 w_q rho (c.u), with E_q built by FMAs from
 // p0 = 1 - 1.5 tr(m).  Every FMA is written out (__fmaf_rn) and every product that must not
-// fuse goes through __fmul_rn: the owner and the rim copies of this function keep different
-// subsets of the populations, and free contraction made the two round differently.
+// fuse goes through __fmul_rn: the copies of this function (step kernel, halo warps, node list) keep different
+// subsets of the populations, and free contraction made them round differently.
 // The Hermite factors 3 (u), 1.5, 4.5 and 9 (m) are parameters so that moments stored with a
 // scale (16-bit storage) can be rebuilt without unscaling them first: pass 3 / s_u, 1.5 / s_m,
 // 4.5 / s_m and 9 / s_m with the stored u and m.

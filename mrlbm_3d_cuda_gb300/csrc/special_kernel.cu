@@ -1,13 +1,16 @@
-// Boundary and other non-bulk nodes: one thread per listed node, beside the step kernel.
+// Boundary and other non-bulk nodes, from a list, beside the step kernel: three lanes a node gather its
+// populations, then one applies the closure.
 //
 // The step kernel updates every plain bulk node in its fused pass, including plain fluid nodes
 // whose only mark is the wall-stencil bit (it also writes their snapshot), and collides the solid
 // nodes of updated blocks in place.  Every other node that carries a node word (domain faces /
 // edges / corners, BCFLUID, BCSOLID, curved-wall nodes) is this kernel's: its closure needs single
-// populations, so the thread rebuilds the 27 that the node pulls from the stored moments of its
-// neighbours, applies the closure, snapshots stencil nodes for the wall kernel, collides and stores.
+// populations, rebuilt here from the stored moments of its neighbours; then it snapshots stencil
+// nodes for the wall kernel, collides and stores.
 // It reads the state before the step only, so it runs beside the step kernel.  Nodes of blocks
 // the reference never updates (frozen) are in no list.
+// Bound by the latency of scattered loads (197 k nodes of an annulus: 191 MB from HBM in 69 us, 19% of the
+// issue slots, 16 warps an SM); all nine rows of a node are loaded at once for that reason.
 //
 // Reference (paths inside sakthi-lbm/MRLBM_3D_CUDA):
 //   evaluate_bounday_moments dispatch   MRLBM_3D/src/solver/mlbm.cu:166-184
@@ -81,8 +84,10 @@ __device__ __forceinline__ float population(const float v[10], int cx, float rho
     const float h3 = f32 ? 3.0f : __fmul_rn(3.0f, sc.is[1]), h15 = f32 ? 1.5f : __fmul_rn(1.5f, sc.is[2]);
     const float h45 = f32 ? 4.5f : __fmul_rn(4.5f, sc.is[2]), h9 = f32 ? 9.0f : __fmul_rn(9.0f, sc.is[2]);
     const float rho = f32 ? __fadd_rn(rho0, v[0]) : __fmaf_rn(v[0], sc.is[0], rho0);
-    const float ux = v[1], uy = v[2], uz = v[3], mxx = v[4], myy = v[5], mzz = v[6], mxy = v[7], mxz = v[8], myz = v[9];
-    const float sx = (float)cx;  // products with it are exact
+    // cx times ux, mxy and mxz (exact; zero for cx = 0 whatever they hold, infinities and NaN too)
+    const float sx = (float)cx;
+    const float uy = v[2], uz = v[3], mxx = v[4], myy = v[5], mzz = v[6], myz = v[9];
+    const float sux = cx ? sx * v[1] : 0.f, smxy = cx ? sx * v[7] : 0.f, smxz = cx ? sx * v[8] : 0.f;
     const float t = __fadd_rn(__fadd_rn(mxx, myy), mzz);
     const float p0 = __fmaf_rn(-h15, t, 1.0f);
     const float a0 = cx ? __fmaf_rn(h45, mxx, p0) : p0;
@@ -93,12 +98,12 @@ __device__ __forceinline__ float population(const float v[10], int cx, float rho
     const float r = __fmul_rn(rho, kW2), q = __fmul_rn(h3, r), n = __fmul_rn(h9, r);
     float f = __fmul_rn(r, e);
     if constexpr (CY != 0 || CZ != 0) {
-        float c = CY == 0 ? 0.f : (CY > 0 ? sx * mxy : -(sx * mxy));
-        if constexpr (CZ != 0) c = CY == 0 ? (CZ > 0 ? sx * mxz : -(sx * mxz)) : __fadd_rn(c, CZ > 0 ? sx * mxz : -(sx * mxz));
+        float c = CY == 0 ? 0.f : (CY > 0 ? smxy : -smxy);
+        if constexpr (CZ != 0) c = CY == 0 ? (CZ > 0 ? smxz : -smxz) : __fadd_rn(c, CZ > 0 ? smxz : -smxz);
         if constexpr (CY * CZ != 0) c = CY * CZ > 0 ? __fadd_rn(c, myz) : __fsub_rn(c, myz);
         f = __fmaf_rn(n, c, f);
     }
-    float s = sx * ux;
+    float s = sux;
     if constexpr (CY != 0) s = CY > 0 ? __fadd_rn(s, uy) : __fsub_rn(s, uy);
     if constexpr (CZ != 0) s = CZ > 0 ? __fadd_rn(s, uz) : __fsub_rn(s, uz);
     f = __fmaf_rn(q, s, f);
@@ -108,8 +113,7 @@ __device__ __forceinline__ float population(const float v[10], int cx, float rho
 
 // The populations of `mask` pulled by node (x, y, z) with this c_x, on the grid that wraps in every
 // axis, into f[direction * stride].  Three lanes share a node, one per c_x: the three neighbours
-// of a row mostly lie on one line, and the kernel is bound by the rate at which scattered loads touch
-// lines.
+// of a row mostly lie on one line.
 template <typename S>
 __device__ __forceinline__ void pull(const StepArgs &a, const S *__restrict__ src, uint32_t mask, int cx, int x, int y,
                                      int z, float *f, int stride) {
@@ -235,7 +239,8 @@ __device__ __forceinline__ int special_node(const StepArgs &a, int parity, bool 
 }
 
 // A warp takes kListNodes nodes at a time: rounds of ten nodes x three lanes gather the populations into
-// shared memory, then one lane per node applies its closure.
+// shared memory, then one lane per node applies its closure.  With 30 nodes a warp the closure fills its
+// lanes, but fewer warps hide the loads: annulus 77 us instead of 72, a cylinder's 17 k nodes 18 instead of 15.
 constexpr int kListWarps = 4, kListThreads = 32 * kListWarps, kListNodes = 10;
 
 // BATCH: each block serves the case named by its entry in BatchArgs::list_blocks.

@@ -19,9 +19,9 @@
 // A row is rebuilt three times (139 packed operations a lane instead of 80), but no population crosses
 // shared memory and no warp waits for another: only the copies of the rows' moments are shared.
 // Bound by issue and FP32 throughput with 16-bit storage (600 warp instructions per 64 nodes, 65% of the
-// issue slots), by HBM with FP32 storage (5.6 TB/s).  256^3 on GB300, before (populations exchanged
-// through shared-memory rings between CTA barriers) and now: FP32 335 -> 240 us a step, FP16 283 -> 213,
-// hybrid 298 -> 218, BF16 283 -> 215.
+// issue slots), by issue and HBM with FP32 storage (54%, 5.8 TB/s).  256^3 on GB300, before (populations exchanged
+// through shared-memory rings between CTA barriers) and now: FP32 335 -> 232 us a step, FP16 283 -> 212,
+// hybrid 298 -> 218, BF16 283 -> 214.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -55,8 +55,8 @@ struct Geo {
     static constexpr int STAGEW = (TY + 2) * ROWW + SIDEC * WPN + MARKW;  // words of one plane stage
     // Stages, and class sums parked in shared memory between planes (all nine class sums and the c_z = +1
     // class do not fit the owners' 104 registers).  Shared memory and L1 share 256 KB, and the owners'
-    // stores and remaining spills need L1: FP32 256^3 takes 240 us with 3 stages and 3 parked sums (164 KB,
-    // 92 KB of L1), 254 us with 6 parked, 285 us with 4 stages (28 KB of L1: 336 us).
+    // remaining spills need L1: FP32 256^3 takes 240 us with 3 stages and 3 parked sums (164 KB, 92 KB of L1),
+    // 254 us with 6 parked, 285 us with 4 stages (28 KB of L1: 336 us); all with stores through L1, 232 us now.
     static constexpr int D = TY == 16 ? (WPN == 10 ? 3 : (WPN == 7 ? 4 : 5)) : (WPN == 10 ? 4 : (WPN == 7 ? 5 : 6));
     static constexpr int PARK = TY != 16 ? 0 : (WPN == 10 ? 3 : 6);
     static constexpr int HALO = 9;                           // floats per row and side: c_y x c_z
@@ -902,8 +902,8 @@ int step_kernel_max_ctas_per_sm(int storage, int tile_y) {
 // the 7).  The node-list kernel runs beside the step kernel on the SMs that have no item, its rest after
 // it: 0.03 units of an SM per node in FP32 (annulus: 196 k nodes, 69 us on 152 SMs, a unit 1.56 us),
 // less with fewer words a node, and a block's latency of 5 units at least.  With that term a channel of 16
-// planes takes l = 3 instead of 2 (31.3 instead of 40.0 us a step), an annulus of 129 planes 52 instead of 43
-// (237, 247; 24: 253, 64: 252).
+// planes takes l = 3 instead of 2 (9 us of 40 less a step), an annulus of 129 planes 52 (43: 10 us of 247 more, 24: 16,
+// 64: 15, 32: 19).
 void choose_tiling(int nx, int ny, int nz, int storage, int n_sm, int &ty, int &lz, int active, int list_nodes) {
     if (ty != 4 && ty != 8 && ty != 16) ty = 16;
     if (lz > 0) {
