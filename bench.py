@@ -545,10 +545,9 @@ def run_ours(args):
                      "traffic_source": "ncu dram__bytes_read+write per node (profiles/dram_traffic.txt) x nodes"},
         "e2e": {"value": e2e_value, "unit": "MLUPS", "h2d_bytes_per_step": hv.nbytes / e2e_steps,
                 "d2h_bytes_per_step": 16 + hv.nbytes / e2e_steps},
-        # per step: the step kernel; the cylinder adds the boundary-tile step kernel, the
-        # node-list kernel and the wall kernel; stochastic rounding adds its counter tick; every
+        # per step: the step kernel; the cylinder adds the node-list kernel and the wall kernel; stochastic rounding adds its counter tick; every
         # 64th step (the divergence watchdog) adds the FP64 sum kernel
-        "gpu_launches": args.steps * ((4 if cyl else 1) + sr) + watchdog_steps(args.warmup, args.steps),
+        "gpu_launches": args.steps * ((3 if cyl else 1) + sr) + watchdog_steps(args.warmup, args.steps),
         "clocks": clk.summary(),
     }
     if not cyl and storage == "f32" and not args.no_storage_comparison:

@@ -168,13 +168,14 @@ int setup_tiling(mrlbm_handle *h, int ty, int lz) {
     for (int t = 0; t < tiles; ++t) {
         const int x0 = (t % h->tiles_x) * TILE_X, y0 = (t / h->tiles_x) * h->tile_y;
         bool special = false, all_frozen = true;
-        for (int z = 0; z < d.nz; ++z)
-            for (int y = y0; y < std::min(d.ny, y0 + h->tile_y); ++y)
-                for (int x = x0; x < std::min(d.nx, x0 + TILE_X); ++x) {
-                    const int64_t i = x + (int64_t)d.nx * (y + (int64_t)d.ny * z);
+        for (int z = 0; z < d.nz && !(special && !all_frozen); ++z)
+            for (int y = y0; y < std::min(d.ny, y0 + h->tile_y); ++y) {
+                const int64_t row = (int64_t)d.nx * (y + (int64_t)d.ny * z);
+                for (int64_t i = row + x0; i < row + std::min(d.nx, x0 + TILE_X); ++i) {
                     if (word[i]) special = true;
                     if (!g.frozen[i]) all_frozen = false;
                 }
+            }
         if (all_frozen) skip[t] = 1;
         else if (special) slot[t] = n_special++;
     }
@@ -194,7 +195,7 @@ int setup_tiling(mrlbm_handle *h, int ty, int lz) {
         for (int z = 0; z < d.nz; ++z)
             for (int y = y0; y < std::min(d.ny, y0 + h->tile_y); ++y)
                 for (int x = x0; x < std::min(d.nx, x0 + TILE_X); ++x) {
-                    const uint32_t wd = word[x + (int64_t)d.nx * (y + (int64_t)d.ny * z)];
+                    const uint32_t wd = word[(int64_t)d.nx * (y + (int64_t)d.ny * z) + x];
                     // plain fluid nodes marked only as wall-stencil nodes are updated (and
                     // snapshotted) by the step kernel itself
                     if (wd == 0u || wd == NW_STENCIL || (wd & NW_FROZEN)) continue;

@@ -901,8 +901,8 @@ int step_kernel_max_ctas_per_sm(int storage, int tile_y) {
 // A work item of l planes costs about 2 l + 7 units (of half a plane: filling and draining its pipeline is
 // the 7).  The node-list kernel runs beside the step kernel on the SMs that have no item, its rest after
 // it: 0.03 units of an SM per node in FP32 (annulus: 196 k nodes, 69 us on 152 SMs, a unit 1.56 us),
-// less with fewer words a node, and a block's latency of 5 units at least.  With that term a channel of 16
-// planes takes l = 3 instead of 2 (9 us of 40 less a step), an annulus of 129 planes 52 (43: 10 us of 247 more, 24: 16,
+// less with fewer words a node, and a block's latency of 5 units at least.  With that term a channel of 32
+// planes takes l = 3 instead of 2 (9 us of 40 less a step), an annulus of 256 planes 52 (43: 10 us of 247 more, 24: 16,
 // 64: 15, 32: 19).
 void choose_tiling(int nx, int ny, int nz, int storage, int n_sm, int &ty, int &lz, int active, int list_nodes) {
     if (ty != 4 && ty != 8 && ty != 16) ty = 16;
