@@ -88,9 +88,18 @@ __device__ __forceinline__ bool mbar_try(uint32_t a, uint32_t parity) {
         : "memory");
     return done != 0;
 }
+// The wait of a whole warp: its lanes poll each by itself and leave together, all with the same answer, so
+// that what follows (shuffles, the release of a stage by lane 0) finds the warp whole.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
     const uint32_t a = smem_addr(bar);
-    if (mbar_try(a, parity)) return true;
+    bool done = mbar_try(a, parity);
+#pragma unroll 1
+    for (int i = 0; !done && i < kWaitLimit; ++i) done = mbar_try(a, parity);
+    return __all_sync(0xffffffffu, done);
+}
+// The wait of one lane.
+__device__ __forceinline__ bool mbar_wait_lane(uint64_t *bar, uint32_t parity) {
+    const uint32_t a = smem_addr(bar);
 #pragma unroll 1
     for (int i = 0; i < kWaitLimit; ++i)
         if (mbar_try(a, parity)) return true;

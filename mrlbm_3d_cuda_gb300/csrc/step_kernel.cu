@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
                 // one answer for all halo warps (two slots: the next one is written a barrier after the
                 // last read of this one)
                 if (leader) {
-                    const bool answered = mbar_wait(&s_taken, n & 1);
+                    const bool answered = mbar_wait_lane(&s_taken, n & 1);
                     s_next[n & 1] = answered ? takeover_result(s_slot + (n & 1)) : -1;
                     ok = ok && answered;
                 }
@@ -508,7 +508,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
             // that was never issued just runs into the wait's limit)
             atomicOr(BATCH ? ba->cases[0]->error : single.error, kErrorWait);
             for (int s = 0; s < G::D; ++s)
-                if (!mbar_wait(landed + s, 0)) mbar_wait(landed + s, 1);
+                if (!mbar_wait_lane(landed + s, 0)) mbar_wait_lane(landed + s, 1);
         }
     } else {
         if constexpr (G::SPLIT) asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
@@ -686,6 +686,8 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
                     }
                     up = finish(2);
                 } else {
+                    // rows past the tile's last one read nothing but the stage's head, all lanes before the release
+                    __syncwarp();
                     if (lane == 0) mbar_arrive(empty + stage);
                 }
                 next_stage();

@@ -1,0 +1,38 @@
+"""The step kernel's pipeline where its warps do unequal work: tiles whose last rows do not exist (their
+warps only hand the stages on, and run as far ahead as the ring allows), over many planes and items."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def fields(monkeypatch, desc, init, steps, ty):
+    from mrlbm_3d_cuda_gb300 import Simulation
+    monkeypatch.setenv("MRLBM_TILE_Y", str(ty))
+    with Simulation(desc, init=False) as sim:
+        sim.init(*init)
+        sim.step(steps)
+        sim.sync()
+        return sim.moments()
+
+
+@pytest.mark.parametrize("storage", [0, 1, 3])
+@pytest.mark.parametrize("kind", ["periodic", "channel"])
+def test_rows_past_the_tile(cuda_device, kind, storage, monkeypatch):
+    """8 of 16 rows missing in every other tile of a 24-row box, and in a third of a 40-row channel's
+    (whose CTAs take over each other's items), against tiles of 8 rows, which are all whole: every
+    store is of the same values, so the fields have the same bits."""
+    from mrlbm_3d_cuda_gb300 import cases
+    from mrlbm_3d_cuda_gb300 import native as N
+    if kind == "periodic":
+        desc = cases.periodic_box(512, 24, 256, u0=0.05, re=100.0, length=8.0, storage=storage)
+        init = N.INIT_NOISY_UNIFORM, (0.03, 0.01, -0.02, 0.3, 13)
+    else:
+        desc = cases.cylinder_channel(320, 40, 128, 10, 63.6, 19.7, 0.05, 60.0, storage=storage)
+        init = N.INIT_NOISY_UNIFORM, (0.05, 0.0, 0.0, 0.01, 5)
+    want = fields(monkeypatch, desc, init, 12, 8)
+    assert np.isfinite(want).all()
+    got = fields(monkeypatch, desc, init, 12, 16)
+    assert np.array_equal(got, want)
