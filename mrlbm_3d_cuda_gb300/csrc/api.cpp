@@ -84,6 +84,7 @@ void free_all(mrlbm_handle *h) {
     if (h->own_stream) cudaStreamDestroy(h->own_stream);
     if (h->list_stream) cudaStreamDestroy(h->list_stream);
     if (h->ev_fork) cudaEventDestroy(h->ev_fork);
+    if (h->ev_placed) cudaEventDestroy(h->ev_placed);
     if (h->ev_list) cudaEventDestroy(h->ev_list);
 }
 
@@ -300,14 +301,18 @@ int step_handle(mrlbm_handle *h, int32_t nsteps) {
         const bool sums = ds || ws;
         if (sums) L.diag_part = h->d_diag_part;
         // The node-list kernel reads only the state before the step: it runs on its own stream beside the step
-        // kernel, and starts when the last CTA of that has: a step CTA needs a whole SM and would wait until
-        // the list runs out of blocks (an annulus 299 -> 261 us a step).  The wall kernel reads the stencil
+        // kernel, after the steps before this one (ev_fork).  ev_placed, which comes when the step kernel's
+        // last CTA has started, only makes it start late: a step CTA needs a whole SM and would wait until the
+        // list runs out of blocks (an annulus 299 -> 261 us a step).  The wall kernel reads the stencil
         // snapshots of both.
-        if (h->n_list > 0 && h->n_items > 0) L.placed = h->ev_fork;
+        if (h->n_list > 0) {
+            CK(h, cudaEventRecord(h->ev_fork, h->stream));
+            CK(h, cudaStreamWaitEvent(h->list_stream, h->ev_fork, 0));
+            if (h->n_items > 0) L.placed = h->ev_placed;
+        }
         if (h->n_items > 0) CK(h, launch_step(L, h->storage, h->tile_y, h->special, h->stream));
         if (h->n_list > 0) {
-            if (!L.placed) CK(h, cudaEventRecord(h->ev_fork, h->stream));
-            CK(h, cudaStreamWaitEvent(h->list_stream, h->ev_fork, 0));
+            if (L.placed) CK(h, cudaStreamWaitEvent(h->list_stream, h->ev_placed, 0));
             CK(h, launch_special_list(L, h->storage, h->n_list_blocks,
                                       sums ? h->d_diag_part + 2 * (size_t)h->n_ctas * h->tile_y : nullptr,
                                       h->list_stream));
@@ -558,6 +563,7 @@ int mrlbm_create(const mrlbm_case_desc *din, mrlbm_handle **out) {
     h->stream = h->own_stream;
     CK(h.get(), cudaStreamCreateWithFlags(&h->list_stream, cudaStreamNonBlocking));
     CK(h.get(), cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
+    CK(h.get(), cudaEventCreateWithFlags(&h->ev_placed, cudaEventDisableTiming));
     CK(h.get(), cudaEventCreateWithFlags(&h->ev_list, cudaEventDisableTiming));
 
     // geometry on the host

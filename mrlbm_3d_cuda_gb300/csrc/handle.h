@@ -32,9 +32,10 @@ struct mrlbm_handle {
     bool host_only = false;
     int dev = 0, n_sm = 0;
     cudaStream_t own_stream = nullptr, stream = nullptr;
-    // the node-list launch runs beside the step kernel: its stream and fork / join events
+    // the node-list launch runs beside the step kernel: its stream, fork / join events, and the event of the
+    // step kernel's last CTA having started
     cudaStream_t list_stream = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_list = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_placed = nullptr, ev_list = nullptr;
     int storage = 0, vbytes = 4;
     StorageScale sc{};
     int64_t n = 0, fs = 0;
