@@ -136,6 +136,13 @@ void default_tiling(int &ty, int &lz) {
 
 int setup_tiling(mrlbm_handle *h, int ty, int lz);
 
+// Test hook for the step kernel's bounded waits: MRLBM_FAULT_WAIT_POLLS=k (0: no poll at all) takes the place
+// of the poll limit, so that a wait runs out and the kernel reports it.
+int wait_limit() {
+    const char *v = std::getenv("MRLBM_FAULT_WAIT_POLLS");
+    return v ? std::max(0, std::atoi(v)) : kWaitLimit;
+}
+
 // Bytes of one storage element: FP32 and the hybrid mode's words 4, FP16 / BF16 halves 2.
 int storage_element_bytes(int storage) {
     return storage == MRLBM_STORAGE_F16 || storage == MRLBM_STORAGE_BF16 ? 2 : 4;
@@ -678,6 +685,7 @@ int mrlbm_create(const mrlbm_case_desc *din, mrlbm_handle **out) {
     a.tag_in = h->d_tag;
     a.tag_out = h->d_tag ? h->d_tag + 256 : nullptr;
     a.error = h->d_error;
+    a.wait_limit = wait_limit();
     if (d.stochastic_rounding && d.storage != MRLBM_STORAGE_F32) {
         CK(H, cudaMalloc((void **)&h->d_sr_step, sizeof(uint32_t)));
         CK(H, cudaMemset(h->d_sr_step, 0, sizeof(uint32_t)));

@@ -66,6 +66,9 @@ struct WallArgs {
     float u_wall[3] = {0.f, 0.f, 0.f};
 };
 
+// Polls after which a wait of the step kernel gives up (see packed.cuh).
+constexpr int kWaitLimit = 1 << 22;
+
 // One copy lives in device memory per handle; kernels receive a pointer to it plus the
 // per-step scalars (ping-pong parity, sampling buffers).
 struct StepArgs {
@@ -92,6 +95,7 @@ struct StepArgs {
     // stochastic rounding of 16-bit stores: the step counter that seeds the random bits
     // (null: round to nearest)
     const uint32_t *sr_step = nullptr;
+    int wait_limit = kWaitLimit;          // of the owner warps' waits (the halo warps': at least 1)
 };
 
 // Several independent cases advanced together: one step-kernel launch over the work items of

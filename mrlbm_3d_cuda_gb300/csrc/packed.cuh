@@ -4,6 +4,8 @@
 
 #include <cstdint>
 
+#include "kernels.h"
+
 namespace mrlbm {
 
 // Two floats in one 64-bit register pair.  Each lane of a packed operation rounds like the scalar
@@ -73,10 +75,9 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
     asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes)
                  : "memory");
 }
-// Wait for the phase of the given parity; gives up after kWaitLimit polls (each at least tens of
-// cycles: far beyond any copy or plane of work) and returns false.  (A suspend-time hint on the polls
-// made them sleep: up to 2.5 times slower steps.)
-constexpr int kWaitLimit = 1 << 22;
+// Waits for the phase of the given parity.  They give up after `limit` polls and return false: kWaitLimit polls
+// that find nothing take 16 s (3.8 us each), far beyond any copy or plane of work.  (A suspend-time hint
+// on the polls made them sleep: up to 2.5 times slower steps.)
 __device__ __forceinline__ bool mbar_try(uint32_t a, uint32_t parity) {
     uint32_t done;
     asm volatile(
@@ -90,14 +91,14 @@ __device__ __forceinline__ bool mbar_try(uint32_t a, uint32_t parity) {
 }
 // The wait of a whole warp: its lanes poll each by itself and leave together, all with the same answer, so
 // that what follows (shuffles, the release of a stage by lane 0) finds the warp whole.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int limit) {
     const uint32_t a = smem_addr(bar);
-    bool done = mbar_try(a, parity);
+    bool done = false;
 #pragma unroll 1
-    for (int i = 0; !done && i < kWaitLimit; ++i) done = mbar_try(a, parity);
+    for (int i = 0; !done && i < limit; ++i) done = mbar_try(a, parity);
     return __all_sync(0xffffffffu, done);
 }
-// The wait of one lane.
+// The wait of one lane for what is on its way into shared memory, whatever limit the other waits have.
 __device__ __forceinline__ bool mbar_wait_lane(uint64_t *bar, uint32_t parity) {
     const uint32_t a = smem_addr(bar);
 #pragma unroll 1

@@ -323,7 +323,8 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
     extern __shared__ __align__(128) unsigned char smem[];
     uint32_t *const stages = reinterpret_cast<uint32_t *>(smem);
     float *const halos = reinterpret_cast<float *>(smem + G::D * G::STAGEW * 4);
-    // {case, work item, its number} of the item that starts with the stage's plane
+    // {case, work item, its number} of the item that starts with the stage's plane; 1 + the parity of the
+    // stage's last use (0: none yet)
     int4 *const heads = reinterpret_cast<int4 *>(smem + G::D * (G::STAGEW * 4 + 2 * TY * G::HALO * 4));
     uint64_t *const full = reinterpret_cast<uint64_t *>(heads + G::D);
     uint64_t *const empty = full + G::D;
@@ -332,6 +333,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
     __shared__ __align__(16) uint4 s_slot[2];  // answers to takeover requests, by item parity
     __shared__ uint64_t s_taken;
     __shared__ int s_next[2];
+    __shared__ int s_failed;  // a halo warp's wait ran out
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -339,8 +341,10 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
             mbar_init(full + s, 1);
             mbar_init(empty + s, TY);
             mbar_init(landed + s, 1);
+            heads[s] = make_int4(0, 0, 0, 0);
         }
         mbar_init(&s_taken, 1);
+        s_failed = 0;
         mbar_init_fence();
     }
     __syncthreads();
@@ -353,6 +357,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
         }
     };
     const int n_items = BATCH ? ba->n_items : single.n_items;
+    const int limit = BATCH ? ba->cases[0]->wait_limit : single.wait_limit;
 
     if (warp >= TY) {
         if constexpr (G::SPLIT) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
@@ -361,6 +366,11 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
         const int hw = warp - TY;
         int q = 0;        // planes so far, over all items: plane q is halo warp q % NH's
         int n = 0;        // items so far
+        auto take_turn = [&]() {
+            if (G::NH > 1 && q > 0) token_wait(3 + hw);
+            if (ok) ok = *(const volatile int *)&s_failed == 0 && mbar_wait(empty + stage, phase ^ 1u, max(limit, 1));
+            if (!ok && lane == 0) *(volatile int *)&s_failed = 1;
+        };
         // Work items.  SPECIAL: one CTA per item is launched, and a CTA that finishes its item takes over
         // one that has not started (tiles with boundary nodes and the cases of a batch cost unevenly).
         // Otherwise the CTAs stride through the items.
@@ -420,15 +430,16 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
                 // The halo warps wait for a free stage in turn, each asleep at a hardware barrier until the one
                 // before it has passed (polling costs issue slots).  Plane q waits for the release of plane
                 // q - D; the turn before has seen that of q - 1 - D, so the release two uses back on the stage
-                // is past, which the one parity bit of the wait could not tell from the last one.
-                if (G::NH > 1 && q > 0) token_wait(3 + hw);
-                if (ok) ok = mbar_wait(empty + stage, phase ^ 1u);
+                // is past, which the one parity bit of the wait could not tell from the last one.  For that, no
+                // turn succeeds after one that failed.
+                take_turn();
                 if (G::NH > 1) token_pass(3 + (hw + 1) % G::NH);
                 if (!ok) continue;
                 uint32_t *const sp = stages + stage * G::STAGEW;
                 uint32_t *const cp = sp + (TY + 2) * G::ROWW;  // [word][column]
                 if (lane == 0) {
-                    if (k == 0) heads[stage] = make_int4(head.x, head.y, it, 0);
+                    if (k == 0) heads[stage] = make_int4(head.x, head.y, it, (int)phase + 1);
+                    else heads[stage].w = (int)phase + 1;
                     mbar_expect_tx(landed + stage, row_bytes * (h + 2) + (marked(k) ? TILE_X * (uint32_t)h : 0u));
                     mbar_arrive(landed + stage);
                 }
@@ -485,7 +496,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
                 if (leader) {
                     const bool answered = mbar_wait_lane(&s_taken, n & 1);
                     s_next[n & 1] = answered ? takeover_result(s_slot + (n & 1)) : -1;
-                    ok = ok && answered;
+                    if (!answered) *(volatile int *)&s_failed = 1;
                 }
                 asm volatile("bar.sync 2, %0;" ::"r"(32 * G::NH) : "memory");
                 it = s_next[n & 1];
@@ -495,21 +506,21 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
             }
         }
         if (q % G::NH == hw) {
-            if (G::NH > 1 && q > 0) token_wait(3 + hw);
-            if (ok) ok = mbar_wait(empty + stage, phase ^ 1u);
+            take_turn();
             if (ok && lane == 0) {
-                heads[stage] = make_int4(0, -1, 0, 0);  // end mark
+                heads[stage] = make_int4(0, -1, 0, (int)phase + 1);  // end mark
                 mbar_arrive(landed + stage);
                 mbar_arrive(full + stage);
             }
         }
-        if (!ok && lane == 0) {
-            // a wait ran out: report, and leave only when the copies in flight have landed (a stage
-            // that was never issued just runs into the wait's limit)
-            atomicOr(BATCH ? ba->cases[0]->error : single.error, kErrorWait);
+        if (!ok && lane == 0) atomicOr(BATCH ? ba->cases[0]->error : single.error, kErrorWait);
+        // The CTA stays until its copies have landed, also when a wait ran out and its owners are gone: the
+        // shared memory that they fill would be the next CTA's.  No halo warp issues another one past the
+        // barrier; a stage's last use is the one under way or the last that ended, so its parity tells.
+        asm volatile("bar.sync 2, %0;" ::"r"(32 * G::NH) : "memory");
+        if (threadIdx.x == 32 * TY)
             for (int s = 0; s < G::D; ++s)
-                if (!mbar_wait_lane(landed + s, 0)) mbar_wait_lane(landed + s, 1);
-        }
+                if (heads[s].w) mbar_wait_lane(landed + s, (uint32_t)(heads[s].w - 1));
     } else {
         if constexpr (G::SPLIT) asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
         // ---- owner warps -----------------------------------------------------------------------
@@ -519,7 +530,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
             // landed before full, here and in every plane: rows past the tile's last one skip the waits on
             // full, and only the landing of a stage (its refill follows the release of its last use) makes
             // the one parity bit of that wait unambiguous
-            ok = mbar_wait(landed + stage, phase) && mbar_wait(full + stage, phase);
+            ok = mbar_wait(landed + stage, phase, limit) && mbar_wait(full + stage, phase, limit);
             if (!ok) break;
             const int4 head = heads[stage];
             if (head.y < 0) break;
@@ -569,7 +580,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
                 }
             };
             auto plane = [&](const int k) {
-                if (k > 0 && ok) ok = mbar_wait(landed + stage, phase);
+                if (k > 0 && ok) ok = mbar_wait(landed + stage, phase, limit);
                 if (!ok) return;
                 Pair o;
                 V2 rho4;  // 4 rho, as the sums in `o`
@@ -584,7 +595,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
                         V2 f[27];
                         rebuild_scaled<S>(load_pair<S>(sp + (1 - cy) * G::ROWW), K, f);
                         // the side columns' populations are evaluated meanwhile
-                        if (cy == -1 && k > 0) ok = mbar_wait(full + stage, phase);
+                        if (cy == -1 && k > 0) ok = mbar_wait(full + stage, phase, limit);
                         const float e[3] = {hv[3 * (cy + 1)], hv[3 * (cy + 1) + 1], hv[3 * (cy + 1) + 2]};
 #pragma unroll
                         for (int c = 0; c < 3; ++c) {

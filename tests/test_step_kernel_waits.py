@@ -1,0 +1,57 @@
+"""The step kernel's bounded waits: one that runs out ends in a status, with the kernel's copies landed and the
+context usable.  The limit comes from the host (MRLBM_FAULT_WAIT_POLLS polls, read when a handle is
+created): with 0 the warps that own the tile's rows give up at their first wait, while the copies of the
+first planes are on their way; with a few, some waits run out and some do not.  A wait on copies that nobody
+has issued would take the full limit, 16 s: each run ends long before that."""
+from __future__ import annotations
+
+import time
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def descs(kind):
+    from mrlbm_3d_cuda_gb300 import cases
+    if kind == "periodic":  # more items than SMs, ragged in x and y, even and odd uses of every stage
+        return cases.periodic_box(200, 136, 92, u0=0.05, re=100.0, length=8.0)
+    return cases.cylinder_channel(128, 40, 64, 10, 32.6, 19.7, 0.05, 60.0)
+
+
+def run(kind, steps, storage=0):
+    from mrlbm_3d_cuda_gb300 import Simulation
+    from mrlbm_3d_cuda_gb300 import native as N
+    desc = descs(kind)
+    desc.storage = storage
+    with Simulation(desc, init=False) as sim:
+        sim.init(N.INIT_NOISY_UNIFORM, (0.05, 0.0, 0.0, 0.01, 5))
+        t = time.perf_counter()
+        sim.step(steps)
+        try:
+            sim.sync()
+            code = N.OK
+        except N.MrlbmError as e:
+            code = e.code
+        assert time.perf_counter() - t < 8.0
+        return code, sim.moments() if code == N.OK else None
+
+
+@pytest.mark.parametrize("storage", [0, 1])
+@pytest.mark.parametrize("tile_y", [4, 8, 16])
+@pytest.mark.parametrize("kind", ["periodic", "channel"])
+def test_wait_that_runs_out_is_a_status(cuda_device, kind, tile_y, storage, monkeypatch):
+    from mrlbm_3d_cuda_gb300 import native as N
+    monkeypatch.setenv("MRLBM_TILE_Y", str(tile_y))
+    code, want = run(kind, 4, storage)
+    assert code == N.OK
+    for polls in (0, 1, 2, 3):
+        monkeypatch.setenv("MRLBM_FAULT_WAIT_POLLS", str(polls))
+        code, got = run(kind, 4, storage)
+        assert code == (N.ERR_TIMEOUT if polls == 0 else code) and code in (N.OK, N.ERR_TIMEOUT)
+        if code == N.OK:
+            assert np.array_equal(got, want)
+        monkeypatch.delenv("MRLBM_FAULT_WAIT_POLLS")
+        code, got = run(kind, 4, storage)  # right behind it, on the same SMs
+        assert code == N.OK and np.array_equal(got, want)
