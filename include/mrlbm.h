@@ -242,10 +242,10 @@ int mrlbm_write_geometry(const mrlbm_handle *h, const char *dir);
 /* ---- allocation-free step (no counterpart in the reference) ------------------------------------
  * One time step of a fully periodic box (no walls, no inlet / outlet) from m_in to m_out,
  * for callers that cannot allocate device memory: it calls no cudaMalloc / cudaFree and no
- * allocating library routine.  The step kernel's scratch (diagnostics partials and sums, error
- * word) is one fixed 64 KiB array in the library's device image; grids are limited to 11776 xy
- * tiles of 32 x 16 nodes (ceil(nx/32) * ceil(ny/16)), e.g. 2048 x 2944 nodes per z plane, and
- * larger ones rejected with MRLBM_ERR_INVALID_ARG.  Every call with diag shares that array
+ * allocating library routine.  The step kernel's scratch (diagnostics partials and sums) is one
+ * fixed 64 KiB array in the library's device image; grids are limited to 11776 xy tiles of 32 x 16
+ * nodes (ceil(nx/32) * ceil(ny/16)), e.g. 2048 x 2944 nodes per z plane, and larger ones rejected
+ * with MRLBM_ERR_INVALID_ARG.  Every call with diag shares that array
  * (each rewrites what it reads): such calls race on it when they overlap on the GPU (two
  * streams or two host threads).
  * m_in / m_out: device pointers, 16-byte aligned, not overlapping, FP32 moments in the
@@ -254,7 +254,10 @@ int mrlbm_write_geometry(const mrlbm_handle *h, const char *dir);
  * MRLBM_FIELD_* with field 0 holding rho - rho0; nz*ny*ceil(nx/32)*320 floats each.
  * Grid: positive multiples of 8 x 8 x 4.  diag: NULL, or {mass, kinetic energy} as
  * mrlbm_get_diagnostics, in which case the call waits for the step.  Otherwise it is
- * asynchronous on `cuda_stream` (a cudaStream_t; NULL = default stream). */
+ * asynchronous on `cuda_stream` (a cudaStream_t; NULL = default stream).
+ * MRLBM_ERR_TIMEOUT: a bounded wait inside the kernel ran out and m_out is incomplete.  A call with
+ * diag returns it for itself; after a call without, the next call on the device made once the kernel has
+ * ended returns it instead of stepping (the message says so), and the one after that steps. */
 int mrlbm_step_periodic_noalloc(const float *m_in, float *m_out, int32_t nx, int32_t ny, int32_t nz, float omega,
                                 float rho0, double *diag, void *cuda_stream);
 

@@ -1033,6 +1033,7 @@ int mrlbm_step_periodic_noalloc(const float *m_in, float *m_out, int32_t nx, int
     p.rho0 = rho0;
     p.diag_host = diag;
     p.stream = (cudaStream_t)cuda_stream;
+    p.wait_limit = wait_limit();
     std::string err;
     const int rc = noalloc_periodic_step(p, err);
     if (rc != MRLBM_OK) return fail(nullptr, rc, err);

@@ -87,7 +87,7 @@ struct StepArgs {
     StorageScale sc;
     WallArgs wall[2];
     const uint32_t *tag_in = nullptr, *tag_out = nullptr;  // [256] BCFLUID masks
-    int *error = nullptr;     // sticky device error flag
+    int *error = nullptr;     // sticky error flag (device memory; managed memory in the allocation-free step)
     // nodes handled by the node-list kernel (those the step kernel does not update itself)
     const uint64_t *list_xyz = nullptr;   // x | y << 21 | z << 42
     const uint32_t *list_word = nullptr;  // node word of each entry
@@ -192,11 +192,9 @@ cudaError_t launch_surface_pressure(const StepArgs *ga, int buf, int storage, in
 // Allocation-free periodic step (mrlbm_step_periodic_noalloc).  What a step needs on the device
 // besides the caller's two moment buffers lives in one fixed array in the library's image:
 //   [0, 16)              mass / energy sums (2 doubles)
-//   [64, 68)             error word
 //   [1024, 65536)        diagnostics partials, 2 doubles per owner warp
 constexpr int kNoAllocScratchBytes = 64 * 1024;
 constexpr int kNoAllocDiagOffset = 0;
-constexpr int kNoAllocErrorOffset = 64;
 constexpr int kNoAllocPartOffset = 1024;
 constexpr int kNoAllocMaxParts = (kNoAllocScratchBytes - kNoAllocPartOffset) / (2 * (int)sizeof(double));
 constexpr int kNoAllocMaxTiles = 11776;  // xy tiles of 32 x 16 nodes
@@ -208,6 +206,7 @@ struct NoAllocStep {
     float omega = 0.f, rho0 = 1.f;
     double *diag_host = nullptr;  // optional: {mass, kinetic energy} as mrlbm_get_diagnostics
     cudaStream_t stream = nullptr;
+    int wait_limit = kWaitLimit;  // as StepArgs::wait_limit
 };
 // Returns an MRLBM_* status; on failure `err` holds the message.
 int noalloc_periodic_step(const NoAllocStep &p, std::string &err);

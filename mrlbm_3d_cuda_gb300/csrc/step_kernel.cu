@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
                 mbar_arrive(full + stage);
             }
         }
-        if (!ok && lane == 0) atomicOr(BATCH ? ba->cases[0]->error : single.error, kErrorWait);
+        if (!ok && lane == 0) atomicOr_system(BATCH ? ba->cases[0]->error : single.error, kErrorWait);
         // The CTA stays until its copies have landed, also when a wait ran out and its owners are gone: the
         // shared memory that they fill would be the next CTA's.  No halo warp issues another one past the
         // barrier; a stage's last use is the one under way or the last that ended, so its parity tells.
@@ -767,7 +767,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
                 ++items;
             }
         }
-        if (!ok && lane == 0) atomicOr(BATCH ? ba->cases[0]->error : single.error, kErrorWait);
+        if (!ok && lane == 0) atomicOr_system(BATCH ? ba->cases[0]->error : single.error, kErrorWait);
     }
 }
 
@@ -963,26 +963,32 @@ int choose_batch_lz(const std::vector<int> &tiles, const std::vector<int> &nz, i
 
 // ---- allocation-free periodic step --------------------------------------------------------
 // For callers that cannot allocate device memory: what a step needs besides the caller's buffers
-// (diagnostics partials and sums, error word) lives in this fixed array of the library's device
-// image, laid out as in kernels.h; the argument block travels with the launch.  Every call that
-// asks for diagnostics shares the array: such calls race on it when they overlap on the GPU (two
-// streams, or two host threads).
+// (diagnostics partials and sums) lives in this fixed array of the library's device image, laid out
+// as in kernels.h; the argument block travels with the launch.  Every call that asks for
+// diagnostics shares the array: such calls race on it when they overlap on the GPU (two streams, or
+// two host threads).
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
+
+constexpr int kNoAllocMaxDevices = 64;
+// Error word of each device's calls, in managed memory: set by a kernel whose wait ran out, and read by the
+// host without a copy or a synchronisation, so that a call without diagnostics (which returns before its
+// kernel has run) is reported by the next one.
+static __managed__ int g_noalloc_error[kNoAllocMaxDevices];
 
 namespace {
 
-constexpr int kNoAllocMaxDevices = 64;
 std::mutex g_noalloc_mu;
-// per device, set up on its first call: the scratch array's device address and the SM count
+// per device, set up on its first call: the scratch array's device address, the error word and the SM count
 struct NoAllocDevice {
     void *scratch = nullptr;
+    int *error = nullptr;
     int n_sm = 0;
 };
 NoAllocDevice g_noalloc_dev[kNoAllocMaxDevices];
 
-// Set-up of device `dev` (the current device), once: the scratch array's device address (in
-// host code the array's name is only a host-side stand-in) and its SM count.  Host-side queries
-// only; nothing is allocated.
+// Set-up of device `dev` (the current device), once: the arrays' addresses (in host code the scratch
+// array's name is only a host-side stand-in) and the SM count.  Host-side queries only; nothing is
+// allocated.
 cudaError_t noalloc_device(int dev, NoAllocDevice &out) {
     std::lock_guard<std::mutex> lock(g_noalloc_mu);
     NoAllocDevice &d = g_noalloc_dev[dev];
@@ -990,10 +996,13 @@ cudaError_t noalloc_device(int dev, NoAllocDevice &out) {
         void *p = nullptr;
         cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
         if (e != cudaSuccess) return e;
+        void *w = nullptr;
+        if ((e = cudaGetSymbolAddress(&w, g_noalloc_error)) != cudaSuccess) return e;
         int n_sm = 0;
         if ((e = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
         d.n_sm = n_sm;
-                d.scratch = p;
+        d.error = (int *)w + dev;
+        d.scratch = p;
     }
     out = d;
     return cudaSuccess;
@@ -1002,6 +1011,11 @@ cudaError_t noalloc_device(int dev, NoAllocDevice &out) {
 int noalloc_cuda_fail(cudaError_t e, const char *what, std::string &err) {
     err = std::string("mrlbm_step_periodic_noalloc: ") + what + ": " + cudaGetErrorString(e);
     return e == cudaErrorNoKernelImageForDevice ? MRLBM_ERR_UNSUPPORTED : MRLBM_ERR_CUDA;
+}
+
+// Whether a kernel has set the error word; clears it.
+bool noalloc_take_error(const NoAllocDevice &d) {
+    return __atomic_load_n(d.error, __ATOMIC_ACQUIRE) != 0 && __atomic_exchange_n(d.error, 0, __ATOMIC_ACQ_REL) != 0;
 }
 
 }  // namespace
@@ -1061,6 +1075,11 @@ int noalloc_periodic_step(const NoAllocStep &p, std::string &err) {
         }
     }
     if ((e = noalloc_device(dev, nd)) != cudaSuccess) return noalloc_cuda_fail(e, "device set-up", err);
+    if (noalloc_take_error(nd)) {
+        err = std::string(fn) + "a wait inside the step kernel of an earlier call ran out: that call's output is not complete "
+                                "(this call has launched nothing)";
+        return MRLBM_ERR_TIMEOUT;
+    }
     unsigned char *scratch = (unsigned char *)nd.scratch;
 
     int ty = 0, lz = 0;
@@ -1085,7 +1104,8 @@ int noalloc_periodic_step(const NoAllocStep &p, std::string &err) {
     sa.omega = p.omega;
     sa.rho0 = p.rho0;
     for (int k = 0; k < 3; ++k) sa.sc.s[k] = sa.sc.is[k] = 1.f;
-    sa.error = (int *)(scratch + kNoAllocErrorOffset);
+    sa.error = nd.error;
+    sa.wait_limit = p.wait_limit;
     double *part = (double *)(scratch + kNoAllocPartOffset);
     double *sums = (double *)(scratch + kNoAllocDiagOffset);
     StepLaunch L;
@@ -1101,6 +1121,10 @@ int noalloc_periodic_step(const NoAllocStep &p, std::string &err) {
         if ((e = cudaMemcpyAsync(v, sums, sizeof(v), cudaMemcpyDeviceToHost, p.stream)) != cudaSuccess ||
             (e = cudaStreamSynchronize(p.stream)) != cudaSuccess)
             return noalloc_cuda_fail(e, "diagnostics read-back", err);
+        if (noalloc_take_error(nd)) {
+            err = std::string(fn) + "a wait inside the step kernel ran out";
+            return MRLBM_ERR_TIMEOUT;
+        }
         p.diag_host[0] = (double)p.nx * p.ny * p.nz * p.rho0 + v[0];
         p.diag_host[1] = v[1];
         if (!std::isfinite(v[0]) || !std::isfinite(v[1])) {

@@ -55,3 +55,35 @@ def test_wait_that_runs_out_is_a_status(cuda_device, kind, tile_y, storage, monk
         monkeypatch.delenv("MRLBM_FAULT_WAIT_POLLS")
         code, got = run(kind, 4, storage)  # right behind it, on the same SMs
         assert code == N.OK and np.array_equal(got, want)
+
+
+def test_allocation_free_step_reports_a_wait_that_ran_out(cuda_device, monkeypatch):
+    """mrlbm_step_periodic_noalloc: with diagnostics the call itself returns the status; without, it has returned
+    before its kernel ran, and the next call does (and launches nothing).  Either is reported once."""
+    import ctypes as C
+
+    import torch
+    from mrlbm_3d_cuda_gb300 import native as N
+    lib, shape = N.lib(), (72, 40, 16)
+    g = torch.Generator().manual_seed(7)
+    src = (1e-3 * torch.randn(96 * 40 * 16 * 10, generator=g)).cuda()
+    stream = torch.cuda.current_stream().cuda_stream
+
+    def call(dst, diag=None):
+        return lib.mrlbm_step_periodic_noalloc(C.c_void_p(src.data_ptr()), C.c_void_p(dst.data_ptr()), *shape,
+                                               C.c_float(1.2), C.c_float(1.0), diag, C.c_void_p(stream))
+
+    want, want_sums = torch.zeros_like(src), (C.c_double * 2)()
+    assert call(want, want_sums) == N.OK
+    for diag in ((C.c_double * 2)(), None):
+        monkeypatch.setenv("MRLBM_FAULT_WAIT_POLLS", "0")
+        assert call(torch.zeros_like(src), diag) == (N.ERR_TIMEOUT if diag is not None else N.OK)
+        monkeypatch.delenv("MRLBM_FAULT_WAIT_POLLS")
+        torch.cuda.synchronize()
+        got, sums = torch.zeros_like(src), (C.c_double * 2)()
+        if diag is None:
+            assert call(got) == N.ERR_TIMEOUT and b"earlier call" in lib.mrlbm_last_error(None)
+            torch.cuda.synchronize()
+            assert not got.any()
+        assert call(got, sums) == N.OK
+        assert torch.equal(got, want) and list(sums) == list(want_sums)
