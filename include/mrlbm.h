@@ -42,7 +42,8 @@ extern "C" {
 #define MRLBM_ERR_INVALID_ARG (-1) /* bad descriptor / argument (also the tau / Mach guards) */
 #define MRLBM_ERR_CUDA (-2)        /* a CUDA runtime call failed                              */
 #define MRLBM_ERR_DIVERGED (-3)    /* NaN / Inf seen by the mass watchdog                     */
-#define MRLBM_ERR_TIMEOUT (-4)     /* a bounded device wait gave up                          */
+#define MRLBM_ERR_TIMEOUT (-4)     /* a bounded device wait gave up: the field is incomplete; every
+                                      read-back returns it until a whole new field is set     */
 #define MRLBM_ERR_IO (-5)          /* file could not be read / written                        */
 #define MRLBM_ERR_UNSUPPORTED (-6) /* option not built (e.g. device has no sm_103a)           */
 #define MRLBM_ERR_STATE (-7)       /* call out of order (e.g. step before init)               */

@@ -105,16 +105,26 @@ int ensure_stage(mrlbm_handle *h, size_t bytes) {
     return MRLBM_OK;
 }
 
-// A new state (init, uploaded moments, loaded checkpoint) starts with a clear divergence flag.
-// The stream is drained first so that no queued watchdog copy lands after the clear.
-int clear_divergence(mrlbm_handle *h) {
+// A new state (init, uploaded moments, loaded checkpoint) starts with a clear divergence flag, and with a
+// clear time-out flag where it replaces the whole field.  The stream is drained first so that no queued
+// watchdog copy lands after the clear.
+int clear_status(mrlbm_handle *h, bool whole) {
     CK(h, cudaStreamSynchronize(h->stream));
     int e = 0;
     CK(h, cudaMemcpy(&e, h->d_error, sizeof(int), cudaMemcpyDeviceToHost));
-    e &= ~kErrorDiverged;
+    e &= whole ? ~(kErrorDiverged | kErrorWait) : ~kErrorDiverged;
     CK(h, cudaMemcpy(h->d_error, &e, sizeof(int), cudaMemcpyHostToDevice));
-    *h->h_status = e;
+    h->h_status[0] = e;
+    h->h_status[1] = e & kErrorWait;
     return MRLBM_OK;
+}
+
+int timed_out(mrlbm_handle *h) { return fail(h, MRLBM_ERR_TIMEOUT, "a wait inside the step kernel ran out: the field is not complete"); }
+
+int settle(mrlbm_handle *h) {
+    CK(h, cudaMemcpyAsync(h->h_status + 1, h->d_error, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    CK(h, cudaStreamSynchronize(h->stream));
+    return (h->h_status[1] & kErrorWait) ? timed_out(h) : MRLBM_OK;
 }
 
 int sync_sr_step(mrlbm_handle *h) {
@@ -137,7 +147,8 @@ void default_tiling(int &ty, int &lz) {
 int setup_tiling(mrlbm_handle *h, int ty, int lz);
 
 // Test hook for the step kernel's bounded waits: MRLBM_FAULT_WAIT_POLLS=k (0: no poll at all) takes the place
-// of the poll limit, so that a wait runs out and the kernel reports it.
+// of the poll limit, so that a wait runs out and the kernel reports it.  Read by each call that steps (for a
+// batch: when it is created).
 int wait_limit() {
     const char *v = std::getenv("MRLBM_FAULT_WAIT_POLLS");
     return v ? std::max(0, std::atoi(v)) : kWaitLimit;
@@ -275,17 +286,23 @@ int setup_tiling(mrlbm_handle *h, int ty, int lz) {
 
 // One or more time steps of one handle: step kernel, node-list kernel, wall kernel and the
 // sampled force / diagnostics reductions, all asynchronous on the handle's stream.
-// The divergence flag as last copied back to the host (no synchronisation: the copy of a
+// The status flags as last copied back to the host (no synchronisation: the copy of a
 // watchdog step lands in the pinned word while later steps are queued).
 bool diverged_seen(const mrlbm_handle *h) {
     return h->h_status && (*(const volatile int *)h->h_status & kErrorDiverged);
 }
+bool timed_out_seen(const mrlbm_handle *h) {
+    const volatile int *s = h->h_status;
+    return s && ((s[0] | s[1]) & kErrorWait);
+}
 
 int step_handle(mrlbm_handle *h, int32_t nsteps) {
+    if (timed_out_seen(h)) return timed_out(h);
     if (diverged_seen(h))
         return fail(h, MRLBM_ERR_DIVERGED, "the divergence watchdog found non-finite mass / energy sums");
     const int nb = (int)(h->geo.wall[0].list.size() + h->geo.wall[1].list.size());
     const int nbf = (int)(h->geo.wall[0].fluid_list.size() + h->geo.wall[1].fluid_list.size());
+    h->args.wait_limit = wait_limit();
     for (int s = 0; s < nsteps; ++s) {
         const int64_t it = h->step;
         const bool fs = h->force_every > 0 && it % h->force_every == 0;
@@ -641,8 +658,8 @@ int mrlbm_create(const mrlbm_case_desc *din, mrlbm_handle **out) {
     CK(H, cudaMalloc((void **)&h->d_error, sizeof(int)));
     CK(H, cudaMemset(h->d_error, 0, sizeof(int)));
     CK(H, cudaMalloc((void **)&h->d_watch, 2 * sizeof(double)));
-    CK(H, cudaHostAlloc((void **)&h->h_status, sizeof(int), cudaHostAllocDefault));
-    *h->h_status = 0;
+    CK(H, cudaHostAlloc((void **)&h->h_status, 2 * sizeof(int), cudaHostAllocDefault));
+    h->h_status[0] = h->h_status[1] = 0;
     h->watchdog_every = d.watchdog_every == 0 ? kWatchdogDefault : (d.watchdog_every < 0 ? 0 : d.watchdog_every);
     CK(H, cudaMalloc((void **)&h->d_force_ring, (size_t)kRing * 10 * sizeof(double)));
     CK(H, cudaMalloc((void **)&h->d_diag_ring, (size_t)kRing * 2 * sizeof(double)));
@@ -766,7 +783,7 @@ int mrlbm_init(mrlbm_handle *h, int32_t kind, const double *params, int32_t n_pa
                      : kind == MRLBM_INIT_NOISY_UNIFORM ? 5 : 0;
     if (n_params < need || (need && !params)) return fail(h, MRLBM_ERR_INVALID_ARG, "missing init parameters");
     for (int k = 0; k < need && k < 8; ++k) ia.p[k] = params[k];
-    if (int rc = clear_divergence(h)) return rc;
+    if (int rc = clear_status(h, true)) return rc;
     CK(h, launch_init(ia, h->storage, h->stream));
     h->parity = 0;
     h->step = 0;
@@ -869,7 +886,7 @@ int mrlbm_sync(mrlbm_handle *h) {
     int e = 0;
     CK(h, cudaMemcpy(&e, h->d_error, sizeof(int), cudaMemcpyDeviceToHost));
     *h->h_status = e;
-    if (e & kErrorWait) return fail(h, MRLBM_ERR_TIMEOUT, "a wait inside the step kernel ran out");
+    if (e & kErrorWait) return timed_out(h);
     if (e & ~kErrorDiverged)
         return fail(h, MRLBM_ERR_CUDA, "device reported a stencil lookup failure (code " + std::to_string(e) + ")");
     if (e & kErrorDiverged)
@@ -899,8 +916,7 @@ int mrlbm_get_moments(mrlbm_handle *h, uint32_t mask, int32_t layout, float *hos
     CK(h, launch_convert(src, nullptr, nullptr, h->d_stage, mask, layout, h->d.nx, h->d.ny, h->d.nz, h->storage, h->sc,
                          0, h->stream));
     CK(h, cudaMemcpyAsync(host, h->d_stage, (size_t)nf * h->n * 4, cudaMemcpyDeviceToHost, h->stream));
-    CK(h, cudaStreamSynchronize(h->stream));
-    return MRLBM_OK;
+    return settle(h);
 }
 
 int mrlbm_set_moments(mrlbm_handle *h, uint32_t mask, int32_t layout, const float *host, size_t count) {
@@ -916,7 +932,7 @@ int mrlbm_set_moments(mrlbm_handle *h, uint32_t mask, int32_t layout, const floa
     void *cur = h->m[h->parity], *oth = h->m[h->parity ^ 1];
     int rc = ensure_stage(h, (size_t)nf * h->n * 4);
     if (rc) return rc;
-    if ((rc = clear_divergence(h)) != MRLBM_OK) return rc;
+    if ((rc = clear_status(h, mask == MRLBM_FIELD_ALL)) != MRLBM_OK) return rc;
     CK(h, cudaMemcpyAsync(h->d_stage, host, (size_t)nf * h->n * 4, cudaMemcpyHostToDevice, h->stream));
     CK(h, launch_convert(nullptr, cur, oth, h->d_stage, mask, layout, h->d.nx, h->d.ny, h->d.nz, h->storage, h->sc, 1,
                          h->stream));
@@ -970,7 +986,7 @@ int mrlbm_get_boundary(mrlbm_handle *h, int32_t wall, int32_t what, int32_t layo
 int mrlbm_get_forces(mrlbm_handle *h, int64_t step, double out[10]) {
     if (!h || !out) return fail(h, MRLBM_ERR_INVALID_ARG, "null argument");
     if (h->host_only) return fail(h, MRLBM_ERR_STATE, "host-only handle has no device state");
-    CK(h, cudaStreamSynchronize(h->stream));
+    if (const int rc = settle(h)) return rc;
     const int64_t lo = std::max<int64_t>(0, h->force_count - kRing);
     for (int64_t c = h->force_count - 1; c >= lo; --c) {
         const int64_t slot = c % kRing;
@@ -985,7 +1001,7 @@ int mrlbm_get_forces(mrlbm_handle *h, int64_t step, double out[10]) {
 int mrlbm_get_force_history(mrlbm_handle *h, int32_t max_steps, int64_t *steps, double *forces, int32_t *n_out) {
     if (!h || !n_out || max_steps < 0) return fail(h, MRLBM_ERR_INVALID_ARG, "bad argument");
     if (h->host_only) return fail(h, MRLBM_ERR_STATE, "host-only handle has no device state");
-    CK(h, cudaStreamSynchronize(h->stream));
+    if (const int rc = settle(h)) return rc;
     const int64_t avail = std::min<int64_t>(h->force_count, kRing);
     const int64_t n = std::min<int64_t>(avail, max_steps);
     std::vector<double> ring((size_t)kRing * 10);
@@ -1003,7 +1019,7 @@ int mrlbm_get_force_history(mrlbm_handle *h, int32_t max_steps, int64_t *steps, 
 int mrlbm_get_diagnostics(mrlbm_handle *h, int32_t max_steps, int64_t *steps, double *values, int32_t *n_out) {
     if (!h || !n_out || max_steps < 0) return fail(h, MRLBM_ERR_INVALID_ARG, "bad argument");
     if (h->host_only) return fail(h, MRLBM_ERR_STATE, "host-only handle has no device state");
-    CK(h, cudaStreamSynchronize(h->stream));
+    if (const int rc = settle(h)) return rc;
     const int64_t avail = std::min<int64_t>(h->diag_count, kRing);
     const int64_t n = std::min<int64_t>(avail, max_steps);
     for (int64_t k = 0; k < n; ++k) {

@@ -68,7 +68,8 @@ struct mrlbm_handle {
     int *d_error = nullptr;
     // divergence watchdog: every watchdog_every steps (0: off) the step computes its FP64 mass /
     // energy sums into d_watch and flags non-finite ones in the error word, whose value is then
-    // copied to the pinned word h_status; mrlbm_step reads h_status without a synchronisation
+    // copied to the pinned word h_status[0]; mrlbm_step reads h_status without a synchronisation.
+    // h_status[1]: the word as of the last read-back (its divergence flag is left to the watchdog)
     int watchdog_every = 0;
     double *d_watch = nullptr;
     int *h_status = nullptr;
@@ -127,8 +128,12 @@ int cuda_fail(mrlbm_handle *h, cudaError_t e, const char *what);
 int ensure_stage(mrlbm_handle *h, size_t bytes);
 // Set the stochastic-rounding step counter to the handle's step (after init, load, restore).
 int sync_sr_step(mrlbm_handle *h);
-// Clear the divergence flag of the device error word and its host copy (new state).
-int clear_divergence(mrlbm_handle *h);
+// Clear the divergence flag of the device error word and its host copies (new state), and the time-out flag
+// when the new state replaces the whole field.
+int clear_status(mrlbm_handle *h, bool whole);
+// Wait for the handle's stream; MRLBM_ERR_TIMEOUT if a step's bounded wait has run out (what the caller is
+// about to hand out is not complete then).
+int settle(mrlbm_handle *h);
 }  // namespace mrlbm
 
 #define CK(h, call)                                                    \

@@ -38,7 +38,7 @@ int check_device(mrlbm_handle *h) {
 
 // Sampled force rows of `wall` not yet written (all of them when `all`), in step order.
 int force_rows(mrlbm_handle *h, int wall, bool all, std::vector<int64_t> &steps, std::vector<double> &f) {
-    CK(h, cudaStreamSynchronize(h->stream));
+    if (const int rc = settle(h)) return rc;
     const int64_t first = std::max<int64_t>(all ? 0 : h->forces_written, h->force_count - kRing);
     const int64_t n = h->force_count - first;
     steps.resize(n);
@@ -256,7 +256,7 @@ int mrlbm_write_inlet_density(mrlbm_handle *h, const char *path, int32_t append)
     if (!h) return fail(nullptr, MRLBM_ERR_INVALID_ARG, "null handle");
     if (h->host_only) return fail(h, MRLBM_ERR_STATE, "host-only handle has no device state");
     if (!path || !h->d_inlet) return fail(h, MRLBM_ERR_INVALID_ARG, "no inlet samples (mrlbm_set_pressure_window)");
-    CK(h, cudaStreamSynchronize(h->stream));
+    if (const int rc = settle(h)) return rc;
     const int64_t first = std::max<int64_t>(append ? h->inlet_written : 0, h->ps_count - kRing);
     const int64_t n = h->ps_count - first;
     std::vector<double> e((size_t)std::max<int64_t>(n, 0) * 2);
@@ -319,7 +319,7 @@ int mrlbm_write_pressure(mrlbm_handle *h, int32_t wall, const char *path) {
         return fail(h, MRLBM_ERR_INVALID_ARG, "no pressure samples for this wall (mrlbm_set_pressure_window)");
     const WallData &W = h->geo.wall[wall];
     std::vector<double> ps(W.list.size());
-    CK(h, cudaStreamSynchronize(h->stream));
+    if (const int rc = settle(h)) return rc;
     CK(h, cudaMemcpy(ps.data(), h->d_ps_avg[wall], ps.size() * sizeof(double), cudaMemcpyDeviceToHost));
     std::ofstream out(path);
     if (!out) return fail(h, MRLBM_ERR_IO, std::string("cannot open ") + path);

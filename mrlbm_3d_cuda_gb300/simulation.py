@@ -119,7 +119,8 @@ class Simulation:
 
     def sync(self):
         """Wait for the queued steps; raises on a device error or non-finite diagnostics
-        (MRLBM_ERR_DIVERGED)."""
+        (MRLBM_ERR_DIVERGED), or when a kernel's bounded wait ran out (MRLBM_ERR_TIMEOUT; every read-back
+        raises that too until a new field is set)."""
         self._ck(N.lib().mrlbm_sync(self._h))
 
     def run(self, max_iter: int, macr_save: int = 0, stat_start: int = 0, stat_end: int = -1):

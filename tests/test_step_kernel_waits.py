@@ -1,6 +1,6 @@
 """The step kernel's bounded waits: one that runs out ends in a status, with the kernel's copies landed and the
-context usable.  The limit comes from the host (MRLBM_FAULT_WAIT_POLLS polls, read when a handle is
-created): with 0 the warps that own the tile's rows give up at their first wait, while the copies of the
+context usable.  The limit comes from the host (MRLBM_FAULT_WAIT_POLLS polls, read by each call that
+steps): with 0 the warps that own the tile's rows give up at their first wait, while the copies of the
 first planes are on their way; with a few, some waits run out and some do not.  A wait on copies that nobody
 has issued would take the full limit, 16 s: each run ends long before that."""
 from __future__ import annotations
@@ -87,3 +87,44 @@ def test_allocation_free_step_reports_a_wait_that_ran_out(cuda_device, monkeypat
             assert not got.any()
         assert call(got, sums) == N.OK
         assert torch.equal(got, want) and list(sums) == list(want_sums)
+
+
+def test_timed_out_handle_hands_out_nothing(cuda_device, monkeypatch, tmp_path):
+    """After a wait ran out every read-back returns the status instead of the field's remains, and so does
+    the next step once a read-back has seen it; a part of a new field does not clear it, a whole one does."""
+    from mrlbm_3d_cuda_gb300 import Simulation
+    from mrlbm_3d_cuda_gb300 import native as N
+    init = N.INIT_NOISY_UNIFORM, (0.05, 0.0, 0.0, 0.01, 5)
+
+    def refused(call):
+        with pytest.raises(N.MrlbmError) as e:
+            call()
+        return e.value.code == N.ERR_TIMEOUT
+
+    with Simulation(descs("channel"), init=False) as sim:
+        sim.init(*init)
+        sim.set_sampling(1, 1)
+        sim.set_pressure_window(0, 100)
+        field = sim.moments()
+        sim.step(3)
+        want = sim.moments()
+        sim.init(*init)
+        monkeypatch.setenv("MRLBM_FAULT_WAIT_POLLS", "0")
+        sim.step(3)
+        monkeypatch.delenv("MRLBM_FAULT_WAIT_POLLS")
+        assert refused(sim.moments)
+        assert refused(sim.force_history) and refused(sim.diagnostics) and refused(lambda: sim.forces(1))
+        assert refused(lambda: sim.checkpoint_save(str(tmp_path / "restart.bin")))
+        assert refused(lambda: sim.write_vti(str(tmp_path / "data.vti")))
+        assert refused(lambda: sim.write_forces(str(tmp_path / "forces.dat")))
+        assert refused(lambda: sim.write_pressure(str(tmp_path / "pressure.dat")))
+        assert refused(lambda: sim.write_inlet_density(str(tmp_path / "inlet.dat")))
+        assert refused(lambda: sim.step(1)) and refused(sim.sync)
+        sim.set_moments(field[1:2], fields=["ux"])
+        assert refused(sim.moments)
+        sim.set_moments(field)
+        assert np.array_equal(sim.moments(), field)
+        sim.init(*init)
+        sim.step(3)
+        sim.sync()
+        assert np.array_equal(sim.moments(), want)
