@@ -1151,6 +1151,7 @@ int batch_set_tiling(mrlbm_batch *b, int ty, int lz) {
     BCK(cudaMemset(b->d_slot, 0, sizeof(int)));
     BatchArgs ba;
     ba.cases = b->d_cases;
+    ba.n_cases = n;
     ba.items = b->d_items;
     ba.n_items = b->n_items;
     ba.list_blocks = b->d_list_blocks;

@@ -103,6 +103,7 @@ struct StepArgs {
 // Lives in device memory; the kernels read each case's own StepArgs through `cases`.
 struct BatchArgs {
     const StepArgs *const *cases = nullptr;  // device StepArgs of each case
+    int n_cases = 0;
     const int2 *items = nullptr;             // {case, tile | z-segment << 20}
     int n_items = 0;
     const int4 *list_blocks = nullptr;       // per node-list block: {case, first block of the case, blocks, 0}

@@ -358,6 +358,13 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
     };
     const int n_items = BATCH ? ba->n_items : single.n_items;
     const int limit = BATCH ? ba->cases[0]->wait_limit : single.wait_limit;
+    // a wait ran out: which items are left undone is not known, so every case of a batch has it
+    auto report = [&]() {
+        if constexpr (BATCH)
+            for (int c = 0; c < ba->n_cases; ++c) atomicOr_system(ba->cases[c]->error, kErrorWait);
+        else
+            atomicOr_system(single.error, kErrorWait);
+    };
 
     if (warp >= TY) {
         if constexpr (G::SPLIT) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
@@ -513,7 +520,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
                 mbar_arrive(full + stage);
             }
         }
-        if (!ok && lane == 0) atomicOr_system(BATCH ? ba->cases[0]->error : single.error, kErrorWait);
+        if (!ok && lane == 0) report();
         // The CTA stays until its copies have landed, also when a wait ran out and its owners are gone: the
         // shared memory that they fill would be the next CTA's.  No halo warp issues another one past the
         // barrier; a stage's last use is the one under way or the last that ended, so its parity tells.
@@ -767,7 +774,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
                 ++items;
             }
         }
-        if (!ok && lane == 0) atomicOr_system(BATCH ? ba->cases[0]->error : single.error, kErrorWait);
+        if (!ok && lane == 0) report();
     }
 }
 

@@ -128,3 +128,30 @@ def test_timed_out_handle_hands_out_nothing(cuda_device, monkeypatch, tmp_path):
         sim.step(3)
         sim.sync()
         assert np.array_equal(sim.moments(), want)
+
+
+def test_timed_out_batch_reports_every_case(cuda_device, monkeypatch):
+    """Which items a batched launch left undone is not known: each case's handle has the status, and a new
+    field for all of them steps again (the limit of a batch is the one it was created with)."""
+    from mrlbm_3d_cuda_gb300 import Batch, cases
+    from mrlbm_3d_cuda_gb300 import native as N
+    monkeypatch.setenv("MRLBM_FAULT_WAIT_POLLS", "0")
+    b = Batch([cases.periodic_box(64, 24, 8, u0=0.05, re=100.0, length=8.0), descs("channel"), descs("periodic")])
+    monkeypatch.delenv("MRLBM_FAULT_WAIT_POLLS")
+    for c in b.cases:
+        c.init(N.INIT_NOISY_UNIFORM, (0.03, 0.0, 0.0, 0.01, 5))
+    before = [c.moments() for c in b.cases]
+    b.step(2)
+    for c in b.cases:
+        for call in (c.sync, c.moments):
+            with pytest.raises(N.MrlbmError) as e:
+                call()
+            assert e.value.code == N.ERR_TIMEOUT
+    with pytest.raises(N.MrlbmError) as e:
+        b.sync()
+    assert e.value.code == N.ERR_TIMEOUT
+    for c, m in zip(b.cases, before):
+        c.set_moments(m)
+        assert np.array_equal(c.moments(), m)
+    b.sync()
+    b.close()
