@@ -238,7 +238,7 @@ int setup_tiling(mrlbm_handle *h, int ty, int lz) {
     h->lz = lz;
     const int nseg = (d.nz + h->lz - 1) / h->lz;
     // work items are int32 `tile | segment << 20` (decoded in step_kernel)
-    if (tiles > (1 << 20) || nseg > (1 << 11))
+    if (tiles > (1 << 20) || nseg > kMaxSegments)
         return fail(h, MRLBM_ERR_INVALID_ARG,
                     "grid too large for the work-item encoding (at most 2^20 xy tiles and 2^11 z segments)");
     // tiles with boundary nodes first: they cost most, and CTAs take over items in this order

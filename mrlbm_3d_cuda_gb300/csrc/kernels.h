@@ -69,6 +69,9 @@ struct WallArgs {
 // Polls after which a wait of the step kernel gives up (see packed.cuh).
 constexpr int kWaitLimit = 1 << 22;
 
+// z-segments of a grid: work items are int32 `tile | segment << 20`.
+constexpr int kMaxSegments = 1 << 11;
+
 // One copy lives in device memory per handle; kernels receive a pointer to it plus the
 // per-step scalars (ping-pong parity, sampling buffers).
 struct StepArgs {

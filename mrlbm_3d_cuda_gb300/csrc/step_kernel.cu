@@ -934,7 +934,7 @@ void choose_tiling(int nx, int ny, int nz, int storage, int n_sm, int &ty, int &
     const int64_t tiles = active > 0 ? active : (int64_t)((nx + TILE_X - 1) / TILE_X) * ((ny + ty - 1) / ty);
     const double list = (storage == MRLBM_STORAGE_F32 ? 0.03 : (storage == MRLBM_STORAGE_F16_U32 ? 0.024 : 0.02)) * list_nodes;
     double best = 1e300;
-    for (int nseg = 1; nseg <= std::min(nz, 1 << 11); ++nseg) {
+    for (int nseg = 1; nseg <= std::min(nz, kMaxSegments); ++nseg) {
         const int l = (nz + nseg - 1) / nseg;
         const int64_t items = tiles * ((nz + l - 1) / l), t = (items + slots - 1) / slots * (2 * l + 7);
         const double rest = list - (double)(slots * t - items * (2 * l + 7));
@@ -952,8 +952,9 @@ int choose_batch_lz(const std::vector<int> &tiles, const std::vector<int> &nz, i
     const double slots = (double)std::max(1, step_kernel_max_ctas_per_sm(storage, ty)) * n_sm;
     const int top = *std::max_element(nz.begin(), nz.end());
     double best = 1e300;
-    int lz = 1;
-    for (int l = 1; l <= top; ++l) {
+    int lz = top;
+    // (a work item holds 11 bits of segment: no more segments than that for the tallest case)
+    for (int l = (top + kMaxSegments - 1) / kMaxSegments; l <= top; ++l) {
         double work = 0.0;
         for (size_t c = 0; c < nz.size(); ++c) {
             const int seg = (nz[c] + l - 1) / l;

@@ -36,3 +36,23 @@ def test_rows_past_the_tile(cuda_device, kind, storage, monkeypatch):
     assert np.isfinite(want).all()
     got = fields(monkeypatch, desc, init, 12, 16)
     assert np.array_equal(got, want)
+
+
+def test_tall_narrow_case_in_a_batch(cuda_device):
+    """The segment length chosen for a batch keeps the tallest case's segments within a work item's 11 bits: one
+    column of 220,000 planes would otherwise be cut into 2200 segments and refused."""
+    from mrlbm_3d_cuda_gb300 import Batch, Simulation, cases
+    from mrlbm_3d_cuda_gb300 import native as N
+    desc = cases.periodic_box(8, 8, 220000, u0=0.05, re=100.0, length=8.0, storage=1)
+    init = N.INIT_NOISY_UNIFORM, (0.03, 0.01, -0.02, 0.3, 13)
+    with Simulation(desc, init=False) as sim:
+        sim.init(*init)
+        sim.step(2)
+        sim.sync()
+        want = sim.moments()
+    b = Batch([desc])
+    b.cases[0].init(*init)
+    b.step(2)
+    b.sync()
+    assert np.array_equal(b.cases[0].moments(), want)
+    b.close()
