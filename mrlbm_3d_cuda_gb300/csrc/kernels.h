@@ -98,7 +98,7 @@ struct StepArgs {
     // stochastic rounding of 16-bit stores: the step counter that seeds the random bits
     // (null: round to nearest)
     const uint32_t *sr_step = nullptr;
-    int wait_limit = kWaitLimit;          // of the owner warps' waits (the halo warps': at least 1)
+    int wait_limit = kWaitLimit;          // 0: the owner warps' first wait counts as run out
 };
 
 // Several independent cases advanced together: one step-kernel launch over the work items of

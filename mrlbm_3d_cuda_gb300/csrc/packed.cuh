@@ -75,7 +75,7 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
     asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes)
                  : "memory");
 }
-// Waits for the phase of the given parity.  They give up after `limit` polls and return false: kWaitLimit polls
+// Waits for the phase of the given parity.  They give up after 1 + `limit` polls and return false: kWaitLimit polls
 // that find nothing take 16 s (3.8 us each), far beyond any copy or plane of work.  (A suspend-time hint
 // on the polls made them sleep: up to 2.5 times slower steps.)
 __device__ __forceinline__ bool mbar_try(uint32_t a, uint32_t parity) {
@@ -93,7 +93,7 @@ __device__ __forceinline__ bool mbar_try(uint32_t a, uint32_t parity) {
 // that what follows (shuffles, the release of a stage by lane 0) finds the warp whole.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int limit) {
     const uint32_t a = smem_addr(bar);
-    bool done = false;
+    bool done = mbar_try(a, parity);
 #pragma unroll 1
     for (int i = 0; !done && i < limit; ++i) done = mbar_try(a, parity);
     return __all_sync(0xffffffffu, done);

@@ -323,8 +323,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
     extern __shared__ __align__(128) unsigned char smem[];
     uint32_t *const stages = reinterpret_cast<uint32_t *>(smem);
     float *const halos = reinterpret_cast<float *>(smem + G::D * G::STAGEW * 4);
-    // {case, work item, its number} of the item that starts with the stage's plane; 1 + the parity of the
-    // stage's last use (0: none yet)
+    // {case, work item, its number} of the item that starts with the stage's plane
     int4 *const heads = reinterpret_cast<int4 *>(smem + G::D * (G::STAGEW * 4 + 2 * TY * G::HALO * 4));
     uint64_t *const full = reinterpret_cast<uint64_t *>(heads + G::D);
     uint64_t *const empty = full + G::D;
@@ -333,7 +332,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
     __shared__ __align__(16) uint4 s_slot[2];  // answers to takeover requests, by item parity
     __shared__ uint64_t s_taken;
     __shared__ int s_next[2];
-    __shared__ int s_failed;  // a halo warp's wait ran out
+    __shared__ int s_failed;  // 1 + the plane at which a halo warp's wait ran out: none is issued from there on
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -341,7 +340,6 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
             mbar_init(full + s, 1);
             mbar_init(empty + s, TY);
             mbar_init(landed + s, 1);
-            heads[s] = make_int4(0, 0, 0, 0);
         }
         mbar_init(&s_taken, 1);
         s_failed = 0;
@@ -375,8 +373,10 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
         int n = 0;        // items so far
         auto take_turn = [&]() {
             if (G::NH > 1 && q > 0) token_wait(3 + hw);
-            if (ok) ok = *(const volatile int *)&s_failed == 0 && mbar_wait(empty + stage, phase ^ 1u, max(limit, 1));
-            if (!ok && lane == 0) *(volatile int *)&s_failed = 1;
+            if (!ok) return;
+            volatile int *const failed = &s_failed;
+            ok = (G::NH == 1 || *failed == 0) && mbar_wait(empty + stage, phase ^ 1u, limit);
+            if (!ok && lane == 0 && *failed == 0) *failed = q + 1;
         };
         // Work items.  SPECIAL: one CTA per item is launched, and a CTA that finishes its item takes over
         // one that has not started (tiles with boundary nodes and the cases of a batch cost unevenly).
@@ -445,8 +445,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
                 uint32_t *const sp = stages + stage * G::STAGEW;
                 uint32_t *const cp = sp + (TY + 2) * G::ROWW;  // [word][column]
                 if (lane == 0) {
-                    if (k == 0) heads[stage] = make_int4(head.x, head.y, it, (int)phase + 1);
-                    else heads[stage].w = (int)phase + 1;
+                    if (k == 0) heads[stage] = make_int4(head.x, head.y, it, 0);
                     mbar_expect_tx(landed + stage, row_bytes * (h + 2) + (marked(k) ? TILE_X * (uint32_t)h : 0u));
                     mbar_arrive(landed + stage);
                 }
@@ -503,10 +502,11 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
                 if (leader) {
                     const bool answered = mbar_wait_lane(&s_taken, n & 1);
                     s_next[n & 1] = answered ? takeover_result(s_slot + (n & 1)) : -1;
-                    if (!answered) *(volatile int *)&s_failed = 1;
+                    if (!answered && s_failed == 0) *(volatile int *)&s_failed = q + 1;
                 }
                 asm volatile("bar.sync 2, %0;" ::"r"(32 * G::NH) : "memory");
                 it = s_next[n & 1];
+                if (*(const volatile int *)&s_failed) ok = false;
                 ++n;
             } else {
                 it += (int)gridDim.x;
@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
         if (q % G::NH == hw) {
             take_turn();
             if (ok && lane == 0) {
-                heads[stage] = make_int4(0, -1, 0, (int)phase + 1);  // end mark
+                heads[stage] = make_int4(0, -1, 0, 0);  // end mark: plane q
                 mbar_arrive(landed + stage);
                 mbar_arrive(full + stage);
             }
@@ -523,15 +523,17 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
         if (!ok && lane == 0) report();
         // The CTA stays until its copies have landed, also when a wait ran out and its owners are gone: the
         // shared memory that they fill would be the next CTA's.  No halo warp issues another one past the
-        // barrier; a stage's last use is the one under way or the last that ended, so its parity tells.
+        // barrier; all planes before the failed one were issued (or all, and the end mark), and the last D
+        // are the stages' last uses, under way or the last that ended, so their parities tell.
         asm volatile("bar.sync 2, %0;" ::"r"(32 * G::NH) : "memory");
-        if (threadIdx.x == 32 * TY)
-            for (int s = 0; s < G::D; ++s)
-                if (heads[s].w) mbar_wait_lane(landed + s, (uint32_t)(heads[s].w - 1));
+        if (threadIdx.x == 32 * TY) {
+            const int issued = s_failed ? s_failed - 1 : q + 1;
+            for (int p = max(0, issued - G::D); p < issued; ++p) mbar_wait_lane(landed + p % G::D, (uint32_t)(p / G::D) & 1u);
+        }
     } else {
         if constexpr (G::SPLIT) asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
         // ---- owner warps -----------------------------------------------------------------------
-        bool ok = true;
+        bool ok = limit > 0;  // 0: the first wait has run out
         int items = 0;
         while (ok) {
             // landed before full, here and in every plane: rows past the tile's last one skip the waits on
