@@ -153,7 +153,7 @@ typedef struct mrlbm_info {
     int32_t storage;
     int32_t bytes_per_value;
     int32_t n_active_items;  /* work items (tile column x z-segment) the step kernel visits */
-    int32_t tile[3];      /* x-block (a tile is two wide), tile height, z-segment length   */
+    int32_t tile[3];      /* x-block, tile height, z-segment length (mrlbm_autotune)       */
     int32_t nb_solid[2];  /* BCSOLID nodes per wall (z walls only)                       */
     int32_t reserved[6];
 } mrlbm_info;
@@ -268,7 +268,7 @@ int mrlbm_step_periodic_noalloc(const float *m_in, float *m_out, int32_t nx, int
  * powers of two below nz) over `trial_steps` steps and keep the fastest.  The moments, step
  * counter and sampling state are restored afterwards; results do not depend on the tiling.
  * tile_out (optional): {32, tile height, z-segment length}; 32 is the x-block of the moment layout, a tile
- * being two blocks wide. */
+ * being two blocks wide (a grid of at most 32 nodes along x: one block, and 32 rows in place of 16). */
 int mrlbm_autotune(mrlbm_handle *h, int32_t trial_steps, int32_t tile_out[3]);
 /* Several independent cases (uneven grids allowed; one moment storage for all) advanced
  * together: per step one persistent step-kernel launch over the work items of every case,

@@ -165,7 +165,7 @@ int storage_element_bytes(int storage) {
 int setup_tiling(mrlbm_handle *h, int ty, int lz) {
     const mrlbm_case_desc &d = h->d;
     const Geometry &g = h->geo;
-    if (ty != 4 && ty != 8 && ty != 16) ty = 16;
+    ty = tile_height(d.nx, ty);
     CK(h, cudaStreamSynchronize(h->stream));
     for (void **p : {(void **)&h->d_tile_slot, (void **)&h->d_side, (void **)&h->d_items, (void **)&h->d_list_xyz,
                      (void **)&h->d_list_word, (void **)&h->d_diag_part}) {
@@ -263,7 +263,7 @@ int setup_tiling(mrlbm_handle *h, int ty, int lz) {
     }
     CK(h, upload(&h->d_items, items.data(), items.size()));
     CK(h, cudaMalloc((void **)&h->d_diag_part,
-                     ((size_t)h->n_ctas * h->tile_y + h->n_list_blocks) * 2 * sizeof(double)));
+                     ((size_t)h->n_ctas * owner_warps(h->tile_y) + h->n_list_blocks) * 2 * sizeof(double)));
     if (h->n_list > 0) {
         CK(h, upload(&h->d_list_xyz, list_xyz.data(), list_xyz.size()));
         CK(h, upload(&h->d_list_word, list_word.data(), list_word.size()));
@@ -338,7 +338,7 @@ int step_handle(mrlbm_handle *h, int32_t nsteps) {
         if (h->n_list > 0) {
             if (L.placed) CK(h, cudaStreamWaitEvent(h->list_stream, h->ev_placed, 0));
             CK(h, launch_special_list(L, h->storage, h->n_list_blocks,
-                                      sums ? h->d_diag_part + 2 * (size_t)h->n_ctas * h->tile_y : nullptr,
+                                      sums ? h->d_diag_part + 2 * (size_t)h->n_ctas * owner_warps(h->tile_y) : nullptr,
                                       h->list_stream));
             CK(h, cudaEventRecord(h->ev_list, h->list_stream));
             CK(h, cudaStreamWaitEvent(h->stream, h->ev_list, 0));
@@ -358,7 +358,7 @@ int step_handle(mrlbm_handle *h, int32_t nsteps) {
                                               h->stream));
         }
         if (sums) {
-            const int parts = h->n_ctas * h->tile_y + (h->n_list > 0 ? h->n_list_blocks : 0);
+            const int parts = h->n_ctas * owner_warps(h->tile_y) + (h->n_list > 0 ? h->n_list_blocks : 0);
             if (ds) {
                 const int64_t slot = h->diag_count % kRing;
                 CK(h, launch_diag_finalize(h->d_diag_part, parts, h->d_diag_ring + slot * 2, h->d_error, h->stream));
@@ -1097,7 +1097,8 @@ int batch_set_tiling(mrlbm_batch *b, int ty, int lz) {
     if (l <= 0) {
         std::vector<int> tiles, nz;
         for (const mrlbm_handle *h : b->h) {
-            tiles.push_back(((h->d.nx + TILE_X - 1) / TILE_X) * ((h->d.ny + ty - 1) / ty));
+            const int rows = tile_height(h->d.nx, ty);
+            tiles.push_back(((h->d.nx + TILE_X - 1) / TILE_X) * ((h->d.ny + rows - 1) / rows));
             nz.push_back(h->d.nz);
         }
         l = choose_batch_lz(tiles, nz, b->storage, b->h[0]->n_sm, ty);
@@ -1112,14 +1113,18 @@ int batch_set_tiling(mrlbm_batch *b, int ty, int lz) {
     const int n = (int)b->h.size();
     std::vector<const StepArgs *> cases(n);
     std::vector<double *> ring(n);
-    std::vector<int2> items, plain;  // tiles with boundary nodes of every case first
+    // work items, by kernel (0: two x-blocks wide, 1: one): tiles with boundary nodes of every case first
+    std::vector<int2> items[2], plain[2];
+    b->special[0] = b->special[1] = false;
     std::vector<int4> lblocks, wblocks;
     for (int c = 0; c < n; ++c) {
         mrlbm_handle *h = b->h[c];
         cases[c] = h->d_args;
         ring[c] = h->d_force_ring;
+        const int kernel = h->tile_y == 32;
+        b->special[kernel] = b->special[kernel] || h->special;
         for (size_t k = 0; k < h->h_items.size(); ++k)
-            ((int)k < h->n_special_items ? items : plain).push_back(make_int2(c, h->h_items[k]));
+            ((int)k < h->n_special_items ? items : plain)[kernel].push_back(make_int2(c, h->h_items[k]));
         if (h->n_list > 0) {
             const int first = (int)lblocks.size();
             for (int k = 0; k < h->n_list_blocks; ++k) lblocks.push_back(make_int4(c, first, h->n_list_blocks, 0));
@@ -1131,8 +1136,11 @@ int batch_set_tiling(mrlbm_batch *b, int ty, int lz) {
             for (int k = 0; k < nblk; ++k) wblocks.push_back(make_int4(c, first, nblk, 0));
         }
     }
-    items.insert(items.end(), plain.begin(), plain.end());
-    b->n_items = (int)items.size();
+    for (int k = 0; k < 2; ++k) {
+        items[k].insert(items[k].end(), plain[k].begin(), plain[k].end());
+        b->n_items[k] = (int)items[k].size();
+    }
+    items[0].insert(items[0].end(), items[1].begin(), items[1].end());
     b->n_list_blocks = (int)lblocks.size();
     b->n_wall_blocks = (int)wblocks.size();
     auto up = [&](auto **dptr, const auto &v) -> cudaError_t {
@@ -1144,7 +1152,7 @@ int batch_set_tiling(mrlbm_batch *b, int ty, int lz) {
     };
     BCK(up(&b->d_cases, cases));
     BCK(up(&b->d_ring, ring));
-    BCK(up(&b->d_items, items));
+    BCK(up(&b->d_items, items[0]));
     BCK(up(&b->d_list_blocks, lblocks));
     BCK(up(&b->d_wall_blocks, wblocks));
     BCK(cudaMalloc((void **)&b->d_slot, sizeof(int)));
@@ -1152,27 +1160,38 @@ int batch_set_tiling(mrlbm_batch *b, int ty, int lz) {
     BatchArgs ba;
     ba.cases = b->d_cases;
     ba.n_cases = n;
-    ba.items = b->d_items;
-    ba.n_items = b->n_items;
     ba.list_blocks = b->d_list_blocks;
     ba.wall_blocks = b->d_wall_blocks;
     ba.force_ring = b->d_ring;
     ba.force_slot = b->d_slot;
-    BCK(cudaMalloc((void **)&b->d_ba, sizeof(BatchArgs)));
-    BCK(cudaMemcpy(b->d_ba, &ba, sizeof(BatchArgs), cudaMemcpyHostToDevice));
-    BCK(prepare_step_batch(b->storage, ty));  // both variants, before any capture
+    BCK(cudaMalloc((void **)&b->d_ba, 2 * sizeof(BatchArgs)));
+    for (int k = 0; k < 2; ++k) {
+        ba.items = b->d_items + (k ? b->n_items[0] : 0);
+        ba.n_items = b->n_items[k];
+        BCK(cudaMemcpy(b->d_ba + k, &ba, sizeof(BatchArgs), cudaMemcpyHostToDevice));
+        if (b->n_items[k] > 0) BCK(prepare_step_batch(b->storage, k ? 32 : ty, b->special[k]));  // before any capture
+    }
     return MRLBM_OK;
 }
 
-// The three batched launches of one step.
+// The batched launches of one step.
 int batch_launch(mrlbm_batch *b, int parity, int force) {
+    const bool both = b->n_items[0] > 0 && b->n_items[1] > 0;  // kinds of tiles: their kernels run side by side
+    if (b->n_list_blocks > 0 || both) BCK(cudaEventRecord(b->ev_fork, b->stream));
     if (b->n_list_blocks > 0) {
-        BCK(cudaEventRecord(b->ev_fork, b->stream));
         BCK(cudaStreamWaitEvent(b->side_stream, b->ev_fork, 0));
         BCK(launch_special_list_batch(b->d_ba, parity, force, b->storage, b->n_list_blocks, b->side_stream));
         BCK(cudaEventRecord(b->ev_join, b->side_stream));
     }
-    if (b->n_items > 0) BCK(launch_step_batch(b->d_ba, parity, b->storage, b->tile_y, b->n_items, b->stream));
+    if (both) BCK(cudaStreamWaitEvent(b->narrow_stream, b->ev_fork, 0));
+    for (int k = 0; k < 2; ++k)
+        if (b->n_items[k] > 0)
+            BCK(launch_step_batch(b->d_ba + k, parity, b->storage, k ? 32 : b->tile_y, b->special[k], b->n_items[k],
+                                  k && both ? b->narrow_stream : b->stream));
+    if (both) {
+        BCK(cudaEventRecord(b->ev_narrow, b->narrow_stream));
+        BCK(cudaStreamWaitEvent(b->stream, b->ev_narrow, 0));
+    }
     if (b->n_list_blocks > 0) BCK(cudaStreamWaitEvent(b->stream, b->ev_join, 0));
     BCK(launch_wall_batch(b->d_ba, parity, force, b->storage, b->n_wall_blocks, b->stream));
     bool any_sr = false;
@@ -1273,6 +1292,8 @@ int mrlbm_batch_create(const mrlbm_case_desc *descs, int32_t n, mrlbm_batch **ou
     b->storage = b->h[0]->storage;
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&b->side_stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&b->narrow_stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&b->ev_narrow, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming) != cudaSuccess) {
         cleanup();
@@ -1308,6 +1329,8 @@ int mrlbm_batch_destroy(mrlbm_batch *b) {
     }
     if (b->stream) cudaStreamDestroy(b->stream);
     if (b->side_stream) cudaStreamDestroy(b->side_stream);
+    if (b->narrow_stream) cudaStreamDestroy(b->narrow_stream);
+    if (b->ev_narrow) cudaEventDestroy(b->ev_narrow);
     if (b->ev_fork) cudaEventDestroy(b->ev_fork);
     if (b->ev_join) cudaEventDestroy(b->ev_join);
     delete b;

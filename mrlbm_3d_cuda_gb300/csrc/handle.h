@@ -101,7 +101,8 @@ struct mrlbm_batch {
     std::vector<mrlbm_handle *> h;
     cudaStream_t stream = nullptr;
     cudaStream_t side_stream = nullptr;  // node-list launch, forked / joined by events
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    cudaStream_t narrow_stream = nullptr;  // step kernel of tiles one x-block wide, beside that of the others
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_narrow = nullptr;
     int storage = 0, tile_y = 16, lz = 0;
     int parity = 0;
     int64_t step = 0;
@@ -109,12 +110,13 @@ struct mrlbm_batch {
     int64_t force_count = 0;  // sampled steps so far (the ring slot of the cases with walls)
     // device tables (BatchArgs and what it points to)
     const StepArgs **d_cases = nullptr;
-    int2 *d_items = nullptr;  // work items, tiles with boundary nodes first
+    int2 *d_items = nullptr;  // work items of the cases with tiles two x-blocks wide, then of those with one
     int4 *d_list_blocks = nullptr, *d_wall_blocks = nullptr;
     double **d_ring = nullptr;
     int *d_slot = nullptr;
-    BatchArgs *d_ba = nullptr;
-    int n_items = 0, n_list_blocks = 0, n_wall_blocks = 0;
+    BatchArgs *d_ba = nullptr;  // [2], by kind of tile
+    bool special[2] = {false, false};  // some case with such tiles has boundary nodes
+    int n_items[2] = {0, 0}, n_list_blocks = 0, n_wall_blocks = 0;
     cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // [parity][force]
 };
 

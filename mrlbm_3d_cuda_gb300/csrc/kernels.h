@@ -121,7 +121,7 @@ struct StepLaunch {
     const StepArgs *args = nullptr;  // host copy, passed by value to the step kernel
     int parity = 0;                // read m[parity], write m[parity ^ 1]
     double *force = nullptr;       // [2][5] FP64 accumulators of a sampled step, or null
-    double *diag_part = nullptr;   // [n_ctas][tile_y][2] mass / energy partials, or null
+    double *diag_part = nullptr;   // [n_ctas][owner_warps(tile_y)][2] mass / energy partials, or null
     int n_ctas = 0;                // special: one per work item
     cudaEvent_t placed = nullptr;  // recorded when the last CTA of the step kernel has started, or null
 };
@@ -132,16 +132,25 @@ inline __host__ __device__ int64_t side_index(int slot, int x, int y, int z, int
     return (((int64_t)slot * nz + z) * tile_y + (y - y0)) * tile_x + (x - x0);
 }
 
+// Tile height: 4, 8 or 16 (the default) rows of TILE_X nodes; grids of at most one x-block take 32 rows of it in
+// place of 16 of two.
+inline int tile_height(int nx, int asked) {
+    return asked == 4 || asked == 8 ? asked : (nx <= kXBlock ? 32 : 16);
+}
+// Warps of the step kernel that own a tile's rows.
+inline int owner_warps(int tile_y) { return tile_y < 16 ? tile_y : 16; }
+
 // storage: 0 f32, 1 f16, 2 bf16
 cudaError_t launch_step(const StepLaunch &l, int storage, int tile_y, bool special, cudaStream_t s);
-cudaError_t launch_step_batch(const BatchArgs *ba, int parity, int storage, int tile_y, int n_items, cudaStream_t s);
-cudaError_t prepare_step_batch(int storage, int tile_y);  // before capturing batched launches
+cudaError_t launch_step_batch(const BatchArgs *ba, int parity, int storage, int tile_y, bool special, int n_items,
+                              cudaStream_t s);
+cudaError_t prepare_step_batch(int storage, int tile_y, bool special);  // before capturing batched launches
 cudaError_t launch_special_list_batch(const BatchArgs *ba, int parity, int force, int storage, int n_blocks,
                                       cudaStream_t s);
 cudaError_t launch_wall_batch(const BatchArgs *ba, int parity, int force, int storage, int n_blocks, cudaStream_t s);
 // Zero the slot of every case's force ring and publish the slot for the batched wall kernel.
 cudaError_t launch_batch_force_begin(double *const *ring, int n_cases, int slot, int *d_slot, cudaStream_t s);
-// Tile height (4, 8 or 16; any other value on entry: the default) and z-segment length (> 0 on entry:
+// Tile height (tile_height of the one on entry) and z-segment length (> 0 on entry:
 // kept, clipped to nz); active: tiles that are updated (0: all); list_nodes: nodes of the node-list kernel.
 void choose_tiling(int nx, int ny, int nz, int storage, int n_sm, int &ty, int &lz, int active = 0, int list_nodes = 0);
 // z-segment length of a batch's merged items: tiles[c] of nz[c] planes each.

@@ -36,7 +36,10 @@
 namespace mrlbm {
 namespace {
 
-// A CTA owns a column of TILE_X x TY nodes and marches along z.
+// A CTA owns a column of TILE_X x TY nodes and marches along z.  (TY = 32, for grids of at most 32 nodes along x: a
+// tile is 32 rows of one x-block, an owner warp holds two rows, 16 lanes each, and a row wraps within
+// itself, so there are no side columns and no halo values.  In 64-node tiles half the lanes or more are idle there:
+// 32 x 512 x 512 194 us a step in FP32 and 212 in FP16, in such tiles 108 and 107; 8 x 1024 x 1024 709 -> 336.)
 //   owner warps (one per row): lane l owns the nodes x0 + 2 l and x0 + 2 l + 1;
 //   halo warps (every NH-th plane each): issue the bulk copies of a plane's rows (own columns, rows
 //     y0 - 1 .. y0 + TY) into a ring of D plane stages, and evaluate the x-pass values that enter the
@@ -48,26 +51,30 @@ namespace {
 // from one work item to the next, so there is no drain between items.
 template <typename S, int TY, bool SPECIAL>
 struct Geo {
+    static constexpr bool NARROW = TY == 32;
+    static constexpr int RPW = NARROW ? 2 : 1;               // rows of one owner warp
+    static constexpr int OW = TY / RPW;                      // owner warps
+    static constexpr int XW = TILE_X / RPW;                  // nodes of one row
     static constexpr int WPN = StorageLayout<S>::words;      // 32-bit words of one node
-    static constexpr int ROWW = 2 * WPN * kXBlock;           // words of one row (two x-blocks)
-    static constexpr int SIDEC = 2 * (TY + 2);               // columns beside the tile, corners included
-    static constexpr int MARKW = SPECIAL ? TY * TILE_X / 4 : 0;  // node marks of the plane, a byte each
+    static constexpr int ROWW = XW * WPN;                    // words of one row (one or two x-blocks)
+    static constexpr int SIDEC = NARROW ? 0 : 2 * (TY + 2);  // columns beside the tile, corners included
+    static constexpr int MARKW = SPECIAL ? TY * XW / 4 : 0;  // node marks of the plane, a byte each
     static constexpr int STAGEW = (TY + 2) * ROWW + SIDEC * WPN + MARKW;  // words of one plane stage
     // Stages, and class sums parked in shared memory between planes (all nine class sums and the c_z = +1
     // class do not fit the owners' 104 registers).  Shared memory and L1 share 256 KB, and the owners'
     // remaining spills need L1: FP32 256^3 takes 240 us with 3 stages and 3 parked sums (164 KB, 92 KB of L1),
     // 254 us with 6 parked, 285 us with 4 stages (28 KB of L1: 336 us); all with stores through L1, 232 us now.
-    static constexpr int D = TY == 16 ? (WPN == 10 ? 3 : (WPN == 7 ? 4 : 5)) : (WPN == 10 ? 4 : (WPN == 7 ? 5 : 6));
-    static constexpr int PARK = TY != 16 ? 0 : (WPN == 10 ? 3 : 6);
-    static constexpr int HALO = 9;                           // floats per row and side: c_y x c_z
-    static constexpr int NH = TY / 4;                        // halo warps
-    static constexpr int NTH = 32 * (TY + NH);
+    static constexpr int D = OW == 16 ? (WPN == 10 ? 3 : (WPN == 7 ? 4 : 5)) : (WPN == 10 ? 4 : (WPN == 7 ? 5 : 6));
+    static constexpr int PARK = OW != 16 ? 0 : (WPN == 10 ? 3 : 6);
+    static constexpr int HALO = NARROW ? 0 : 9;              // floats per row and side: c_y x c_z
+    static constexpr int NH = OW / 4;                        // halo warps
+    static constexpr int NTH = 32 * (OW + NH);
     // 20 warps share 16,384 registers per scheduler: 96 each at launch (640 x 96 = 61,440), then 104 for the
     // four warpgroups of owners and 64 for the halo warps (512 x 104 + 128 x 64 = 61,440)
-    static constexpr bool SPLIT = TY == 16;
+    static constexpr bool SPLIT = OW == 16;
     static constexpr int MINB = TY == 4 ? 3 : (TY == 8 ? 2 : 1);  // resident CTAs per SM targeted
-    static constexpr int SMEM = D * (STAGEW * 4 + 2 * TY * HALO * 4 + 3 * 8 + 16) + PARK * 32 * TY * 8;
-    static_assert(2 * TY <= 32, "one halo lane per row and side");
+    static constexpr int SMEM = D * (STAGEW * 4 + 2 * TY * HALO * 4 + 3 * 8 + 16) + PARK * 32 * OW * 8;
+    static_assert(NARROW || 2 * TY <= 32, "one halo lane per row and side");
     static_assert(STAGEW % 4 == 0 && ROWW % 4 == 0 && (SIDEC * WPN) % 4 == 0 && (2 * TY * HALO) % 4 == 0 && MARKW % 4 == 0,
                   "bulk copies and 16-byte accesses on 16-byte boundaries");
 };
@@ -320,6 +327,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
     step_kernel(const __grid_constant__ StepArgs single, const BatchArgs *__restrict__ ba, const int parity,
                 double *__restrict__ diag_part) {
     using G = Geo<S, TY, SPECIAL>;
+    constexpr bool TAKEOVER = SPECIAL || BATCH;
     extern __shared__ __align__(128) unsigned char smem[];
     uint32_t *const stages = reinterpret_cast<uint32_t *>(smem);
     float *const halos = reinterpret_cast<float *>(smem + G::D * G::STAGEW * 4);
@@ -328,7 +336,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
     uint64_t *const full = reinterpret_cast<uint64_t *>(heads + G::D);
     uint64_t *const empty = full + G::D;
     uint64_t *const landed = empty + G::D;
-    V2 *const park = reinterpret_cast<V2 *>(landed + G::D) + threadIdx.x;  // owners: the thread's slots, 32 TY apart
+    V2 *const park = reinterpret_cast<V2 *>(landed + G::D) + threadIdx.x;  // owners: the thread's slots, 32 OW apart
     __shared__ __align__(16) uint4 s_slot[2];  // answers to takeover requests, by item parity
     __shared__ uint64_t s_taken;
     __shared__ int s_next[2];
@@ -338,7 +346,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
     if (threadIdx.x == 0) {
         for (int s = 0; s < G::D; ++s) {
             mbar_init(full + s, 1);
-            mbar_init(empty + s, TY);
+            mbar_init(empty + s, G::OW);
             mbar_init(landed + s, 1);
         }
         mbar_init(&s_taken, 1);
@@ -364,11 +372,11 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
             atomicOr_system(single.error, kErrorWait);
     };
 
-    if (warp >= TY) {
+    if (warp >= G::OW) {
         if constexpr (G::SPLIT) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
         // ---- halo warps ------------------------------------------------------------------------
         bool ok = true;
-        const int hw = warp - TY;
+        const int hw = warp - G::OW;
         int q = 0;        // planes so far, over all items: plane q is halo warp q % NH's
         int n = 0;        // items so far
         auto take_turn = [&]() {
@@ -378,10 +386,10 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
             ok = (G::NH == 1 || *failed == 0) && mbar_wait(empty + stage, phase ^ 1u, limit);
             if (!ok && lane == 0 && *failed == 0) *failed = q + 1;
         };
-        // Work items.  SPECIAL: one CTA per item is launched, and a CTA that finishes its item takes over
+        // Work items.  TAKEOVER: one CTA per item is launched, and a CTA that finishes its item takes over
         // one that has not started (tiles with boundary nodes and the cases of a batch cost unevenly).
         // Otherwise the CTAs stride through the items.
-        const bool leader = threadIdx.x == 32 * TY;
+        const bool leader = threadIdx.x == 32 * G::OW;
         for (int it = blockIdx.x; it >= 0 && it < n_items;) {
             int2 head;
             if constexpr (BATCH) head = ba->items[it];
@@ -393,15 +401,16 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
             const RebuildK K = rebuild_k<S>(a.rho0, a.sc);
             const int tile = head.y & 0xFFFFF, seg = head.y >> 20;
             const int tix = tile % a.tiles_x, tiy = tile / a.tiles_x;
-            const int x0 = tix * TILE_X, y0 = tiy * TY;
-            const int w = min(TILE_X, nx - x0), h = min(TY, ny - y0);
+            const int x0 = tix * G::XW, y0 = tiy * TY;
+            const int w = min(G::XW, nx - x0), h = min(TY, ny - y0);
             const int zs = seg * a.lz, ze = min(zs + a.lz, nz), last = ze - zs + 1;
             const int64_t zst = (int64_t)ny * nxb * G::WPN * kXBlock;
             auto wrap = [](int v, int n) { return v < 0 ? v + n : (v >= n ? v - n : v); };
-            // rows of the bulk copies: lane r copies row y0 - 1 + r
+            // rows of the bulk copies: lane r copies row y0 - 1 + r (and row y0 + 31 + r)
             const uint32_t row_bytes = (uint32_t)min(2, nxb - 2 * tix) * G::WPN * kXBlock * 4;
-            const bool copies = lane < h + 2;
-            const int64_t copy_off = copies ? row_word<S>(2 * tix, wrap(y0 - 1 + lane, ny), 0, nxb, ny) : 0;
+            auto copies = [&](int r) { return r < h + 2; };
+            auto row_off = [&](int r) { return copies(r) ? row_word<S>(2 * tix, wrap(y0 - 1 + r, ny), 0, nxb, ny) : (int64_t)0; };
+            const int64_t copy_off = row_off(lane), copy_off2 = G::NARROW ? row_off(lane + 32) : 0;
             // node marks of the planes that this segment updates (row by row)
             const uint32_t mark_pitch = (uint32_t)a.tiles_x * TILE_X;
             const uint8_t *marks = SPECIAL && lane < h && a.tile_slot && a.tile_slot[tile] >= 0
@@ -413,6 +422,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
             // x0 - 1 (side 0, entering with c_x = +1) or x0 + w (side 1), rows -1 .. h; lane c fetches
             // column c, and the columns past the 32nd are spread over the lanes
             auto side_column = [&](int c) {
+                if (G::NARROW) return (int64_t)-1;
                 const int sd = c / (TY + 2), r = c - sd * (TY + 2) - 1;
                 if (sd > 1 || r > h) return (int64_t)-1;
                 const int gx = wrap(sd ? x0 + w : x0 - 1, nx);
@@ -423,17 +433,17 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
             constexpr int NE = EXTRA ? EXTRA : 1, PER = 32 / NE;  // words of such a column fetched per round
             const int64_t ext_off = EXTRA ? side_column(32 + lane % NE) : -1;
             const int side = lane / TY, row = lane - side * TY;  // the column this lane evaluates
-            const bool active = side < 2 && row < h;
+            const bool active = !G::NARROW && side < 2 && row < h;
             const int mine = (hw + G::NH - q % G::NH) % G::NH;  // this warp's first plane of the item
             int zk = (zs == 0 ? nz - 1 : zs - 1) + mine;
             if (zk >= nz) zk -= nz;
             // The next item is asked for as the last planes of this one are issued: the answer is there before
             // their stages are free, and an item whose CTA is only late (the node-list kernel's blocks are in
             // its place) is not put behind this one's whole length (an annulus of 132 items: 321 -> 265 us a step).
-            if (SPECIAL && leader && mine > last) takeover_request(s_slot + (n & 1), &s_taken);
+            if (TAKEOVER && leader && mine > last) takeover_request(s_slot + (n & 1), &s_taken);
             for (int k = 0; k <= last; ++k, ++q, next_stage()) {
                 if ((k - mine) % G::NH != 0) continue;
-                if (SPECIAL && leader && k + G::NH > last) takeover_request(s_slot + (n & 1), &s_taken);
+                if (TAKEOVER && leader && k + G::NH > last) takeover_request(s_slot + (n & 1), &s_taken);
                 // The halo warps wait for a free stage in turn, each asleep at a hardware barrier until the one
                 // before it has passed (polling costs issue slots).  Plane q waits for the release of plane
                 // q - D; the turn before has seen that of q - 1 - D, so the release two uses back on the stage
@@ -446,57 +456,63 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
                 uint32_t *const cp = sp + (TY + 2) * G::ROWW;  // [word][column]
                 if (lane == 0) {
                     if (k == 0) heads[stage] = make_int4(head.x, head.y, it, 0);
-                    mbar_expect_tx(landed + stage, row_bytes * (h + 2) + (marked(k) ? TILE_X * (uint32_t)h : 0u));
+                    mbar_expect_tx(landed + stage, row_bytes * (h + 2) + (marked(k) ? G::XW * (uint32_t)h : 0u));
                     mbar_arrive(landed + stage);
                 }
                 __syncwarp();
                 const uint32_t *const zsrc = src + zk * zst;
-                if (copies) bulk_load(sp + lane * G::ROWW, zsrc + copy_off, row_bytes, landed + stage);
+                if (copies(lane)) bulk_load(sp + lane * G::ROWW, zsrc + copy_off, row_bytes, landed + stage);
+                if (G::NARROW && copies(lane + 32))
+                    bulk_load(sp + (lane + 32) * G::ROWW, zsrc + copy_off2, row_bytes, landed + stage);
                 if (marked(k) && lane < h)
-                    bulk_load(cp + G::SIDEC * G::WPN + lane * (TILE_X / 4), marks + (int64_t)(k - 1) * ny * mark_pitch, TILE_X,
+                    bulk_load(cp + G::SIDEC * G::WPN + lane * (G::XW / 4), marks + (int64_t)(k - 1) * ny * mark_pitch, G::XW,
                               landed + stage);
-                // (not through L1: a line per word would push out what the owners spill)
-                uint32_t w0[G::WPN], w1[(G::WPN + PER - 1) / PER];
-                if (col_off >= 0) {
+                if constexpr (!G::NARROW) {
+                    // (not through L1: a line per word would push out what the owners spill)
+                    uint32_t w0[G::WPN], w1[(G::WPN + PER - 1) / PER];
+                    if (col_off >= 0) {
 #pragma unroll
-                    for (int f = 0; f < G::WPN; ++f) w0[f] = load_uncached(zsrc + col_off + f * kXBlock);
-                }
-                if (EXTRA && ext_off >= 0) {
-#pragma unroll
-                    for (int i = 0; i < (G::WPN + PER - 1) / PER; ++i) {
-                        const int f = i * PER + lane / NE;
-                        if (f < G::WPN) w1[i] = load_uncached(zsrc + ext_off + f * kXBlock);
+                        for (int f = 0; f < G::WPN; ++f) w0[f] = load_uncached(zsrc + col_off + f * kXBlock);
                     }
-                }
-                if (col_off >= 0) {
+                    if (EXTRA && ext_off >= 0) {
 #pragma unroll
-                    for (int f = 0; f < G::WPN; ++f) cp[f * G::SIDEC + lane] = w0[f];
-                }
-                if (EXTRA && ext_off >= 0) {
+                        for (int i = 0; i < (G::WPN + PER - 1) / PER; ++i) {
+                            const int f = i * PER + lane / NE;
+                            if (f < G::WPN) w1[i] = load_uncached(zsrc + ext_off + f * kXBlock);
+                        }
+                    }
+                    if (col_off >= 0) {
 #pragma unroll
-                    for (int i = 0; i < (G::WPN + PER - 1) / PER; ++i) {
-                        const int f = i * PER + lane / NE;
-                        if (f < G::WPN) cp[f * G::SIDEC + 32 + lane % NE] = w1[i];
+                        for (int f = 0; f < G::WPN; ++f) cp[f * G::SIDEC + lane] = w0[f];
+                    }
+                    if (EXTRA && ext_off >= 0) {
+#pragma unroll
+                        for (int i = 0; i < (G::WPN + PER - 1) / PER; ++i) {
+                            const int f = i * PER + lane / NE;
+                            if (f < G::WPN) cp[f * G::SIDEC + 32 + lane % NE] = w1[i];
+                        }
                     }
                 }
                 __syncwarp();
                 zk += G::NH;
                 while (zk >= nz) zk -= nz;
-                if (active) {
-                    float *e = halos + ((stage * 2 + side) * TY + row) * G::HALO;
+                if constexpr (!G::NARROW) {
+                    if (active) {
+                        float *e = halos + ((stage * 2 + side) * TY + row) * G::HALO;
 #pragma unroll
-                    for (int cy = -1; cy <= 1; ++cy) {
-                        float f[27];
-                        rebuild_scaled<S>(side_values<S, G::SIDEC>(cp + side * (TY + 2) + row + 1 - cy), K, f);
+                        for (int cy = -1; cy <= 1; ++cy) {
+                            float f[27];
+                            rebuild_scaled<S>(side_values<S, G::SIDEC>(cp + side * (TY + 2) + row + 1 - cy), K, f);
 #pragma unroll
-                        for (int cz = -1; cz <= 1; ++cz)
-                            e[3 * (cy + 1) + cz + 1] = side ? f[direction(-1, cy, cz)] : f[direction(1, cy, cz)];
+                            for (int cz = -1; cz <= 1; ++cz)
+                                e[3 * (cy + 1) + cz + 1] = side ? f[direction(-1, cy, cz)] : f[direction(1, cy, cz)];
+                        }
                     }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(full + stage);
                 }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(full + stage);
             }
-            if constexpr (SPECIAL) {
+            if constexpr (TAKEOVER) {
                 // one answer for all halo warps (two slots: the next one is written a barrier after the
                 // last read of this one)
                 if (leader) {
@@ -517,7 +533,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
             if (ok && lane == 0) {
                 heads[stage] = make_int4(0, -1, 0, 0);  // end mark: plane q
                 mbar_arrive(landed + stage);
-                mbar_arrive(full + stage);
+                if (!G::NARROW) mbar_arrive(full + stage);
             }
         }
         if (!ok && lane == 0) report();
@@ -526,7 +542,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
         // barrier; all planes before the failed one were issued (or all, and the end mark), and the last D
         // are the stages' last uses, under way or the last that ended, so their parities tell.
         asm volatile("bar.sync 2, %0;" ::"r"(32 * G::NH) : "memory");
-        if (threadIdx.x == 32 * TY) {
+        if (threadIdx.x == 32 * G::OW) {
             const int issued = s_failed ? s_failed - 1 : q + 1;
             for (int p = max(0, issued - G::D); p < issued; ++p) mbar_wait_lane(landed + p % G::D, (uint32_t)(p / G::D) & 1u);
         }
@@ -539,7 +555,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
             // landed before full, here and in every plane: rows past the tile's last one skip the waits on
             // full, and only the landing of a stage (its refill follows the release of its last use) makes
             // the one parity bit of that wait unambiguous
-            ok = mbar_wait(landed + stage, phase, limit) && mbar_wait(full + stage, phase, limit);
+            ok = mbar_wait(landed + stage, phase, limit) && (G::NARROW || mbar_wait(full + stage, phase, limit));
             if (!ok) break;
             const int4 head = heads[stage];
             if (head.y < 0) break;
@@ -548,14 +564,18 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
             const RebuildK K = rebuild_k<S>(a.rho0, a.sc);
             const int tile = head.y & 0xFFFFF, seg = head.y >> 20;
             const int tix = tile % a.tiles_x, tiy = tile / a.tiles_x;
-            const int x0 = tix * TILE_X, y0 = tiy * TY;
-            const int w = min(TILE_X, nx - x0), h = min(TY, ny - y0);
+            const int x0 = tix * G::XW, y0 = tiy * TY;
+            const int w = min(G::XW, nx - x0), h = min(TY, ny - y0);
             const int zs = seg * a.lz, ze = min(zs + a.lz, a.nz), last = ze - zs + 1;
-            const int y = y0 + warp, x = x0 + 2 * lane;
-            const bool own = warp < h && 2 * lane < w;
+            // the lane's row of the tile, and its place in the row
+            const int row = G::NARROW ? 2 * warp + (lane >> 4) : warp, at = G::NARROW ? lane & 15 : lane;
+            const int y = y0 + row, x = x0 + 2 * at;
+            const bool own = row < h && 2 * at < w;
             const int last_lane = (w >> 1) - 1;
+            // (two rows a warp) the lanes of the x-neighbours in a row that wraps
+            const int west = at == 0 ? lane + last_lane : lane - 1, east = at == last_lane ? lane - at : lane + 1;
             const int64_t zst = (int64_t)ny * nxb * G::WPN * kXBlock;
-            const int in_row = (lane >> 4) * (G::WPN * kXBlock) + 2 * (lane & 15);  // the lane's word in a row
+            const int in_row = (G::NARROW ? 0 : (lane >> 4) * (G::WPN * kXBlock)) + 2 * (lane & 15);  // the lane's word in a row
             uint32_t *dst = reinterpret_cast<uint32_t *>(a.m[parity ^ 1]) + row_word<S>(2 * tix, y, zs, nxb, ny) + in_row;
             const float su = kScaled<S> ? a.sc.s[1] : 1.0f, sm = kScaled<S> ? a.sc.s[2] : 1.0f;
             const float iu = kScaled<S> ? a.sc.is[1] : 1.0f, im = kScaled<S> ? a.sc.is[2] : 1.0f;
@@ -594,8 +614,8 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
                 Pair o;
                 V2 rho4;  // 4 rho, as the sums in `o`
                 uint32_t marks_in = 0u;
-                if (warp < h) {
-                    const uint32_t *sp = stages + stage * G::STAGEW + warp * G::ROWW + in_row;
+                if (G::RPW * warp < h) {  // (a tile has whole pairs of rows: ny is a multiple of 8)
+                    const uint32_t *sp = stages + stage * G::STAGEW + row * G::ROWW + in_row;
                     const float *hv = halos + ((stage * 2 + (lane >= 16 || lane == last_lane)) * TY + warp) * G::HALO;
                     // the nine populations of the row y - cy that enter this row, shifted along x;
                     // g[cx + 1][cz + 1]
@@ -603,6 +623,16 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
                         constexpr int cy = decltype(cyc)::value;
                         V2 f[27];
                         rebuild_scaled<S>(load_pair<S>(sp + (1 - cy) * G::ROWW), K, f);
+                        if constexpr (G::NARROW) {
+#pragma unroll
+                            for (int c = 0; c < 3; ++c) {
+                                const V2 fp = f[direction(1, cy, c - 1)], fm = f[direction(-1, cy, c - 1)];
+                                g[2][c] = v2(__shfl_sync(0xffffffffu, hi(fp), west), lo(fp));
+                                g[1][c] = f[direction(0, cy, c - 1)];
+                                g[0][c] = v2(hi(fm), __shfl_sync(0xffffffffu, lo(fm), east));
+                            }
+                            return;
+                        }
                         // the side columns' populations are evaluated meanwhile
                         if (cy == -1 && k > 0) ok = mbar_wait(full + stage, phase, limit);
                         const float e[3] = {hv[3 * (cy + 1)], hv[3 * (cy + 1) + 1], hv[3 * (cy + 1) + 2]};
@@ -642,7 +672,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
                         if (slot >= 0 && own && k >= 1 && k < last)
                             marks_in = *reinterpret_cast<const uint16_t *>(
                                 reinterpret_cast<const uint8_t *>(stages + stage * G::STAGEW + (TY + 2) * G::ROWW + G::SIDEC * G::WPN) +
-                                warp * TILE_X + 2 * lane);
+                                row * G::XW + 2 * at);
                         const bool q0 = marks_in & MARK_SOLID, q1 = marks_in & (MARK_SOLID << 8);
                         if (q0 || q1) {
                             const Stored<V2> q = load_pair<S>(sp + G::ROWW);
@@ -677,7 +707,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
                     {
                         V2 *const v[] = {&uys, &uxs, &pxy, &pyy, &pxx, &u0s, &py, &px, &pr};
 #pragma unroll
-                        for (int i = 0; i < G::PARK; ++i) *v[i] = park[i * 32 * TY];
+                        for (int i = 0; i < G::PARK; ++i) *v[i] = park[i * 32 * G::OW];
                     }
                     rho4 = add(pr, dn.s0);
                     o.ux = add(px, dn.sx);
@@ -702,7 +732,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
                     {
                         V2 *const v[] = {&uys, &uxs, &pxy, &pyy, &pxx, &u0s, &py, &px, &pr};
 #pragma unroll
-                        for (int i = 0; i < G::PARK; ++i) park[i * 32 * TY] = *v[i];
+                        for (int i = 0; i < G::PARK; ++i) park[i * 32 * G::OW] = *v[i];
                     }
                     up = finish(2);
                 } else {
@@ -765,7 +795,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
                     deD += __shfl_down_sync(0xffffffffu, deD, o);
                 }
                 if (lane == 0) {
-                    const int at = (SPECIAL ? head.z : (int)blockIdx.x) * TY + warp;
+                    const int at = (SPECIAL ? head.z : (int)blockIdx.x) * G::OW + warp;
                     if (!SPECIAL && items > 0) {
                         dmD += diag_part[2 * at + 0];
                         deD += diag_part[2 * at + 1];
@@ -821,7 +851,8 @@ cudaError_t configure_t() {
         // allocates less (the owners would wait for registers that never come)
         cudaFuncAttributes at;
         if ((e = cudaFuncGetAttributes(&at, step_kernel<S, TY, SP, BATCH>)) != cudaSuccess) return e;
-        if ((at.numRegs + 7) / 8 * 8 * Geo<S, TY, SP>::NTH < 32 * (TY * 104 + Geo<S, TY, SP>::NH * 64))
+        if ((at.numRegs + 7) / 8 * 8 * Geo<S, TY, SP>::NTH <
+            32 * (Geo<S, TY, SP>::OW * 104 + Geo<S, TY, SP>::NH * 64))
             return cudaErrorLaunchOutOfResources;
     }
     e = cudaFuncSetAttribute(step_kernel<S, TY, SP, BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -861,6 +892,7 @@ auto dispatch(int storage, int tile_y, F f) -> decltype(f(Tag<float>{}, std::int
         switch (tile_y) {
             case 4: return f(tag, std::integral_constant<int, 4>{});
             case 8: return f(tag, std::integral_constant<int, 8>{});
+            case 32: return f(tag, std::integral_constant<int, 32>{});
             default: return f(tag, std::integral_constant<int, 16>{});
         }
     };
@@ -872,7 +904,7 @@ auto dispatch(int storage, int tile_y, F f) -> decltype(f(Tag<float>{}, std::int
     }
 }
 bool known(int storage, int tile_y) {
-    return storage >= MRLBM_STORAGE_F32 && storage <= MRLBM_STORAGE_F16_U32 && (tile_y == 4 || tile_y == 8 || tile_y == 16);
+    return storage >= MRLBM_STORAGE_F32 && storage <= MRLBM_STORAGE_F16_U32 && (tile_y == 4 || tile_y == 8 || tile_y == 16 || tile_y == 32);
 }
 
 }  // namespace
@@ -886,7 +918,7 @@ cudaError_t launch_step(const StepLaunch &l, int storage, int tile_y, bool speci
     });
 }
 
-cudaError_t prepare_step_batch(int storage, int tile_y) {
+cudaError_t prepare_step_batch(int storage, int tile_y, bool /*special*/) {
     if (!known(storage, tile_y)) return cudaErrorInvalidValue;
     return dispatch(storage, tile_y, [&](auto t, auto ty) {
         using S = typename decltype(t)::type;
@@ -894,7 +926,8 @@ cudaError_t prepare_step_batch(int storage, int tile_y) {
     });
 }
 
-cudaError_t launch_step_batch(const BatchArgs *ba, int parity, int storage, int tile_y, int n_items, cudaStream_t s) {
+cudaError_t launch_step_batch(const BatchArgs *ba, int parity, int storage, int tile_y, bool /*special*/, int n_items,
+                              cudaStream_t s) {
     if (!known(storage, tile_y)) return cudaErrorInvalidValue;
     return dispatch(storage, tile_y, [&](auto t, auto ty) {
         using S = typename decltype(t)::type;
@@ -927,7 +960,7 @@ int step_kernel_max_ctas_per_sm(int storage, int tile_y) {
 // planes takes l = 3 instead of 2 (9 us of 40 less a step), an annulus of 256 planes 52 (43: 10 us of 247 more, 24: 16,
 // 64: 15, 32: 19).
 void choose_tiling(int nx, int ny, int nz, int storage, int n_sm, int &ty, int &lz, int active, int list_nodes) {
-    if (ty != 4 && ty != 8 && ty != 16) ty = 16;
+    ty = tile_height(nx, ty);
     if (lz > 0) {
         lz = std::min(nz, lz);
         return;
@@ -1097,7 +1130,7 @@ int noalloc_periodic_step(const NoAllocStep &p, std::string &err) {
     const int tiles_x = (p.nx + TILE_X - 1) / TILE_X, tiles_y = (p.ny + ty - 1) / ty;
     const int n_items = tiles_x * tiles_y * ((p.nz + lz - 1) / lz);
     const int n_ctas = std::min(std::min(n_items, step_kernel_max_ctas_per_sm(MRLBM_STORAGE_F32, ty) * nd.n_sm),
-                                kNoAllocMaxParts / ty);
+                                kNoAllocMaxParts / owner_warps(ty));
 
     StepArgs sa;
     sa.m[0] = const_cast<float *>(p.m_in);
@@ -1125,7 +1158,7 @@ int noalloc_periodic_step(const NoAllocStep &p, std::string &err) {
     if ((e = launch_step(L, MRLBM_STORAGE_F32, ty, false, p.stream)) != cudaSuccess)
         return noalloc_cuda_fail(e, "step launch", err);
     if (p.diag_host) {
-        if ((e = launch_diag_finalize(part, n_ctas * ty, sums, nullptr, p.stream)) != cudaSuccess)
+        if ((e = launch_diag_finalize(part, n_ctas * owner_warps(ty), sums, nullptr, p.stream)) != cudaSuccess)
             return noalloc_cuda_fail(e, "diagnostics launch", err);
         double v[2];
         if ((e = cudaMemcpyAsync(v, sums, sizeof(v), cudaMemcpyDeviceToHost, p.stream)) != cudaSuccess ||
