@@ -98,3 +98,22 @@ def test_narrow_and_wide_cases_in_a_batch(cuda_device):
             if f.size:
                 assert np.all(np.abs(got - f) <= 1e-9 * np.maximum(np.abs(f).max(), 1e-12))
         b.close()
+
+
+@pytest.mark.parametrize("storage,sr", [(0, 0), (1, 1), (2, 0), (3, 1)])
+def test_batch_of_plain_cases(cuda_device, storage, sr):
+    """A batch without boundary nodes runs a kernel that reads no node marks: each case as if stepped alone."""
+    from mrlbm_3d_cuda_gb300 import Batch
+    from mrlbm_3d_cuda_gb300 import native as N
+    descs = [narrow(k, storage) for k in ((72, 24, 12), (32, 40, 8), (136, 136, 20), (8, 8, 4), (64, 16, 32))]
+    for d in descs:
+        d.stochastic_rounding = sr
+    want = [run(d, 5)[0] for d in descs]
+    b = Batch(descs)
+    for c in b.cases:
+        c.init(N.INIT_NOISY_UNIFORM, INIT)
+    b.step(5)
+    b.sync()
+    for c, m in zip(b.cases, want):
+        assert np.array_equal(c.moments(), m)
+    b.close()
