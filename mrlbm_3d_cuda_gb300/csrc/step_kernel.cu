@@ -64,7 +64,8 @@ struct Geo {
     // class do not fit the owners' 104 registers).  Shared memory and L1 share 256 KB, and the owners'
     // remaining spills need L1: FP32 256^3 takes 240 us with 3 stages and 3 parked sums (164 KB, 92 KB of L1),
     // 254 us with 6 parked, 285 us with 4 stages (28 KB of L1: 336 us); all with stores through L1, 232 us now.
-    static constexpr int D = OW == 16 ? (WPN == 10 ? 3 : (WPN == 7 ? 4 : 5)) : (WPN == 10 ? 4 : (WPN == 7 ? 5 : 6));
+    // (FP32 tiles of 8 rows, two CTAs an SM: 410 us with 4 stages each, 327 with 3.)
+    static constexpr int D = OW == 16 ? (WPN == 10 ? 3 : (WPN == 7 ? 4 : 5)) : (WPN == 10 ? (TY == 8 ? 3 : 4) : (WPN == 7 ? 5 : 6));
     static constexpr int PARK = OW != 16 ? 0 : (WPN == 10 ? 3 : 6);
     static constexpr int HALO = NARROW ? 0 : 9;              // floats per row and side: c_y x c_z
     static constexpr int NH = OW / 4;                        // halo warps
