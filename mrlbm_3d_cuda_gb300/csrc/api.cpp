@@ -135,7 +135,7 @@ int sync_sr_step(mrlbm_handle *h) {
     return MRLBM_OK;
 }
 
-// Tile height and z-segment length from MRLBM_TILE_Y / MRLBM_LZ, else 0: choose_tiling's.
+// Tile height and z-segment length from MRLBM_TILE_Y / MRLBM_LZ, else 0: tile_height's and choose_lz's.
 void default_tiling(int &ty, int &lz) {
     const char *ety = std::getenv("MRLBM_TILE_Y");
     const char *elz = std::getenv("MRLBM_LZ");
@@ -234,8 +234,9 @@ int setup_tiling(mrlbm_handle *h, int ty, int lz) {
         return fail(h, MRLBM_ERR_INVALID_ARG, "too many boundary nodes");
     h->n_list = (int)list_xyz.size();
     h->n_list_blocks = special_list_blocks(h->n_list);
-    choose_tiling(d.nx, d.ny, d.nz, h->storage, h->n_sm, ty, lz, tiles - (int)std::count(skip.begin(), skip.end(), 1), h->n_list);
-    h->lz = lz;
+    h->lz = lz > 0 ? std::min(d.nz, lz)
+                   : choose_lz(d.nx, d.ny, d.nz, h->storage, ty, resident,
+                               tiles - (int)std::count(skip.begin(), skip.end(), 1), h->n_list);
     const int nseg = (d.nz + h->lz - 1) / h->lz;
     // work items are int32 `tile | segment << 20` (decoded in step_kernel)
     if (tiles > (1 << 20) || nseg > kMaxSegments)

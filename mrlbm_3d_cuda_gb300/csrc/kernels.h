@@ -150,9 +150,9 @@ cudaError_t launch_special_list_batch(const BatchArgs *ba, int parity, int force
 cudaError_t launch_wall_batch(const BatchArgs *ba, int parity, int force, int storage, int n_blocks, cudaStream_t s);
 // Zero the slot of every case's force ring and publish the slot for the batched wall kernel.
 cudaError_t launch_batch_force_begin(double *const *ring, int n_cases, int slot, int *d_slot, cudaStream_t s);
-// Tile height (tile_height of the one on entry) and z-segment length (> 0 on entry:
-// kept, clipped to nz); active: tiles that are updated (0: all); list_nodes: nodes of the node-list kernel.
-void choose_tiling(int nx, int ny, int nz, int storage, int n_sm, int &ty, int &lz, int active = 0, int list_nodes = 0);
+// z-segment length for tiles of tile_y rows on a device that holds `slots` CTAs; active: tiles that are updated
+// (0: all); list_nodes: nodes of the node-list kernel.
+int choose_lz(int nx, int ny, int nz, int storage, int tile_y, int64_t slots, int active = 0, int list_nodes = 0);
 // z-segment length of a batch's merged items: tiles[c] of nz[c] planes each.
 int choose_batch_lz(const std::vector<int> &tiles, const std::vector<int> &nz, int storage, int n_sm, int ty);
 int step_kernel_max_ctas_per_sm(int storage, int tile_y);

@@ -966,17 +966,13 @@ int step_kernel_max_ctas_per_sm(int storage, int tile_y) {
 // less with fewer words a node, and a block's latency of 5 units at least.  With that term a channel of 32
 // planes takes l = 3 instead of 2 (9 us of 40 less a step), an annulus of 256 planes 52 (43: 10 us of 247 more, 24: 16,
 // 64: 15, 32: 19).
-void choose_tiling(int nx, int ny, int nz, int storage, int n_sm, int &ty, int &lz, int active, int list_nodes) {
-    ty = tile_height(nx, ty);
-    if (lz > 0) {
-        lz = std::min(nz, lz);
-        return;
-    }
-    const int64_t slots = (int64_t)std::max(1, step_kernel_max_ctas_per_sm(storage, ty)) * n_sm;
-    const int64_t tiles = active > 0 ? active : (int64_t)((nx + TILE_X - 1) / TILE_X) * ((ny + ty - 1) / ty);
+int choose_lz(int nx, int ny, int nz, int storage, int tile_y, int64_t slots, int active, int list_nodes) {
+    const int64_t tiles = active > 0 ? active : (int64_t)((nx + TILE_X - 1) / TILE_X) * ((ny + tile_y - 1) / tile_y);
     const double list = (storage == MRLBM_STORAGE_F32 ? 0.03 : (storage == MRLBM_STORAGE_F16_U32 ? 0.024 : 0.02)) * list_nodes;
     double best = 1e300;
-    for (int nseg = 1; nseg <= std::min(nz, kMaxSegments); ++nseg) {
+    int lz = nz;
+    // each segment length once, with the fewest segments that give it
+    for (int nseg = 1; nseg <= std::min(nz, kMaxSegments);) {
         const int l = (nz + nseg - 1) / nseg;
         const int64_t items = tiles * ((nz + l - 1) / l), t = (items + slots - 1) / slots * (2 * l + 7);
         const double rest = list - (double)(slots * t - items * (2 * l + 7));
@@ -985,7 +981,10 @@ void choose_tiling(int nx, int ny, int nz, int storage, int n_sm, int &ty, int &
             best = cost;
             lz = l;
         }
+        if (l == 1) break;
+        nseg = (nz + l - 2) / (l - 1);
     }
+    return lz;
 }
 
 // A batch has many more items than the SMs hold, and a CTA takes the next one as it finishes: the items'
@@ -1028,16 +1027,28 @@ static __managed__ int g_noalloc_error[kNoAllocMaxDevices];
 namespace {
 
 std::mutex g_noalloc_mu;
-// per device, set up on its first call: the scratch array's device address, the error word and the SM count
+// per device, set up on its first call: the scratch array's device address, the error word, and how many CTAs of
+// the plain FP32 step kernel it holds with tiles of 16 and of 32 rows
 struct NoAllocDevice {
     void *scratch = nullptr;
     int *error = nullptr;
-    int n_sm = 0;
+    int slots[2] = {0, 0};
 };
 NoAllocDevice g_noalloc_dev[kNoAllocMaxDevices];
 
+// CTAs of the plain FP32 step kernel that an SM holds (0: a query failed).
+template <int TY>
+int plain_ctas_per_sm() {
+    int n = 0;
+    if (configure_t<float, TY, false, false>() != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, step_kernel<float, TY, false, false>, Geo<float, TY, false>::NTH,
+                                                      Geo<float, TY, false>::SMEM) != cudaSuccess)
+        return 0;
+    return n;
+}
+
 // Set-up of device `dev` (the current device), once: the arrays' addresses (in host code the scratch
-// array's name is only a host-side stand-in) and the SM count.  Host-side queries only; nothing is
+// array's name is only a host-side stand-in) and the CTAs it holds.  Host-side queries only; nothing is
 // allocated.
 cudaError_t noalloc_device(int dev, NoAllocDevice &out) {
     std::lock_guard<std::mutex> lock(g_noalloc_mu);
@@ -1050,7 +1061,11 @@ cudaError_t noalloc_device(int dev, NoAllocDevice &out) {
         if ((e = cudaGetSymbolAddress(&w, g_noalloc_error)) != cudaSuccess) return e;
         int n_sm = 0;
         if ((e = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-        d.n_sm = n_sm;
+        for (int k = 0; k < 2; ++k) {
+            const int per_sm = k ? plain_ctas_per_sm<32>() : plain_ctas_per_sm<16>();
+            if (per_sm <= 0) return cudaErrorLaunchOutOfResources;
+            d.slots[k] = per_sm * n_sm;
+        }
         d.error = (int *)w + dev;
         d.scratch = p;
     }
@@ -1132,12 +1147,11 @@ int noalloc_periodic_step(const NoAllocStep &p, std::string &err) {
     }
     unsigned char *scratch = (unsigned char *)nd.scratch;
 
-    int ty = 0, lz = 0;
-    choose_tiling(p.nx, p.ny, p.nz, MRLBM_STORAGE_F32, nd.n_sm, ty, lz);
+    const int ty = tile_height(p.nx, 0), slots = nd.slots[ty == 32];
+    const int lz = choose_lz(p.nx, p.ny, p.nz, MRLBM_STORAGE_F32, ty, slots);
     const int tiles_x = (p.nx + TILE_X - 1) / TILE_X, tiles_y = (p.ny + ty - 1) / ty;
     const int n_items = tiles_x * tiles_y * ((p.nz + lz - 1) / lz);
-    const int n_ctas = std::min(std::min(n_items, step_kernel_max_ctas_per_sm(MRLBM_STORAGE_F32, ty) * nd.n_sm),
-                                kNoAllocMaxParts / owner_warps(ty));
+    const int n_ctas = std::min(std::min(n_items, slots), kNoAllocMaxParts / owner_warps(ty));
 
     StepArgs sa;
     sa.m[0] = const_cast<float *>(p.m_in);
