@@ -180,10 +180,19 @@ int setup_tiling(mrlbm_handle *h, int ty, int lz) {
     const int resident = per_sm * h->n_sm;
     const int tiles = h->tiles_x * h->tiles_y;
     std::vector<uint32_t> word(h->n, 0);
-    for (int64_t i = 0; i < h->n; ++i) word[i] = make_word(g.cls[i], g.payload[i], g.frozen[i] != 0, g.stencil[i] != 0);
+    // tiles with nodes whose values go through the side buffer (64 bytes for each node of such a tile)
+    std::vector<char> uses(tiles, 0);
+    for (int64_t i = 0; i < h->n;) {
+        char *const row = uses.data() + (size_t)((i / d.nx) % d.ny / h->tile_y) * h->tiles_x;
+        for (int x = 0; x < d.nx; ++x, ++i) {
+            word[i] = make_word(g.cls[i], g.payload[i], g.frozen[i] != 0, g.stencil[i] != 0);
+            if (uses_side(word[i])) row[x / TILE_X] = 1;
+        }
+    }
     std::vector<int32_t> slot(tiles, -1);
     std::vector<char> skip(tiles, 0);
     int n_special = 0;
+    int32_t side_columns = 0;  // in eights
     for (int t = 0; t < tiles; ++t) {
         const int x0 = (t % h->tiles_x) * TILE_X, y0 = (t / h->tiles_x) * h->tile_y;
         bool special = false, all_frozen = true;
@@ -196,7 +205,14 @@ int setup_tiling(mrlbm_handle *h, int ty, int lz) {
                 }
             }
         if (all_frozen) skip[t] = 1;
-        else if (special) slot[t] = n_special++;
+        else if (special) {
+            ++n_special;
+            slot[t] = 0;
+            if (uses[t]) {
+                slot[t] = side_columns;
+                side_columns += std::min(TILE_X, d.nx - x0) / 8;
+            }
+        }
     }
     h->n_special = n_special;
 
@@ -256,8 +272,8 @@ int setup_tiling(mrlbm_handle *h, int ty, int lz) {
 
     if (h->d_mark) {
         CK(h, upload(&h->d_tile_slot, slot.data(), slot.size()));
-        if (n_special > 0) {
-            const size_t side_floats = (size_t)n_special * d.nz * TILE_X * h->tile_y * 16;
+        if (side_columns > 0) {
+            const size_t side_floats = (size_t)side_columns * 8 * d.nz * h->tile_y * 16;
             CK(h, cudaMalloc((void **)&h->d_side, side_floats * sizeof(float)));
             CK(h, cudaMemset(h->d_side, 0, side_floats * sizeof(float)));
         }

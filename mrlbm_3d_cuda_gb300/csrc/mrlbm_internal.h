@@ -50,6 +50,13 @@ inline uint8_t node_mark(uint32_t word) {
     return MARK_OTHER;
 }
 
+// Whether a node's values go through the side buffer: snapshots of wall-stencil and wall nodes, and the force
+// terms of BCFLUID nodes.
+inline bool uses_side(uint32_t word) {
+    const uint32_t cls = word & NW_CLASS_MASK;
+    return (word & NW_STENCIL) || (cls >= C_INNER && cls <= C_BCFLUID_OUTER);
+}
+
 // Step-kernel tiling: a CTA owns a TILE_X x tile_y column of nodes (two x-blocks wide) and marches
 // along z.
 constexpr int TILE_X = 64;
