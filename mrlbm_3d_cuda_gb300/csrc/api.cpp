@@ -179,21 +179,30 @@ int setup_tiling(mrlbm_handle *h, int ty, int lz) {
     if (per_sm <= 0) per_sm = 1;
     const int resident = per_sm * h->n_sm;
     const int tiles = h->tiles_x * h->tiles_y;
-    std::vector<uint32_t> word(h->n, 0);
+    // node words; none, and no tile with boundary nodes, where all nodes are plain
+    std::vector<uint32_t> word(h->d_mark ? h->n : 0);
     // tiles with nodes whose values go through the side buffer (64 bytes for each node of such a tile)
     std::vector<char> uses(tiles, 0);
-    for (int64_t i = 0; i < h->n;) {
-        char *const row = uses.data() + (size_t)((i / d.nx) % d.ny / h->tile_y) * h->tiles_x;
-        for (int x = 0; x < d.nx; ++x, ++i) {
-            word[i] = make_word(g.cls[i], g.payload[i], g.frozen[i] != 0, g.stencil[i] != 0);
-            if (uses_side(word[i])) row[x / TILE_X] = 1;
+    if (!word.empty()) {
+        const auto *cls = g.cls.data();
+        const auto *payload = g.payload.data();
+        const auto *frozen = g.frozen.data();
+        const auto *stencil = g.stencil.data();
+        uint32_t *wd = word.data();
+        for (int64_t i = 0, r = 0; r < (int64_t)d.ny * d.nz; ++r) {
+            char *const row = uses.data() + (size_t)(r % d.ny / h->tile_y) * h->tiles_x;
+            for (int x = 0; x < d.nx; ++x, ++i) {
+                const uint32_t v = make_word(cls[i], payload[i], frozen[i] != 0, stencil[i] != 0);
+                wd[i] = v;
+                if (uses_side(v)) row[x / TILE_X] = 1;
+            }
         }
     }
     std::vector<int32_t> slot(tiles, -1);
     std::vector<char> skip(tiles, 0);
     int n_special = 0;
     int32_t side_columns = 0;  // in eights
-    for (int t = 0; t < tiles; ++t) {
+    for (int t = 0; t < (h->d_mark ? tiles : 0); ++t) {
         const int x0 = (t % h->tiles_x) * TILE_X, y0 = (t / h->tiles_x) * h->tile_y;
         bool special = false, all_frozen = true;
         for (int z = 0; z < d.nz && !(special && !all_frozen); ++z)
@@ -216,7 +225,7 @@ int setup_tiling(mrlbm_handle *h, int ty, int lz) {
     }
     h->n_special = n_special;
 
-    // Non-bulk nodes of special tiles, by slot, kind of closure, z, tile row, x: the lanes of a warp of the
+    // Non-bulk nodes of special tiles, by tile, kind of closure, z, tile row, x: the lanes of a warp of the
     // node-list kernel then mostly run one closure.  Solid nodes of updated blocks need no populations:
     // the step kernel collides them in place; frozen nodes are never updated.  Neither is in the list.
     auto kind = [](uint32_t cls) {
@@ -631,15 +640,26 @@ int mrlbm_create(const mrlbm_case_desc *din, mrlbm_handle **out) {
         h->sc.is[k] = 1.0f / s;
     }
 
-    // node words (tile independent)
-    std::vector<uint32_t> word(h->n, 0);
+    // node marks (the step kernel's rows of whole tiles); plain pointers: the byte stores could alias anything else
+    const size_t pitch = (size_t)(d.nx + TILE_X - 1) / TILE_X * TILE_X, rows = (size_t)d.ny * d.nz;
+    std::vector<uint8_t> mark(d.geometry == MRLBM_GEOM_NONE && d.periodic[0] && d.periodic[1] && d.periodic[2] ? 0 : pitch * rows);
     bool any_special = false;
     int64_t n_fluid = 0;
-    for (int64_t i = 0; i < h->n; ++i) {
-        word[i] = make_word(g.cls[i], g.payload[i], g.frozen[i] != 0, g.stencil[i] != 0);
-        if (word[i]) any_special = true;
-        const uint32_t c = g.cls[i];
-        if (!g.frozen[i] && c != C_SOLID && c != C_INNER && c != C_OUTER) ++n_fluid;
+    {
+        const auto *cls = g.cls.data();
+        const auto *payload = g.payload.data();
+        const auto *frozen = g.frozen.data();
+        const auto *stencil = g.stencil.data();
+        uint8_t *m = mark.empty() ? nullptr : mark.data();
+        for (size_t r = 0, i = 0; r < rows; ++r) {
+            for (int x = 0; x < d.nx; ++x, ++i) {
+                const uint32_t c = cls[i], wd = make_word(c, payload[i], frozen[i] != 0, stencil[i] != 0);
+                n_fluid += !frozen[i] && c != C_SOLID && c != C_INNER && c != C_OUTER;
+                any_special |= wd != 0u;
+                if (m) m[x] = node_mark(wd);
+            }
+            if (m) m += pitch;
+        }
     }
     h->n_fluid = n_fluid;
 
@@ -649,13 +669,7 @@ int mrlbm_create(const mrlbm_case_desc *din, mrlbm_handle **out) {
     CK(H, cudaMalloc(&h->m[1], mbytes));
     CK(H, cudaMemset(h->m[0], 0, mbytes));
     CK(H, cudaMemset(h->m[1], 0, mbytes));
-    if (any_special) {
-        const size_t pitch = (size_t)(d.nx + TILE_X - 1) / TILE_X * TILE_X, rows = (size_t)d.ny * d.nz;
-        std::vector<uint8_t> mark(pitch * rows, 0);
-        for (size_t r = 0; r < rows; ++r)
-            for (int x = 0; x < d.nx; ++x) mark[r * pitch + x] = node_mark(word[r * d.nx + x]);
-        CK(H, upload(&h->d_mark, mark.data(), mark.size()));
-    }
+    if (any_special) CK(H, upload(&h->d_mark, mark.data(), mark.size()));
     for (int w = 0; w < g.n_walls; ++w) {
         const WallData &wd = g.wall[w];
         CK(H, upload(&h->d_wf[w][0], wd.nx.data(), wd.nx.size()));
