@@ -99,46 +99,6 @@ __device__ __forceinline__ void reconstruct_h(const Mom &m, float h3, float h15,
 
 __device__ __forceinline__ void reconstruct(const Mom &m, float f[27]) { reconstruct_h(m, 3.0f, 1.5f, 4.5f, 9.0f, f); }
 
-// rho = sum f, u = sum c f / rho, m_ab = sum c_a c_b f / rho - cs2 delta_ab, via the 13
-// opposite-pair sums e and differences d.
-__device__ __forceinline__ void evaluate(const float f[27], Mom &m) {
-    const float e1 = f[1] + f[2], d1 = f[1] - f[2];
-    const float e3 = f[3] + f[4], d3 = f[3] - f[4];
-    const float e5 = f[5] + f[6], d5 = f[5] - f[6];
-    const float e7 = f[7] + f[8], d7 = f[7] - f[8];
-    const float e9 = f[9] + f[10], d9 = f[9] - f[10];
-    const float e11 = f[11] + f[12], d11 = f[11] - f[12];
-    const float e13 = f[13] + f[14], d13 = f[13] - f[14];
-    const float e15 = f[15] + f[16], d15 = f[15] - f[16];
-    const float e17 = f[17] + f[18], d17 = f[17] - f[18];
-    const float e19 = f[19] + f[20], d19 = f[19] - f[20];
-    const float e21 = f[21] + f[22], d21 = f[21] - f[22];
-    const float e23 = f[23] + f[24], d23 = f[23] - f[24];
-    const float e25 = f[25] + f[26], d25 = f[25] - f[26];
-    const float ec = (e19 + e21) + (e23 + e25);
-    const float sxx = (e1 + e7) + (e9 + e13) + e15 + ec;
-    const float syy = (e3 + e7) + (e11 + e13) + e17 + ec;
-    const float szz = (e5 + e9) + (e11 + e15) + e17 + ec;
-    const float rho = f[0] + ((e1 + e3) + e5) + ((e7 + e9) + (e11 + e13)) + ((e15 + e17) + ec);
-    const float jx = (d1 + d7) + (d9 + d13) + (d15 + d19) + (d21 + d23) - d25;
-    const float jy = (d3 + d7) + (d11 - d13) + (d17 + d19) + (d21 - d23) + d25;
-    const float jz = (d5 + d9) + (d11 - d15) - (d17 - d19) + (d23 - d21) + d25;
-    const float sxy = (e7 - e13) + ((e19 + e21) - (e23 + e25));
-    const float sxz = (e9 - e15) + ((e19 - e21) + (e23 - e25));
-    const float syz = (e11 - e17) + ((e19 - e21) - (e23 - e25));
-    const float inv = __frcp_rn(rho);  // correctly rounded, as 1.0f / rho
-    m.rho = rho;
-    m.ux = jx * inv;
-    m.uy = jy * inv;
-    m.uz = jz * inv;
-    m.mxx = sxx * inv - kCs2;
-    m.myy = syy * inv - kCs2;
-    m.mzz = szz * inv - kCs2;
-    m.mxy = sxy * inv;
-    m.mxz = sxz * inv;
-    m.myz = syz * inv;
-}
-
 // m_ab <- (1 - omega) m_ab + omega u_a u_b; rho and u are collision invariants.  The rounding order is spelled out with
 // intrinsics: `a*b + c*d` has two possible FMA contractions, and leaving the choice to the
 // compiler let different kernel instantiations (tile heights) round differently.

@@ -175,48 +175,42 @@ __device__ __forceinline__ int special_node(const StepArgs &a, int parity, bool 
     const S *__restrict__ src = (const S *)a.m[parity];
     bool wall_node = false;
     bool fluid = true;
-    if (cls == C_BULK) {
-        evaluate(fl, m);
+    const Mom prev = load_mom<S>(src, aos_at<S>(x, y, z, a.nxb, a.ny), a.rho0, a.sc);
+    m = prev;  // nodes without a closure keep their pre-stream moments
+    if (cls == C_INNER || cls == C_OUTER) {
+        const int wi = cls == C_INNER ? 0 : 1;
+        const uint32_t bi = w >> NW_PAYLOAD_SHIFT;
+        incoming_rotated(a.wall[wi].nx[bi], a.wall[wi].ny[bi], a.wall[wi].in_mask[bi], fl, m);
+        wall_node = true;
+        fluid = false;
+    } else if (cls == C_BCFLUID_INNER || cls == C_BCFLUID_OUTER) {
+        const uint32_t tag = (w >> NW_PAYLOAD_SHIFT) & 0xFFu;
+        Mom o = prev;
+        if (bcfluid_closure(tag, a.tag_in[tag], fl, a.bcf_strong, a.omega, o)) m = o;
+    } else if (cls == C_BCSOLID_INNER || cls == C_BCSOLID_OUTER) {
+        const uint32_t tag = (w >> NW_PAYLOAD_SHIFT) & 0xFFu;
+        Mom o = prev;
+        if (bcsolid_closure(tag, fl, a.omega, o)) m = o;
     } else {
-        const Mom prev = load_mom<S>(src, aos_at<S>(x, y, z, a.nxb, a.ny), a.rho0, a.sc);
-        m = prev;  // nodes without a closure keep their pre-stream moments
-        if (cls == C_SOLID) {
-            fluid = false;
-        } else if (cls == C_INNER || cls == C_OUTER) {
-            const int wi = cls == C_INNER ? 0 : 1;
-            const uint32_t bi = w >> NW_PAYLOAD_SHIFT;
-            incoming_rotated(a.wall[wi].nx[bi], a.wall[wi].ny[bi], a.wall[wi].in_mask[bi], fl, m);
-            wall_node = true;
-            fluid = false;
-        } else if (cls == C_BCFLUID_INNER || cls == C_BCFLUID_OUTER) {
-            const uint32_t tag = (w >> NW_PAYLOAD_SHIFT) & 0xFFu;
-            Mom o = prev;
-            if (bcfluid_closure(tag, a.tag_in[tag], fl, a.bcf_strong, a.omega, o)) m = o;
-        } else if (cls == C_BCSOLID_INNER || cls == C_BCSOLID_OUTER) {
-            const uint32_t tag = (w >> NW_PAYLOAD_SHIFT) & 0xFFu;
-            Mom o = prev;
-            if (bcsolid_closure(tag, fl, a.omega, o)) m = o;
-        } else {
-            PlanarCtx c;
-            c.omega = a.omega;
-            c.u_max = a.u_max;
-            c.rho0 = a.rho0;
-            c.convective = a.convective;
-            c.self_prev = prev;
-            c.west_prev = prev;
-            if (class_walls(cls) & 2u) {
-                if (a.current_update) {
-                    // NEUMANN_CURRENT_UPDATE (boundaries.cuh:96-161): post-stream rho, u of the
-                    // x-1 neighbour and of the node itself instead of their stored moments
-                    c.west_prev = pulled_rho_u<S>(a, src, x - 1, y, z);
-                    c.self_prev = rho_u_of(fl);
-                } else {
-                    c.west_prev = load_mom<S>(src, aos_at<S>(x - 1, y, z, a.nxb, a.ny), a.rho0, a.sc);
-                }
+        PlanarCtx c;
+        c.omega = a.omega;
+        c.u_max = a.u_max;
+        c.rho0 = a.rho0;
+        c.convective = a.convective;
+        c.self_prev = prev;
+        c.west_prev = prev;
+        if (class_walls(cls) & 2u) {
+            if (a.current_update) {
+                // NEUMANN_CURRENT_UPDATE (boundaries.cuh:96-161): post-stream rho, u of the
+                // x-1 neighbour and of the node itself instead of their stored moments
+                c.west_prev = pulled_rho_u<S>(a, src, x - 1, y, z);
+                c.self_prev = rho_u_of(fl);
+            } else {
+                c.west_prev = load_mom<S>(src, aos_at<S>(x - 1, y, z, a.nxb, a.ny), a.rho0, a.sc);
             }
-            Mom o = prev;
-            if (planar_closure(cls, fl, c, o)) m = o;
         }
+        Mom o = prev;
+        if (planar_closure(cls, fl, c, o)) m = o;
     }
     if ((w & NW_STENCIL) && slot >= 0) {
         float *e = a.side + side_index(slot, x, y, z, x0, y0, min(TILE_X, a.nx - x0), a.nz, a.tile_y) * 16;
@@ -238,9 +232,9 @@ __device__ __forceinline__ int special_node(const StepArgs &a, int parity, bool 
     return fluid ? 2 : 1;
 }
 
-// A warp takes kListNodes nodes at a time: rounds of ten nodes x three lanes gather the populations into
-// shared memory, then one lane per node applies its closure.  With 30 nodes a warp the closure fills its
-// lanes, but fewer warps hide the loads: annulus 77 us instead of 72, a cylinder's 17 k nodes 18 instead of 15.
+// A warp takes ten nodes at a time: three lanes of each gather its populations into shared memory, then one lane
+// per node applies its closure.  With three such rounds a warp the closure fills its lanes, but fewer warps hide
+// the loads: annulus 77 us instead of 72, a cylinder's 17 k nodes 18 instead of 15.
 constexpr int kListWarps = 4, kListThreads = 32 * kListWarps, kListNodes = 10;
 
 // BATCH: each block serves the case named by its entry in BatchArgs::list_blocks.
@@ -264,14 +258,10 @@ __global__ void __launch_bounds__(kListThreads)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double dm = 0.0, de = 0.0;
     for (int first = (b0 * kListWarps + warp) * kListNodes; first < n_all; first += nblk * kListWarps * kListNodes) {
-#pragma unroll 1
-        for (int r = 0; r < kListNodes / 10; ++r) {
-            const int j = 10 * r + lane / 3, i = first + j;
-            if (lane < 30 && i < n_all) {
-                const uint64_t p = a.list_xyz[i];
-                pull<S>(a, (const S *)a.m[parity], needed(a, a.list_word[i]), lane % 3 - 1, (int)(p & 0x1FFFFFu),
-                        (int)((p >> 21) & 0x1FFFFFu), (int)(p >> 42), &gathered[warp][0][j], kListNodes + 1);
-            }
+        if (const int j = lane / 3; lane < 3 * kListNodes && first + j < n_all) {
+            const uint64_t p = a.list_xyz[first + j];
+            pull<S>(a, (const S *)a.m[parity], needed(a, a.list_word[first + j]), lane % 3 - 1, (int)(p & 0x1FFFFFu),
+                    (int)((p >> 21) & 0x1FFFFFu), (int)(p >> 42), &gathered[warp][0][j], kListNodes + 1);
         }
         __syncwarp();
         const int i = first + lane;
