@@ -201,7 +201,7 @@ int setup_tiling(mrlbm_handle *h, int ty, int lz) {
     std::vector<int32_t> slot(tiles, -1);
     std::vector<char> skip(tiles, 0);
     int n_special = 0;
-    int32_t side_columns = 0;  // in eights
+    int32_t side_slots = 0, shared = 0;  // slots of TILE_X columns; next free column of the one that narrower tiles share
     for (int t = 0; t < (h->d_mark ? tiles : 0); ++t) {
         const int x0 = (t % h->tiles_x) * TILE_X, y0 = (t / h->tiles_x) * h->tile_y;
         bool special = false, all_frozen = true;
@@ -218,8 +218,14 @@ int setup_tiling(mrlbm_handle *h, int ty, int lz) {
             ++n_special;
             slot[t] = 0;
             if (uses[t]) {
-                slot[t] = side_columns;
-                side_columns += std::min(TILE_X, d.nx - x0) / 8;
+                const int w = std::min(TILE_X, d.nx - x0);
+                if (w == TILE_X || shared % TILE_X == 0 || shared % TILE_X + w > TILE_X) {
+                    slot[t] = TILE_X * side_slots++;
+                    if (w < TILE_X) shared = slot[t] + w;
+                } else {
+                    slot[t] = shared;
+                    shared += w;
+                }
             }
         }
     }
@@ -281,8 +287,8 @@ int setup_tiling(mrlbm_handle *h, int ty, int lz) {
 
     if (h->d_mark) {
         CK(h, upload(&h->d_tile_slot, slot.data(), slot.size()));
-        if (side_columns > 0) {
-            const size_t side_floats = (size_t)side_columns * 8 * d.nz * h->tile_y * 16;
+        if (side_slots > 0) {
+            const size_t side_floats = (size_t)side_slots * TILE_X * d.nz * h->tile_y * 16;
             CK(h, cudaMalloc((void **)&h->d_side, side_floats * sizeof(float)));
             CK(h, cudaMemset(h->d_side, 0, side_floats * sizeof(float)));
         }

@@ -80,7 +80,7 @@ struct StepArgs {
     const uint8_t *mark = nullptr;      // node marks, rows of tiles_x * TILE_X bytes; null if all bulk
     const int32_t *items = nullptr;     // work items: tile index | (z-segment << 20); null: all, segment by segment
     int n_items = 0;
-    const int32_t *tile_slot = nullptr; // per xy tile: -1 plain, >= 0 marked nodes; its place in the side buffer (side_index)
+    const int32_t *tile_slot = nullptr; // per xy tile: -1 plain, >= 0 marked nodes; its first column in the side buffer
     float *side = nullptr;              // post-stream moments of stencil nodes, 10 floats each
     int nx = 0, ny = 0, nz = 0;
     int tiles_x = 0, tiles_y = 0, tile_y = 8, lz = 32;
@@ -126,10 +126,11 @@ struct StepLaunch {
     cudaEvent_t placed = nullptr;  // recorded when the last CTA of the step kernel has started, or null
 };
 
-// Side-buffer index of node (x, y, z) of the tile at (x0, y0), `w` nodes wide.  A tile takes w columns of tile_y x nz
-// nodes; places are counted in 8 such columns (every width is a multiple of 8).
-inline __host__ __device__ int64_t side_index(int slot, int x, int y, int z, int x0, int y0, int w, int nz, int tile_y) {
-    return (int64_t)slot * 8 * nz * tile_y + ((int64_t)z * tile_y + (y - y0)) * w + (x - x0);
+// Side-buffer index of node (x, y, z) of the tile at (x0, y0) whose first column is `first`.  Slots of tile_x columns (tile_y x
+// nz nodes each, a power of two of them) are shared by tiles that are narrower.
+inline __host__ __device__ int64_t side_index(int first, int x, int y, int z, int x0, int y0, int nz, int tile_x,
+                                              int tile_y) {
+    return (((int64_t)(first / tile_x) * nz + z) * tile_y + (y - y0)) * tile_x + (x - (x0 - first % tile_x));
 }
 
 // Tile height: 4, 8 or 16 (the default) rows of TILE_X nodes; grids of at most one x-block take 32 rows of it in

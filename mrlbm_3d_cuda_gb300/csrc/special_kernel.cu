@@ -213,7 +213,7 @@ __device__ __forceinline__ int special_node(const StepArgs &a, int parity, bool 
         if (planar_closure(cls, fl, c, o)) m = o;
     }
     if ((w & NW_STENCIL) && slot >= 0) {
-        float *e = a.side + side_index(slot, x, y, z, x0, y0, min(TILE_X, a.nx - x0), a.nz, a.tile_y) * 16;
+        float *e = a.side + side_index(slot, x, y, z, x0, y0, a.nz, TILE_X, a.tile_y) * 16;
         store_side(e, m.rho - a.rho0, m.ux, m.uy, m.uz, m.mxx, m.myy, m.mzz, m.mxy, m.mxz, m.myz);
     }
     if (wall_node) return 0;
@@ -225,7 +225,7 @@ __device__ __forceinline__ int special_node(const StepArgs &a, int parity, bool 
     if (bcf) {
         double fo[4];
         masked_momentum(a.tag_out[tag], m, fo);
-        float *e = a.side + side_index(slot, x, y, z, x0, y0, min(TILE_X, a.nx - x0), a.nz, a.tile_y) * 16;
+        float *e = a.side + side_index(slot, x, y, z, x0, y0, a.nz, TILE_X, a.tile_y) * 16;
         reinterpret_cast<float2 *>(e)[5] = make_float2((float)(fin[0] - fo[0]), (float)(fin[1] - fo[1]));
         reinterpret_cast<float2 *>(e)[6] = make_float2((float)(fin[2] - fo[2]), (float)(fin[3] - fo[3]));
     }

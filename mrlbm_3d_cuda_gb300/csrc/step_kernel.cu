@@ -586,7 +586,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
             const bool sr_on = kScaled<S> && a.sr_step != nullptr;
             const uint32_t sr_seed = sr_on ? sr_step_seed(*a.sr_step) : 0u;
             const int slot = SPECIAL && a.tile_slot ? a.tile_slot[tile] : -1;  // -1: no boundary nodes
-            float *side = SPECIAL ? a.side + side_index(slot, x, y, zs, x0, y0, w, a.nz, TY) * 16 : nullptr;
+            float *side = SPECIAL ? a.side + side_index(slot, x, y, zs, x0, y0, a.nz, TILE_X, TY) * 16 : nullptr;
             uint32_t marks = 0u;  // of the lane's nodes in plane k - 1, a byte each
             float dm = 0.f, de = 0.f;
             volatile float totals[2];  // of sampled steps: kept on the stack, not in registers
@@ -689,7 +689,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
                                 so.r = sub(fma(q.r, bc<V2>(K.ir), bc<V2>(K.rho0)), bc<V2>(K.rho0));
                                 rescale(bc<V2>(iu), bc<V2>(im));
                             }
-                            float *const e = side + (int64_t)(k - 1) * (w * (TY * 16));
+                            float *const e = side + (int64_t)(k - 1) * (TILE_X * TY * 16);
                             if (q0 && (marks_in & MARK_SNAPSHOT)) snapshot(e, node_of(so, 0), 1.0f, 1.0f);
                             if (q1 && (marks_in & (MARK_SNAPSHOT << 8))) snapshot(e + 16, node_of(so, 1), 1.0f, 1.0f);
                             collide_pair(so, omega, omega);
@@ -763,7 +763,7 @@ __global__ void __launch_bounds__(Geo<S, TY, SPECIAL>::NTH, Geo<S, TY, SPECIAL>:
                         if constexpr (SPECIAL) {
                             u0 = !(marks & MARK_OTHER);
                             u1 = !(marks & (MARK_OTHER << 8));
-                            float *const e = side + (int64_t)(k - 2) * (w * (TY * 16));
+                            float *const e = side + (int64_t)(k - 2) * (TILE_X * TY * 16);
                             if (u0 && (marks & MARK_SNAPSHOT)) snapshot(e, node_of(o, 0), iu, im);
                             if (u1 && (marks & (MARK_SNAPSHOT << 8))) snapshot(e + 16, node_of(o, 1), iu, im);
                         }

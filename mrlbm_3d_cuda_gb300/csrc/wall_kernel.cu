@@ -30,7 +30,7 @@ __device__ __forceinline__ const float *side_entry(const StepArgs &a, int x, int
     const int tx = x / TILE_X, ty = y / a.tile_y;
     const int slot = a.tile_slot[ty * a.tiles_x + tx];
     if (slot < 0) return nullptr;
-    return a.side + side_index(slot, x, y, z, tx * TILE_X, ty * a.tile_y, min(TILE_X, a.nx - tx * TILE_X), a.nz, a.tile_y) * 16;
+    return a.side + side_index(slot, x, y, z, tx * TILE_X, ty * a.tile_y, a.nz, TILE_X, a.tile_y) * 16;
 }
 
 // Bilinear interpolation of the 9 velocity / second-moment fields in the plane z, then

@@ -59,15 +59,15 @@ def test_tall_narrow_case_in_a_batch(cuda_device):
 
 
 def test_side_buffer_holds_the_tiles_that_use_it(cuda_device):
-    """Snapshots take 64 bytes for each node of a tile with stencil, wall or BCFLUID nodes, as wide as the tile is, and
-    none for a tile that only touches a domain face.  A channel with a small cylinder needs little more on the
+    """Snapshots take 64 bytes for each node of a tile with stencil, wall or BCFLUID nodes, narrow tiles sharing slots of
+    64 columns, and none for a tile that only touches a domain face.  A channel with a small cylinder needs little more on the
     device than its moments (131 MB; 126 MB more if each of its tiles, which all have face nodes, held 64 x 16
-    columns), and a 136 x 136 x 112 annulus 134 MB of them beside its 186 MB of moments (189 MB if all were 64 wide)."""
+    columns), and a 136 x 136 x 112 annulus 20 slots, 140 MB, beside its 186 MB of moments (189 MB if all 27 tiles had one)."""
     import torch
     from mrlbm_3d_cuda_gb300 import Simulation, cases
     Simulation(cases.cylinder_channel(64, 40, 8, 10, 24.3, 19.7, 0.05, 60.0), init=False).close()  # context and module
     for desc, most in ((cases.cylinder_channel(320, 40, 128, 10, 63.6, 19.7, 0.05, 60.0), 48),
-                       (cases.annulus(136, 136, 112, 32.0, 64.0, 0.03, 70.0), 134 + 24)):
+                       (cases.annulus(136, 136, 112, 32.0, 64.0, 0.03, 70.0), 140 + 24)):
         free = torch.cuda.mem_get_info()[0]
         with Simulation(desc, init=False):
             used = free - torch.cuda.mem_get_info()[0]
