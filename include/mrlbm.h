@@ -271,8 +271,9 @@ int mrlbm_step_periodic_noalloc(const float *m_in, float *m_out, int32_t nx, int
  * being two blocks wide (a grid of at most 32 nodes along x: one block, and 32 rows in place of 16). */
 int mrlbm_autotune(mrlbm_handle *h, int32_t trial_steps, int32_t tile_out[3]);
 /* Several independent cases (uneven grids allowed; one moment storage for all) advanced
- * together: per step one persistent step-kernel launch over the work items of every case,
- * one node-list launch and one wall launch, replayed from CUDA graphs.  Proposed in place of
+ * together: per step one step-kernel launch over the work items of every case (two when some
+ * cases are at most 32 nodes wide), one node-list launch and one wall launch, replayed from CUDA
+ * graphs.  Proposed in place of
  * running the reference once per case (MRLBM_3D/src/main.cu:7-40). */
 int mrlbm_batch_create(const mrlbm_case_desc *descs, int32_t n, mrlbm_batch **out);
 int mrlbm_batch_destroy(mrlbm_batch *b);

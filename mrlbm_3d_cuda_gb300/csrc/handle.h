@@ -94,7 +94,7 @@ struct mrlbm_handle {
     size_t stage_bytes = 0;
 };
 
-// Independent cases advanced together: every step is one persistent step-kernel launch over
+// Independent cases advanced together: every step is one step-kernel launch (one per kind of tile) over
 // the work items of all cases, one node-list launch and one wall launch, replayed from CUDA
 // graphs (one per ping-pong parity and force sampling).
 struct mrlbm_batch {

@@ -9,8 +9,8 @@
 // nodes for the wall kernel, collides and stores.
 // It reads the state before the step only, so it runs beside the step kernel.  Nodes of blocks
 // the reference never updates (frozen) are in no list.
-// Bound by the latency of scattered loads (197 k nodes of an annulus: 191 MB from HBM in 69 us, 19% of the
-// issue slots, 16 warps an SM); all nine rows of a node are loaded at once for that reason.
+// Bound by the latency of scattered loads (197 k nodes of an annulus: 196 MB of HBM traffic in 67 us, 34% of the
+// issue slots, 15 warps an SM); all nine rows of a node are loaded at once for that reason.
 //
 // Reference (paths inside sakthi-lbm/MRLBM_3D_CUDA):
 //   evaluate_bounday_moments dispatch   MRLBM_3D/src/solver/mlbm.cu:166-184
@@ -234,7 +234,7 @@ __device__ __forceinline__ int special_node(const StepArgs &a, int parity, bool 
 
 // A warp takes ten nodes at a time: three lanes of each gather its populations into shared memory, then one lane
 // per node applies its closure.  With three such rounds a warp the closure fills its lanes, but fewer warps hide
-// the loads: annulus 77 us instead of 72, a cylinder's 17 k nodes 18 instead of 15.
+// the loads: annulus 77 us instead of 72 (67 now), a cylinder's 17 k nodes 18 instead of 15.
 constexpr int kListWarps = 4, kListThreads = 32 * kListWarps, kListNodes = 10;
 
 // BATCH: each block serves the case named by its entry in BatchArgs::list_blocks.

@@ -20,8 +20,8 @@
 // shared memory and no warp waits for another: only the copies of the rows' moments are shared.
 // Bound by issue and FP32 throughput with 16-bit storage (600 warp instructions per 64 nodes, 65% of the
 // issue slots), by issue and HBM with FP32 storage (54%, 5.8 TB/s).  256^3 on GB300, before (populations exchanged
-// through shared-memory rings between CTA barriers) and now: FP32 335 -> 232 us a step, FP16 283 -> 212,
-// hybrid 298 -> 218, BF16 283 -> 214.
+// through shared-memory rings between CTA barriers) and now: FP32 335 -> 231 us a step, FP16 283 -> 206,
+// hybrid 298 -> 216, BF16 283 -> 213.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
